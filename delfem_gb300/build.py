@@ -26,6 +26,8 @@ SOURCES = {
     "capi.cu": [],
     "sched.cpp": [],
     "meshio.cpp": ["-Xcompiler", "-ffp-contract=off"],
+    "strip.cpp": [],
+    "k_strip.cu": [],
     "k_sweep.cu": [],
     "k_solo.cu": [],
     "k_solve.cu": [],

@@ -919,6 +919,16 @@ void setup_sweep_plan(dfg_ctx ctx_, SweepDev& S) {
   upload(ctx_, S.step_rows, P.step_rows.data(), std::max<size_t>(P.step_rows.size(), 1));
 }
 
+void pack_strips(dfg_ctx ctx_, dfg_precond pr, bool fp32) {
+  for (int dir = 0; dir < 2; ++dir) {
+    const StripDev& D = pr->strip[dir][fp32 ? 1 : 0];
+    const StripPackArgs a{D.d, D.ne, pr->b, D.nsteps, D.rec.as<unsigned char>(), D.ent_slot.as<int>(),
+                          D.step_rows.as<int>(), pr->fdiag.as<double>(), pr->foffd.as<double>()};
+    CK(launch_strip_pack(dir == 0, fp32, a, ctx_->stream));
+    launched(ctx_);
+  }
+}
+
 void pack_sweep(dfg_ctx ctx_, dfg_precond pr, SweepDev& S, bool fp32) {
   if (S.levels) return;  // the level-scheduled sweep reads the factor itself
   if (S.solo) {
@@ -969,6 +979,9 @@ struct SweepLaunch {
   const int* spos = nullptr;
   const void* ssrc = nullptr;
   void* sdst = nullptr;
+  // strips
+  bool strip = false;
+  StripArgs ta{};
 };
 
 // The factor's block pattern: the system's for ILU(0), the preconditioner's
@@ -1113,12 +1126,65 @@ SweepLaunch sweep_launch(dfg_ctx ctx_, dfg_precond pr, SweepDev& S, bool fp32, c
   return L;
 }
 
+SweepLaunch strip_launch(dfg_ctx ctx_, dfg_precond pr, int dir, bool fp32, void* out, int* ticket, const int* done) {
+  StripDev& D = pr->strip[dir][fp32 ? 1 : 0];
+  SweepLaunch L{};
+  L.forward = dir == 0;
+  L.fp32 = fp32;
+  L.b = pr->b;
+  L.strip = true;
+  L.grid = D.grid;
+  L.smem = D.smem;
+  StripSlot& s = L.ta.one;
+  s.rec = D.rec.as<unsigned char>();
+  s.strip_chunk = D.strip_chunk.as<int>();
+  s.item_ptr = D.item_ptr.as<int>();
+  s.items = D.items.as<int2>();
+  s.in = D.in.p;
+  s.out = out;
+  s.xch = D.xch.p;
+  s.done = done;
+  s.nstrips = D.nstrips;
+  L.ta.ticket = ticket;
+  L.ta.err = ctx_->err_word.as<int>();
+  L.ta.ne = D.ne;
+  L.ta.W = D.W;
+  L.ta.NS = D.NS;
+  return L;
+}
+
+// One application of the preconditioner, z := (LU)^-1 r, as two sweep
+// launches.  r: the residual in row order, read by the sweeps of the ranged,
+// level-scheduled and one-CTA kinds; strips read their input from feed.in.
+struct PrecondLaunch {
+  SweepLaunch F, B;
+  SweepFeed feed{};  // for the kernel that writes r (r32: where it keeps an FP32 copy of an FP64 r)
+};
+PrecondLaunch precond_launch(dfg_ctx ctx_, dfg_precond pr, bool fp32, const void* r, void* r32, void* z,
+                             int* tickets, const int* done) {
+  PrecondLaunch L;
+  const long long m = (long long)pr->n * pr->b;
+  if (pr->strips) {
+    StripDev &f = pr->strip[0][fp32 ? 1 : 0], &b = pr->strip[1][fp32 ? 1 : 0];
+    L.F = strip_launch(ctx_, pr, 0, fp32, b.in.p, tickets, done);
+    L.B = strip_launch(ctx_, pr, 1, fp32, z, tickets + 1, done);
+    L.feed = SweepFeed{f.in.p, f.pos.as<int>(), {f.xch.p, b.xch.p}, {f.nxch, b.nxch}};
+    return L;
+  }
+  void* y = fp32 ? pr->ybuf32.p : pr->ybuf64.p;
+  L.F = sweep_launch(ctx_, pr, pr->fwd, fp32, r32 ? r32 : r, y, tickets, done);
+  L.B = sweep_launch(ctx_, pr, pr->bwd, fp32, y, z, tickets + 1, done);
+  L.feed = SweepFeed{r32, nullptr, {y, z}, {m, m}};
+  return L;
+}
+
 // Launches one sweep on stream st (no error check and no launch count, so
 // that it can be captured into a graph); the ranged kernel or one launch per
 // level.  dep: the ranged kernel as a programmatic dependent of the previous
 // kernel in the stream (a level sweep's first launch always waits in stream
 // order: it reads the solve's stop flag before waiting).
 cudaError_t enqueue_sweep(const SweepLaunch& L, cudaStream_t st, bool dep = false) {
+  if (L.strip) return launch_strip(L.forward, L.fp32, L.b, L.ta, L.grid, L.smem, st, dep);
   if (L.solo) {
     const cudaError_t e = launch_solo_permute(L.fp32, L.sn, L.b, L.spos, L.ssrc, L.sdst, st);
     if (e != cudaSuccess) return e;
@@ -1141,6 +1207,14 @@ void run_sweep(dfg_ctx ctx_, const SweepLaunch& L) {
   launched(ctx_, launches_of(L));
 }
 
+// Strips whose input no kernel feeds: r (row order, FP64) into step order and
+// the exchange buffers to the sentinel.
+cudaError_t enqueue_strip_feed(const PrecondLaunch& L, const double* r, long long m, cudaStream_t st) {
+  cudaError_t e = launch_solo_permute(false, m, 1, L.feed.pos, r, L.feed.in, st);
+  for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = fill_sentinel(L.feed.nfill[i], L.feed.fill[i], false, st);
+  return e;
+}
+
 struct GraphHolder {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -1150,13 +1224,86 @@ struct GraphHolder {
   }
 };
 
+// Uploads one direction and precision of the strip sweeps; false when the
+// rows do not fit them (strip_plan).  out_pos: where results go (nullptr: row
+// order).
+bool setup_strip(dfg_ctx ctx_, dfg_precond pr, const FactorPattern& F, bool forward, bool fp32, const int* out_pos,
+                 std::vector<int>* pos) {
+  StripDev& D = pr->strip[forward ? 0 : 1][fp32 ? 1 : 0];
+  D = StripDev{};
+  const int n = pr->n, b = pr->b, elem = fp32 ? 4 : 8;
+  StripPlan P;
+  if (!strip_plan(n, b, elem, F.rowptr, F.colind, F.diaind, forward, P)) return false;
+  D.d = P.d;
+  D.ne = P.ne;
+  D.nstrips = P.nstrips;
+  D.nsteps = P.steps();
+  D.nxch = (long long)P.nexport * (P.d.VS / elem);
+  // one strip per CTA while the strips fit the SMs
+  D.W = std::min(kStripMaxWarps, std::max(1, (P.nstrips + ctx_->nsm - 1) / ctx_->nsm));
+  const size_t budget = ctx_->smem_optin;
+  D.NS = 8;
+  while (D.NS > 2 && strip_smem_bytes(D.d, D.W, D.NS) > budget) --D.NS;
+  while (D.W > 1 && strip_smem_bytes(D.d, D.W, D.NS) > budget) --D.W;
+  D.smem = strip_smem_bytes(D.d, D.W, D.NS);
+  if (D.smem > budget) return false;
+  D.grid = std::min((P.nstrips + D.W - 1) / D.W, ctx_->nsm);
+  std::vector<int> ident;
+  if (!out_pos) {
+    ident.resize(n);
+    for (int i = 0; i < n; ++i) ident[i] = i;
+    out_pos = ident.data();
+  }
+  const std::vector<int> meta = strip_meta(P, out_pos, D.W, D.NS);
+  std::vector<int> epos((size_t)n * b);
+  for (int i = 0; i < n; ++i)
+    for (int c = 0; c < b; ++c) epos[(size_t)i * b + c] = P.pos[i] * b + c;
+  DBuf dmeta, dneed;
+  upload(ctx_, dmeta, meta.data(), meta.size());
+  upload(ctx_, dneed, P.need.data(), P.need.size());
+  dalloc(ctx_, D.rec, (size_t)P.nchunks * P.d.chunk_bytes);
+  CK(cudaMemsetAsync(D.rec.p, 0, D.rec.bytes, ctx_->stream));
+  CK(launch_strip_meta(P.d, P.nchunks, dmeta.as<int>(), dneed.as<int>(), D.rec.as<unsigned char>(), ctx_->stream));
+  launched(ctx_);
+  upload(ctx_, D.strip_chunk, P.strip_chunk.data(), P.strip_chunk.size());
+  upload(ctx_, D.item_ptr, P.item_ptr.data(), P.item_ptr.size());
+  upload(ctx_, D.items, P.items.data(), P.items.size(), 16);
+  upload(ctx_, D.ent_slot, P.ent_slot.data(), P.ent_slot.size());
+  upload(ctx_, D.step_rows, P.step_rows.data(), P.step_rows.size());
+  upload(ctx_, D.pos, epos.data(), epos.size());
+  dalloc(ctx_, D.in, (size_t)D.nsteps * D.d.rhs_bytes + 64);
+  CK(cudaMemsetAsync(D.in.p, 0, D.in.bytes, ctx_->stream));
+  dalloc(ctx_, D.xch, (size_t)D.nxch * elem + 64);
+  CK(cudaStreamSynchronize(ctx_->stream));  // the host plan goes away
+  if (pos) *pos = std::move(P.pos);
+  return true;
+}
+
+// Both directions and precisions of the strip sweeps.
+bool setup_strips(dfg_ctx ctx_, dfg_precond pr) {
+  const FactorPattern F = factor_pattern(pr);
+  for (int k = 0; k < 2; ++k) {
+    std::vector<int> ypos;  // y lies where the backward sweep reads it
+    if (!setup_strip(ctx_, pr, F, false, k == 1, nullptr, &ypos) ||
+        !setup_strip(ctx_, pr, F, true, k == 1, ypos.data(), nullptr)) {
+      for (auto& dir : pr->strip)
+        for (StripDev& D : dir) D = StripDev{};
+      return false;
+    }
+  }
+  CK(strip_set_smem_limits(ctx_->smem_optin));
+  return true;
+}
+
 // Schedule choice.  Ranged: the cost model keeps a few candidate range sizes
 // and the fullest-step plan joins them.  Level-scheduled: one launch per
 // dependency level.  Each candidate is timed on the device as one FP32 sweep
 // of the real structure (values do not change the timing; the level launches
 // as a graph, as the solvers replay them) and the fastest wins.  The
 // preconditioner's sweep mode can restrict the choice to one kind.
-void setup_sweep(dfg_ctx ctx_, dfg_precond pr, SweepDev& S, const dfg_system sys, bool forward) {
+// strips: the strip sweeps take the place of the ranged and the one-CTA kinds;
+// they are timed as the ranged kind and the caller makes the choice.
+void setup_sweep(dfg_ctx ctx_, dfg_precond pr, SweepDev& S, const dfg_system sys, bool forward, bool strips) {
   const FactorPattern F = factor_pattern(pr);
   const int mode = pr->sweep_mode;
   const long long m = (long long)sys->n * sys->b;
@@ -1192,7 +1339,22 @@ void setup_sweep(dfg_ctx ctx_, dfg_precond pr, SweepDev& S, const dfg_system sys
   std::vector<SweepPlan> cands;
   size_t best = 0;
   float best_ms = 1e30f;
-  if (mode != 2) {
+  if (strips) {
+    SweepLaunch L = strip_launch(ctx_, pr, forward ? 0 : 1, true, forward ? pr->strip[1][1].in.p : vout.p,
+                                 sc.tickets + 2, nullptr);
+    const StripDev& D = pr->strip[forward ? 0 : 1][1];
+    S.t_ranged = elapsed([&] {
+      CK(fill_sentinel(D.nxch, D.xch.p, true, ctx_->stream));
+      CK(cudaMemsetAsync(sc.tickets + 2, 0, sizeof(int), ctx_->stream));
+      CK(enqueue_sweep(L, ctx_->stream));
+    });
+    launched(ctx_, 4);
+    if (read_err(ctx_) != 0) {
+      CK(cudaMemsetAsync(ctx_->err_word.p, 0, sizeof(int), ctx_->stream));
+      set_err(ctx_, "a triangular-sweep wait timed out while choosing the schedule");
+      throw Fail{DFG_TIMEOUT};
+    }
+  } else if (mode != 2) {
     cands = candidate_sweep_plans(sys->n, sys->b, F.rowptr, F.colind, F.diaind, forward, 32, 4);
     // and the fullest-step plan (ranges of up to 32 grid lines), if it differs
     SweepPlan full = fullest_sweep_plan(sys->n, sys->b, F.rowptr, F.colind, F.diaind, forward, 32);
@@ -1229,7 +1391,7 @@ void setup_sweep(dfg_ctx ctx_, dfg_precond pr, SweepDev& S, const dfg_system sys
   // one-CTA candidate (k_solo.cu), timed in FP32 with its input permutation
   S.solo = false;
   S.t_solo = -1.f;
-  if (mode == 0 || mode == 3) {
+  if ((mode == 0 && !strips) || mode == 3) {
     const bool fits = setup_solo(ctx_, pr, S, F, forward);
     REQUIRE(fits || mode != 3, DFG_INVALID_ARGUMENT, "the one-CTA sweep's records do not fit in shared memory");
     if (fits) {
@@ -1297,7 +1459,7 @@ void setup_sweep(dfg_ctx ctx_, dfg_precond pr, SweepDev& S, const dfg_system sys
       const float ms = elapsed([&] { CK(cudaGraphLaunch(g.exec, ctx_->stream)); });
       launched(ctx_, 3 * launches_of(L));
       S.t_levels = ms;
-      take = ms < best_ms;
+      take = strips || ms < best_ms;
     }
     if (take) {
       S.levels = true;
@@ -1312,7 +1474,7 @@ void setup_sweep(dfg_ctx ctx_, dfg_precond pr, SweepDev& S, const dfg_system sys
       return;
     }
   }
-  if (S.solo) {
+  if (S.solo || strips) {
     S.plan = SweepPlan{};
     return;
   }
@@ -1365,6 +1527,11 @@ extern "C" int dfg_precond_get_sweep_mode(dfg_precond prec, int* fwd, int* bwd) 
   if (!prec->symbolic) {
     prec->ctx->last_error = "dfg_precond_set_linear_system must come first";
     return DFG_NOT_READY;
+  }
+  if (prec->strips) {  // the ranged kind's kernel where the rows fit it
+    if (fwd) *fwd = 1;
+    if (bwd) *bwd = 1;
+    return DFG_OK;
   }
   if (fwd) *fwd = prec->fwd.solo ? 3 : prec->fwd.levels ? 2 : 1;
   if (bwd) *bwd = prec->bwd.solo ? 3 : prec->bwd.levels ? 2 : 1;
@@ -1440,8 +1607,25 @@ extern "C" int dfg_precond_set_linear_system(dfg_precond prec, dfg_system sys) {
     dalloc(ctx, prec->foffd, (size_t)std::max<long long>(prec->nnz, 1) * bs * 8);
     prec->lev_fwd = build_levels(sys->n, F.rowptr, F.colind, F.diaind, true);
     upload(ctx, prec->lev_rows, prec->lev_fwd.rows.data(), std::max<size_t>(prec->lev_fwd.rows.size(), 1));
-    setup_sweep(ctx, prec, prec->fwd, sys, true);
-    setup_sweep(ctx, prec, prec->bwd, sys, false);
+    // strips where the rows fit them, unless both directions together are
+    // faster level-scheduled
+    prec->fwd = SweepDev{};
+    prec->bwd = SweepDev{};
+    prec->strips = (prec->sweep_mode == 0 || prec->sweep_mode == 1) && setup_strips(ctx, prec);
+    setup_sweep(ctx, prec, prec->fwd, sys, true, prec->strips);
+    setup_sweep(ctx, prec, prec->bwd, sys, false, prec->strips);
+    if (prec->strips && prec->sweep_mode == 0 &&
+        prec->fwd.t_levels + prec->bwd.t_levels < prec->fwd.t_ranged + prec->bwd.t_ranged) {
+      prec->strips = false;
+      for (auto& dir : prec->strip)
+        for (StripDev& D : dir) D = StripDev{};
+    } else if (prec->strips) {
+      for (SweepDev* S : {&prec->fwd, &prec->bwd}) {
+        S->levels = false;
+        S->lev = Levels{};
+        S->lev_info.release();
+      }
+    }
     dalloc(ctx, prec->ybuf64, vec_bytes(sys, 8));
     dalloc(ctx, prec->ybuf32, vec_bytes(sys, 4));
     CK(cudaStreamSynchronize(ctx->stream));
@@ -1481,8 +1665,12 @@ extern "C" int dfg_precond_set_value(dfg_precond prec, dfg_system sys) {
     launched(ctx, nl);
     int h_nsing = 0;
     CK(cudaMemcpyAsync(&h_nsing, nsing, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    pack_sweep(ctx, prec, prec->fwd, false);
-    pack_sweep(ctx, prec, prec->bwd, false);
+    if (prec->strips) {
+      pack_strips(ctx, prec, false);
+    } else {
+      pack_sweep(ctx, prec, prec->fwd, false);
+      pack_sweep(ctx, prec, prec->bwd, false);
+    }
     CK(cudaStreamSynchronize(ctx->stream));
     prec->numeric = true;
     prec->numeric32 = false;
@@ -1497,6 +1685,11 @@ extern "C" int dfg_precond_set_value(dfg_precond prec, dfg_system sys) {
 namespace {
 void ensure_numeric32(dfg_ctx ctx_, dfg_precond prec) {
   if (prec->numeric32) return;
+  if (prec->strips) {
+    pack_strips(ctx_, prec, true);
+    prec->numeric32 = true;
+    return;
+  }
   pack_sweep(ctx_, prec, prec->fwd, true);
   pack_sweep(ctx_, prec, prec->bwd, true);
   if (prec->fwd.levels || prec->bwd.levels) {  // the level-scheduled sweeps read the factor in CRS
@@ -1521,12 +1714,17 @@ extern "C" int dfg_precond_solve(dfg_precond prec, dfg_system sys, int iv) {
     const long long m = (long long)sys->n * sys->b;
     Scratch sc = scratch_of(ctx);
     CK(cudaMemsetAsync(sc.tickets, 0, 2 * sizeof(int), ctx->stream));
-    CK(fill_sentinel(m, prec->ybuf64.p, false, ctx->stream));
-    SweepLaunch F = sweep_launch(ctx, prec, prec->fwd, false, v, prec->ybuf64.p, sc.tickets, nullptr);
-    run_sweep(ctx, F);
-    CK(fill_sentinel(m, v, false, ctx->stream));
-    SweepLaunch B = sweep_launch(ctx, prec, prec->bwd, false, prec->ybuf64.p, v, sc.tickets + 1, nullptr);
-    run_sweep(ctx, B);
+    PrecondLaunch L = precond_launch(ctx, prec, false, v, nullptr, v, sc.tickets, nullptr);
+    if (prec->strips) {
+      CK(enqueue_strip_feed(L, v, m, ctx->stream));
+      launched(ctx, 1);
+      run_sweep(ctx, L.F);
+    } else {
+      CK(fill_sentinel(m, prec->ybuf64.p, false, ctx->stream));
+      run_sweep(ctx, L.F);
+      CK(fill_sentinel(m, v, false, ctx->stream));
+    }
+    run_sweep(ctx, L.B);
     launched(ctx, 2);  // the two sentinel fills
     if (read_err(ctx) != 0) {
       CK(cudaMemsetAsync(ctx->err_word.p, 0, sizeof(int), ctx->stream));
@@ -1638,16 +1836,14 @@ static int solve_pcg_f64vec(dfg_system sys, dfg_precond prec, bool fp32z, bool t
     v.x = sys->upd.as<double>();
     v.p = sys->w_p.as<double>();
     v.q = sys->w_q.as<double>();
-    v.y = fp32z ? prec->ybuf32.p : prec->ybuf64.p;
     v.z = fp32z ? sys->w_z32.p : sys->w_z.p;
     v.m = m;
-    v.r32 = fp32z ? sys->w_r32.as<float>() : nullptr;
     v.rd = sys->w_rd.as<double>();
     v.b = sys->rhs0_valid ? sys->rhs0.as<double>() : nullptr;
     const int* done = reinterpret_cast<const int*>(reinterpret_cast<const char*>(st) + offsetof(PcgState, done));
-    const void* sweep_in = fp32z ? (const void*)v.r32 : (const void*)v.r;
-    SweepLaunch F = sweep_launch(ctx, prec, prec->fwd, fp32z, sweep_in, v.y, sc.tickets, done);
-    SweepLaunch B = sweep_launch(ctx, prec, prec->bwd, fp32z, v.y, v.z, sc.tickets + 1, done);
+    const PrecondLaunch PL = precond_launch(ctx, prec, fp32z, v.r, fp32z ? sys->w_r32.p : nullptr, v.z, sc.tickets, done);
+    const SweepLaunch &F = PL.F, &B = PL.B;
+    v.feed = PL.feed;
     const int maxit = (int)std::min<unsigned>(*iteration, 0x7fffffffu);
     const double tol = *conv_ratio;
     // prologue (solver_ls_iter.cpp:106-128)
@@ -1774,14 +1970,14 @@ extern "C" int dfg_solve_pcg_mixed(dfg_system sys, dfg_precond prec, double* con
     Scratch sc = scratch_of(ctx);
     Red red = red_of(ctx, 2);
     MixVecs v{sys->rhs0.as<double>(), sys->upd.as<double>(), sys->w_rd.as<double>(), sys->w_d.as<double>(),
-              sys->w_r32.as<float>(), sys->w_p32.as<float>(), sys->w_q32.as<float>(), prec->ybuf32.as<float>(),
-              sys->w_z32.as<float>(), m};
+              sys->w_r32.as<float>(), sys->w_p32.as<float>(), sys->w_q32.as<float>(), sys->w_z32.as<float>(), m, {}};
     ensure_sell(ctx, sys, true);
     const MatView A64 = view64(sys);
     const MatView A32 = view32(sys);
     const int* done = reinterpret_cast<const int*>(reinterpret_cast<const char*>(st) + offsetof(PcgState, done));
-    SweepLaunch F = sweep_launch(ctx, prec, prec->fwd, true, v.r, v.y, sc.tickets, done);
-    SweepLaunch B = sweep_launch(ctx, prec, prec->bwd, true, v.y, v.z, sc.tickets + 1, done);
+    const PrecondLaunch PL = precond_launch(ctx, prec, true, v.r, nullptr, v.z, sc.tickets, done);
+    const SweepLaunch &F = PL.F, &B = PL.B;
+    v.feed = PL.feed;
     CK(cudaMemsetAsync(v.x, 0, (size_t)m * 8, ctx->stream));
     CK(cudaMemsetAsync(v.d, 0, (size_t)m * 8, ctx->stream));
     CK(api_dot(m, v.b, v.b, red, ctx->stream));
@@ -1891,10 +2087,10 @@ extern "C" int dfg_solve_pbicgstab(dfg_system sys, dfg_precond prec, int mode, d
     Scratch sc = scratch_of(ctx);
     Red red = red_of(ctx, 1);
     const int* done = reinterpret_cast<const int*>(reinterpret_cast<const char*>(st) + offsetof(BicgState, done));
-    SweepLaunch F1 = sweep_launch(ctx, prec, prec->fwd, false, v.p, v.y, sc.tickets, done);
-    SweepLaunch B1 = sweep_launch(ctx, prec, prec->bwd, false, v.y, v.mp, sc.tickets + 1, done);
-    SweepLaunch F2 = sweep_launch(ctx, prec, prec->fwd, false, v.s, v.y, sc.tickets, done);
-    SweepLaunch B2 = sweep_launch(ctx, prec, prec->bwd, false, v.y, v.ms, sc.tickets + 1, done);
+    const PrecondLaunch P1 = precond_launch(ctx, prec, false, v.p, nullptr, v.mp, sc.tickets, done);
+    const PrecondLaunch P2 = precond_launch(ctx, prec, false, v.s, nullptr, v.ms, sc.tickets, done);
+    const SweepLaunch &F1 = P1.F, &B1 = P1.B, &F2 = P2.F, &B2 = P2.B;
+    const int feed_launches = prec->strips ? 3 : 0;  // strips: the sweeps' input and exchange buffers
     const int maxit = (int)std::min<unsigned>(*iteration, 0x7fffffffu);
     const double tol = *conv_ratio;
     CK(bicg_init(v, st, red, tol, maxit, sc.tickets, ctx->stream));
@@ -1905,15 +2101,18 @@ extern "C" int dfg_solve_pbicgstab(dfg_system sys, dfg_precond prec, int mode, d
     if (h.done == 0) {
       ensure_sell(ctx, sys, false);
       const MatView A = view64(sys);
-      const long long per_it = 5 + launches_of(F1) + launches_of(B1) + launches_of(F2) + launches_of(B2);
+      const long long per_it =
+          5 + launches_of(F1) + launches_of(B1) + launches_of(F2) + launches_of(B2) + 2 * feed_launches;
       const int chunk = std::max(2, std::min(m < 200000 ? 4 : 16, (int)(4096 / per_it)));
       Chunk g;
       CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
       for (int c = 0; c < chunk; ++c) {
+        if (feed_launches) enqueue_strip_feed(P1, v.p, m, ctx->stream);
         enqueue_sweep(F1, ctx->stream);
         enqueue_sweep(B1, ctx->stream);
         bicg_amp(A, v, st, red, ctx->stream);
         bicg_s(v, st, sc.tickets, ctx->stream);
+        if (feed_launches) enqueue_strip_feed(P2, v.s, m, ctx->stream);
         enqueue_sweep(F2, ctx->stream);
         enqueue_sweep(B2, ctx->stream);
         bicg_ams(A, v, st, red2, ctx->stream);
@@ -2040,17 +2239,15 @@ extern "C" int dfg_profile_kernels(dfg_system sys, dfg_precond prec, int mode, i
     if (fp32z && !mixed) CK(cudaMemcpyAsync(tr32.p, sys->w_r32.p, (size_t)m * 4, cudaMemcpyDeviceToDevice, ctx->stream));
     PcgVecs v{};
     v.r = tr.as<double>(); v.x = tx.as<double>(); v.p = tp.as<double>(); v.q = sys->w_q.as<double>();
-    v.y = fp32z ? prec->ybuf32.p : prec->ybuf64.p;
     v.z = fp32z ? sys->w_z32.p : sys->w_z.p;
-    v.m = m; v.r32 = tr32.as<float>(); v.rd = td.as<double>(); v.b = sys->rhs0.as<double>();
+    v.m = m; v.rd = td.as<double>(); v.b = sys->rhs0.as<double>();
     MixVecs w{sys->rhs0.as<double>(), tx.as<double>(), sys->w_rd.as<double>(), td.as<double>(),
-              tr.as<float>(), tp.as<float>(), sys->w_q32.as<float>(), prec->ybuf32.as<float>(),
-              sys->w_z32.as<float>(), m};
-    const void* rin = mixed ? (const void*)w.r : (fp32z ? (const void*)v.r32 : (const void*)v.r);
-    void* ybuf = fp32z ? prec->ybuf32.p : prec->ybuf64.p;
+              tr.as<float>(), tp.as<float>(), sys->w_q32.as<float>(), sys->w_z32.as<float>(), m, {}};
     void* zbuf = fp32z ? sys->w_z32.p : sys->w_z.p;
-    SweepLaunch F = sweep_launch(ctx, prec, prec->fwd, fp32z, rin, ybuf, sc.tickets, nullptr);
-    SweepLaunch B = sweep_launch(ctx, prec, prec->bwd, fp32z, ybuf, zbuf, sc.tickets + 1, nullptr);
+    const PrecondLaunch PL = precond_launch(ctx, prec, fp32z, tr.p, fp32z && !mixed ? tr32.p : nullptr, zbuf,
+                                            sc.tickets, nullptr);
+    const SweepLaunch &F = PL.F, &B = PL.B;
+    v.feed = w.feed = PL.feed;
     auto timed = [&](int slot, auto&& pre, auto&& body) {
       for (int r = 0; r < reps + 1; ++r) {
         pre();
@@ -2067,11 +2264,11 @@ extern "C" int dfg_profile_kernels(dfg_system sys, dfg_precond prec, int mode, i
     if (mixed) timed(0, nop, [&] { CK(mix_spmv_pap(A32, w, st, red, ctx->stream)); });
     else timed(0, nop, [&] { CK(pcg_spmv_pap(A64, v, st, red, ctx->stream)); });
     timed(1, [&] {
-        CK(fill_sentinel(m, ybuf, fp32z, ctx->stream));
+        CK(fill_sentinel(PL.feed.nfill[0], PL.feed.fill[0], fp32z, ctx->stream));
         CK(cudaMemsetAsync(sc.tickets, 0, 2 * sizeof(int), ctx->stream));
       }, [&] { run_sweep(ctx, F); });
     timed(2, [&] {
-        CK(fill_sentinel(m, zbuf, fp32z, ctx->stream));
+        CK(fill_sentinel(PL.feed.nfill[1], PL.feed.fill[1], fp32z, ctx->stream));
         CK(cudaMemsetAsync(sc.tickets, 0, 2 * sizeof(int), ctx->stream));
       }, [&] { run_sweep(ctx, B); });
     if (mixed) {

@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "../../include/dfg.h"
+#include "k_strip.h"
 #include "k_sweep.h"
 
 namespace dfg {
@@ -214,6 +215,17 @@ struct SweepDev {
   SweepPlan plan;
 };
 
+// One direction of the strip sweeps (k_strip.cu) in one precision.
+struct StripDev {
+  StripDims d{};
+  int ne = 0, nstrips = 0, W = 1, NS = 2, grid = 1;
+  long long nsteps = 0, nxch = 0;  // nxch: elements of the exchange buffer
+  size_t smem = 0;
+  DBuf rec, strip_chunk, item_ptr, items, ent_slot, step_rows;
+  DBuf pos;                        // per vector element (n*b): its place in `in`
+  DBuf in, xch;
+};
+
 }  // namespace dfg
 
 struct dfg_ctx_s {
@@ -280,5 +292,7 @@ struct dfg_precond_s {
   dfg::Levels lev_fwd;
   dfg::DBuf lev_rows;
   dfg::SweepDev fwd, bwd;
+  bool strips = false;             // both directions sweep in strips (fwd, bwd then unused)
+  dfg::StripDev strip[2][2];       // [forward, backward][FP64, FP32]
   dfg::DBuf ybuf64, ybuf32;        // forward-sweep outputs
 };

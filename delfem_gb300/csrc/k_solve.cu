@@ -86,6 +86,20 @@ __device__ __forceinline__ double zval(const void* z, long long k) {
   return (double)reinterpret_cast<const Z*>(z)[k];
 }
 
+// element k of a residual into the forward sweep's input (Z: the sweeps' type)
+template <typename Z, typename R>
+__device__ __forceinline__ void feed_put(const SweepFeed& f, long long k, R r) {
+  if (f.in) reinterpret_cast<Z*>(f.in)[f.pos ? f.pos[k] : k] = (Z)r;
+}
+template <typename Z>
+__device__ __forceinline__ void feed_fill(const SweepFeed& f) {
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < f.nfill[i];
+         k += (long long)gridDim.x * blockDim.x)
+      reinterpret_cast<Z*>(f.fill[i])[k] = sentinel_value<Z>();
+}
+
 // x := 0 * x (SCAL(0,x)); rr0 = r.r; early exit below 1e-30; sentinels
 template <typename Z>
 __global__ void k_pcg_init(PcgVecs v, PcgState* st, Red red, double tol, int maxit, int* tickets) {
@@ -94,10 +108,9 @@ __global__ void k_pcg_init(PcgVecs v, PcgState* st, Red red, double tol, int max
     v.x[k] = v.x[k] * 0.0;
     const double r = v.r[k];
     part += r * r;
-    reinterpret_cast<Z*>(v.y)[k] = sentinel_value<Z>();
-    reinterpret_cast<Z*>(v.z)[k] = sentinel_value<Z>();
-    if constexpr (sizeof(Z) == 4) v.r32[k] = (float)r;
+    feed_put<Z>(v.feed, k, r);
   }
+  feed_fill<Z>(v.feed);
   double tot;
   if (grid_sum(part, red, &tot) && threadIdx.x == 0) {
     st->rr0 = tot;
@@ -133,7 +146,7 @@ __global__ void k_pcg_after_precond0(PcgVecs v, PcgState* st, Red red) {
 }
 
 // r := r - alpha q; x := x + alpha p (AXPY, no-op for alpha == 0); rr = r.r;
-// convergence check; sentinel refill for the sweeps; sweep tickets reset
+// convergence check; the sweeps' feed; sweep tickets reset
 template <typename Z>
 __global__ void k_pcg_update_rx(PcgVecs v, PcgState* st, Red red, int* tickets) {
   pdl_enter();
@@ -148,10 +161,9 @@ __global__ void k_pcg_update_rx(PcgVecs v, PcgState* st, Red red, int* tickets) 
       v.x[k] = __dadd_rn(v.x[k], __dmul_rn(alpha, v.p[k]));
     }
     part += r * r;
-    reinterpret_cast<Z*>(v.y)[k] = sentinel_value<Z>();
-    reinterpret_cast<Z*>(v.z)[k] = sentinel_value<Z>();
-    if constexpr (sizeof(Z) == 4) v.r32[k] = (float)r;
+    feed_put<Z>(v.feed, k, r);
   }
+  feed_fill<Z>(v.feed);
   double tot;
   if (grid_sum(part, red, &tot) && threadIdx.x == 0) {
     st->rr = tot;
@@ -226,10 +238,9 @@ __global__ void k_pcg_replace(PcgVecs v, PcgState* st, int* tickets) {
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < v.m; k += (long long)gridDim.x * blockDim.x) {
     const double r = v.rd[k];
     v.r[k] = r;
-    if constexpr (sizeof(Z) == 4) v.r32[k] = (float)r;
-    reinterpret_cast<Z*>(v.y)[k] = sentinel_value<Z>();
-    reinterpret_cast<Z*>(v.z)[k] = sentinel_value<Z>();
+    feed_put<Z>(v.feed, k, r);
   }
+  feed_fill<Z>(v.feed);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     st->done = 0;
     tickets[0] = 0;
@@ -275,10 +286,11 @@ __global__ void k_mix_start(PcgState* st, double tol, double bb, double delta, i
 // true residual; the correction is folded into the FP64 solution
 __global__ void k_mix_replace(MixVecs v, PcgState* st, int* tickets) {
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < v.m; k += (long long)gridDim.x * blockDim.x) {
-    v.r[k] = (float)v.rd[k];
-    v.y[k] = sentinel_value<float>();
-    v.z[k] = sentinel_value<float>();
+    const float r = (float)v.rd[k];
+    v.r[k] = r;
+    feed_put<float>(v.feed, k, r);
   }
+  feed_fill<float>(v.feed);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     st->rr_ref = st->rr;
     st->done = 0;
@@ -312,9 +324,9 @@ __global__ void k_mix_update_rx(MixVecs v, PcgState* st, Red red, int* tickets) 
       v.d[k] = v.d[k] + alpha * (double)v.p[k];
     }
     part += (double)r * (double)r;
-    v.y[k] = sentinel_value<float>();
-    v.z[k] = sentinel_value<float>();
+    feed_put<float>(v.feed, k, r);
   }
+  feed_fill<float>(v.feed);
   double tot;
   if (grid_sum(part, red, &tot) && threadIdx.x == 0) {
     st->rr = tot;

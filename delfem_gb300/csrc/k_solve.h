@@ -51,16 +51,26 @@ struct MatView {
 cudaError_t sell_pack(int nslices, int b, const long long* ptr, const int* src, const double* diag,
                       const double* offd, void* out, bool fp32, cudaStream_t s);
 
+// What the kernel that writes a residual prepares for the sweeps that follow:
+// the forward input where the sweep reads it (in[pos[k]], pos == nullptr: row
+// order; in == nullptr: the sweep reads the residual itself) and the sentinel
+// in the buffers through which the sweeps hand values over.
+struct SweepFeed {
+  void* in;
+  const int* pos;
+  void* fill[2];
+  long long nfill[2];
+};
+
 // ---- FP64 PCG (plain path) -------------------------------------------------
 struct PcgVecs {
   double* r;   // residual slot
   double* x;   // update slot
   double* p;
   double* q;   // A p
-  void* y;     // forward-sweep output (double, or float with an FP32 factor)
-  void* z;     // backward-sweep output (preconditioned residual)
+  void* z;     // backward-sweep output (preconditioned residual; double, or float with an FP32 factor)
   long long m; // n*b
-  float* r32;  // FP32 copy of r fed to FP32 sweeps (nullptr with an FP64 factor)
+  SweepFeed feed;
   double* rd;  // true-residual scratch (b - A x)
   const double* b;  // finalized right-hand side (true-residual checks)
 };
@@ -76,7 +86,7 @@ cudaError_t pcg_rz_beta(const PcgVecs& v, PcgState* st, Red red, bool fp32z, cud
 cudaError_t pcg_update_p(const PcgVecs& v, PcgState* st, bool fp32z, cudaStream_t s, bool dep = false);
 // rd = b - A x, rr = rd.rd (into st->rr; state otherwise untouched)
 cudaError_t pcg_true_residual(const MatView& A, const PcgVecs& v, PcgState* st, Red red, cudaStream_t s);
-// r = rd (and r32), sentinels, tickets reset, done = 0: continue from the true residual
+// r = rd (and the sweeps' feed), tickets reset, done = 0: continue from the true residual
 cudaError_t pcg_replace(const PcgVecs& v, PcgState* st, int* tickets, bool fp32z, cudaStream_t s);
 
 // ---- mixed precision ----------------------------------------------------
@@ -88,9 +98,9 @@ struct MixVecs {
   float* r;        // inner residual
   float* p;
   float* q;
-  float* y;
   float* z;
   long long m;
+  SweepFeed feed;
 };
 // rd = b - A64 x; rr = rd.rd (FP64)
 cudaError_t mix_true_residual(const MatView& A64, const MixVecs& v, PcgState* st, Red red, cudaStream_t s);

@@ -1,0 +1,540 @@
+// k_strip.cu -- forward / backward substitution of the block ILU factor
+// (CMatDiaFrac_BlkCrs::ForwardSubstitution / BackwardSubstitution,
+// src/matvec/matdiafrac_blkcrs.cpp:332-669) in the reference's natural order,
+// one warp per strip of rows.
+//
+// What bounds a sweep is its chain of dependency levels, so the kernel is
+// built around the time from one level to the next.  A strip (strip.cpp) holds
+// up to RW grid lines; its warp takes one level of the strip per step, the
+// rows' dependencies inside the strip coming from a shared-memory ring of the
+// warp's own results: store, __syncwarp, load -- 33 cycles on GB300 -- and no
+// barrier between warps.  Everything else a step needs is brought to shared
+// memory ahead of it:
+//   * the step records (dependency codes, factor blocks, output positions) and
+//     the right-hand sides, both contiguous in step order, by two TMA bulk
+//     copies per chunk of steps, issued by the warp itself NS chunks ahead (it
+//     frees a stage by finishing it, so no barrier with a producer);
+//   * the values of other strips by a receiver warp beside each compute warp.
+//     A row that another strip needs is also written to an exchange buffer in
+//     global memory that was filled with a NaN sentinel; the receiver's lanes
+//     poll the strip's items, listed in the order of first use, four each in
+//     flight, and put them into the warp's mailbox (a ring of slots) as they
+//     arrive.  `delivered` counts the arrived prefix; a step says how many
+//     items it needs, one compare when they are there.
+// Measured on GB300, FP32, per sweep (forward / backward): the 1000x500
+// cantilever 0.21 / 0.16 ms (ranged kernel 1.09 / 1.10), Poisson on 301x257
+// cells 63 / 62 us (one CTA per sweep 200 / 196), elasticity on 56^3 cells 136 /
+// 127 us (a launch per level 345 / 306).  FP64: the cantilever 0.70 / 0.51 ms
+// (2.36 / 2.08), Poisson on 128x128 cells 71 / 63 us (133 / 123).  Inside one
+// strip a level costs 165 cycles (1x1 blocks, FP32) to 820 (2x2, FP64); a
+// hand-off between strips about 3,000, of which the L2 takes 600-900.
+//
+// Strips are claimed in order, W per CTA, through a ticket, so a strip only
+// waits on strips already running, whatever the number of resident CTAs.
+// Every wait is bounded; one that gives up records kErrTimeout, and the launch
+// drains its copies and returns.
+//
+// A row is evaluated by the operations of the other sweep kernels in their
+// order (entries ascending, FMA chain, then D^-1), so the ranged and one-CTA
+// kernels give the same bits.
+//
+// Chunk layout: [need: CH ints, kStripHdr bytes][steps: step_bytes each]; a
+// step is pieces of 16 bytes per lane, piece j of lane l at (j*32 + l)*16:
+// MC pieces of metadata (16-bit codes, output position, exchange slot), then
+// VC pieces of values (the lane's factor rows entry by entry, then its D^-1
+// row(s) in the forward sweep).
+#include "dfg_common.cuh"
+#include "k_mbar.cuh"
+#include "k_strip.h"
+
+namespace dfg {
+
+__device__ __forceinline__ int ld_acquire_s(const int* p) {
+  int v;
+  asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];" : "=r"(v) : "r"(smem_u32(p)) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_release_s(int* p, int v) {
+  asm volatile("st.release.cta.shared::cta.s32 [%0], %1;" ::"r"(smem_u32(p)), "r"(v) : "memory");
+}
+
+// a row's value as the ring, mailbox and exchange buffer hold it
+template <typename T, int N>
+struct alignas(N * sizeof(T) > 16 ? 16 : N * sizeof(T)) Vec {
+  T v[N];
+};
+
+// Relaxed gpu-scope load of a row's value under a predicate (no branch); v is
+// left as it is otherwise.  Each element is compared with the sentinel by
+// itself, so no atomicity beyond an element is needed.
+__device__ __forceinline__ void xload(bool on, const float* p, Vec<float, 1>& v) {
+  asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %1, 0;\n @q ld.relaxed.gpu.global.f32 %0, [%2];\n}"
+               : "+f"(v.v[0]) : "r"((int)on), "l"(p));
+}
+__device__ __forceinline__ void xload(bool on, const double* p, Vec<double, 1>& v) {
+  asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %1, 0;\n @q ld.relaxed.gpu.global.f64 %0, [%2];\n}"
+               : "+d"(v.v[0]) : "r"((int)on), "l"(p));
+}
+__device__ __forceinline__ void xload(bool on, const float* p, Vec<float, 2>& v) {
+  asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %2, 0;\n @q ld.relaxed.gpu.global.v2.f32 {%0, %1}, [%3];\n}"
+               : "+f"(v.v[0]), "+f"(v.v[1]) : "r"((int)on), "l"(p));
+}
+__device__ __forceinline__ void xload(bool on, const double* p, Vec<double, 2>& v) {
+  asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %2, 0;\n @q ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%3];\n}"
+               : "+d"(v.v[0]), "+d"(v.v[1]) : "r"((int)on), "l"(p));
+}
+__device__ __forceinline__ void xload(bool on, const float* p, Vec<float, 4>& v) {
+  asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %4, 0;\n @q ld.relaxed.gpu.global.v4.f32 {%0, %1, %2, %3}, [%5];\n}"
+               : "+f"(v.v[0]), "+f"(v.v[1]), "+f"(v.v[2]), "+f"(v.v[3]) : "r"((int)on), "l"(p));
+}
+__device__ __forceinline__ void xload(bool on, const double* p, Vec<double, 4>& v) {
+  asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %3, 0;\n @q ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%4];\n"
+               " @q ld.relaxed.gpu.global.f64 %2, [%4+16];\n}"
+               : "+d"(v.v[0]), "+d"(v.v[1]), "+d"(v.v[2]) : "r"((int)on), "l"(p));
+}
+// Stores under a predicate (no branch): a row's value at p when on >= 0.  The
+// exchange stores are gpu-scope relaxed.
+__device__ __forceinline__ void xstore(int on, float* p, const Vec<float, 1>& y) {
+  asm volatile("{\n .reg .pred q;\n setp.ge.s32 q, %0, 0;\n @q st.relaxed.gpu.global.f32 [%1], %2;\n}" ::"r"(on), "l"(p),
+               "f"(y.v[0]));
+}
+__device__ __forceinline__ void xstore(int on, double* p, const Vec<double, 1>& y) {
+  asm volatile("{\n .reg .pred q;\n setp.ge.s32 q, %0, 0;\n @q st.relaxed.gpu.global.f64 [%1], %2;\n}" ::"r"(on), "l"(p),
+               "d"(y.v[0]));
+}
+__device__ __forceinline__ void xstore(int on, float* p, const Vec<float, 2>& y) {
+  asm volatile("{\n .reg .pred q;\n setp.ge.s32 q, %0, 0;\n @q st.relaxed.gpu.global.v2.f32 [%1], {%2, %3};\n}" ::"r"(on),
+               "l"(p), "f"(y.v[0]), "f"(y.v[1]));
+}
+__device__ __forceinline__ void ostore(int on, float* p, const Vec<float, 1>& y) {
+  asm volatile("{\n .reg .pred q;\n setp.ge.s32 q, %0, 0;\n @q st.global.f32 [%1], %2;\n}" ::"r"(on), "l"(p), "f"(y.v[0]));
+}
+__device__ __forceinline__ void ostore(int on, double* p, const Vec<double, 1>& y) {
+  asm volatile("{\n .reg .pred q;\n setp.ge.s32 q, %0, 0;\n @q st.global.f64 [%1], %2;\n}" ::"r"(on), "l"(p), "d"(y.v[0]));
+}
+__device__ __forceinline__ void ostore(int on, float* p, const Vec<float, 2>& y) {
+  asm volatile("{\n .reg .pred q;\n setp.ge.s32 q, %0, 0;\n @q st.global.v2.f32 [%1], {%2, %3};\n}" ::"r"(on), "l"(p),
+               "f"(y.v[0]), "f"(y.v[1]));
+}
+
+// The receiver of one strip: polls its items in the exchange buffer and
+// delivers them to the mailbox in order.  Two sets of H batches of 32 items are
+// in flight; a set that is through makes room for the next one.
+template <typename T, int B, int H>
+__device__ __forceinline__ void receive(const StripSlot& S, int r, unsigned char* mail, int* delivered,
+                                        const int* consumed, int* err, int lane) {
+  constexpr int BP = B == 3 ? 4 : B;
+  constexpr int VS = BP * (int)sizeof(T);
+  constexpr int M = strip_mailbox(VS);
+  constexpr int U = 2 * H;
+  const int i0 = S.item_ptr[r], cnt = S.item_ptr[r + 1] - i0;
+  const int2* __restrict__ items = S.items + i0;
+  const T* xch = reinterpret_cast<const T*>(S.xch);
+  auto item = [&](int q) { return q < cnt ? items[q] : make_int2(0, 0); };
+  int2 it[U], nxt[H];
+  unsigned got = 0;  // bit u: this lane's item of batch u has been delivered
+#pragma unroll
+  for (int u = 0; u < U; ++u) it[u] = item(u * 32 + lane);
+#pragma unroll
+  for (int u = 0; u < H; ++u) nxt[u] = item((U + u) * 32 + lane);
+  int base = 0;
+  long long t0 = clock64();
+  for (unsigned n = 1; base < cnt; ++n) {
+    if ((n & 63) == 0) {
+      if (ld_relaxed_int(err) != 0) return;
+      if (clock64() - t0 > kWaitCycles) {
+        if (lane == 0) record_fail(err, kErrTimeout, kSitePoll, -1, r);
+        return;
+      }
+    }
+    const int done_steps = cnt > M ? ld_acquire_s(consumed) : 0;
+    Vec<T, BP> v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+#pragma unroll
+      for (int d = 0; d < BP; ++d) v[u].v[d] = sentinel_value<T>();
+      xload(!(got >> u & 1) && base + u * 32 + lane < cnt && it[u].y <= done_steps, xch + (size_t)it[u].x * BP, v[u]);
+    }
+    const unsigned had = got;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      bool ok = true;
+#pragma unroll
+      for (int d = 0; d < B; ++d) ok &= !is_sentinel(v[u].v[d]);
+      if (ok) *reinterpret_cast<Vec<T, BP>*>(mail + (size_t)((base + u * 32 + lane) % M) * VS) = v[u];
+      got |= (unsigned)ok << u;
+    }
+    if (!__any_sync(0xffffffffu, got != had)) continue;
+    t0 = clock64();
+    // the delivered prefix over the batches in flight
+    int pre = base;
+    bool whole = true;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const unsigned b = __ballot_sync(0xffffffffu, got >> u & 1);
+      pre += whole ? __popc(b & ~(b + 1u)) : 0;
+      whole = whole && b == 0xffffffffu;
+    }
+    __syncwarp();
+    if (lane == 0) st_release_s(delivered, pre);
+    if (pre >= cnt) break;
+    if (pre - base >= 32 * H) {
+#pragma unroll
+      for (int u = 0; u < H; ++u) {
+        it[u] = it[H + u];
+        it[H + u] = nxt[u];
+      }
+      got >>= H;
+      base += 32 * H;
+#pragma unroll
+      for (int u = 0; u < H; ++u) nxt[u] = item(base + (U + u) * 32 + lane);
+    }
+  }
+}
+
+template <typename T, int B, bool FWD, int NE>
+__global__ void __launch_bounds__(2 * kStripMaxWarps * 32) k_strip(StripArgs a) {
+  constexpr int SZ = (int)sizeof(T);
+  constexpr StripDims D = strip_dims(B, SZ, FWD, NE);
+  constexpr int LPR = D.LPR, RW = D.RW, MC = D.MC, VC = D.VC, CH = D.CH, VS = D.VS;
+  constexpr int BP = B == 3 ? 4 : B;          // elements of a row's value, padded
+  constexpr int PER16 = 16 / SZ;
+  constexpr int EV = B * (LPR == 1 ? B : 1);  // values per entry and lane
+  constexpr int RHS_CHUNK = CH * D.rhs_bytes;
+  // steps per test of the mailbox: short steps share one (a test is a branch,
+  // about 10 cycles, and waiting for the last of four steps' items costs a
+  // hand-off three steps)
+  constexpr int G = NE <= 4 && CH >= 4 ? 4 : 1;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ int s_ticket, s_stop;
+  const int W = a.W, NS = a.NS;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool compute = warp < W;
+  const int w = compute ? warp : warp - W;
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem) + w * NS;
+  int* delivered = reinterpret_cast<int*>(smem + (size_t)W * NS * 8) + w * 4;
+  int* consumed = delivered + 1;
+  unsigned char* rstage = smem + strip_stage_offset(D, W, NS, w);  // NS chunks of records
+  unsigned char* vstage = rstage + (size_t)NS * D.chunk_bytes;     // NS chunks of right-hand sides
+  unsigned char* region = smem + strip_region_offset(D, W, NS, w);
+  if (compute && lane < kStripZero / 4) reinterpret_cast<unsigned*>(region)[lane] = 0u;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < W * NS; ++s) mbar_init(reinterpret_cast<uint64_t*>(smem) + s, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  pdl_enter();
+  if (a.one.done && *a.one.done) return;
+  const StripSlot& S = a.one;
+  int st = 0, ph = 0;  // stage and phase of the next chunk this warp takes
+  for (;;) {
+    if (compute && lane == 0) {
+      *delivered = 0;
+      *consumed = 0;
+    }
+    if (threadIdx.x == 0) s_ticket = atomicAdd(a.ticket, 1);
+    __syncthreads();
+    const int r = s_ticket * W + w;
+    if (s_ticket * W >= S.nstrips) break;
+    if (r < S.nstrips) {
+      if (!compute) {
+        receive<T, B, RW == 32 ? 4 : 2>(S, r, region + kStripZero + kStripRing * RW * VS, delivered, consumed, a.err, lane);
+      } else {
+        const int c0 = S.strip_chunk[r], nch = S.strip_chunk[r + 1] - c0;
+        const unsigned char* rec = S.rec + (size_t)c0 * D.chunk_bytes;
+        const unsigned char* in = reinterpret_cast<const unsigned char*>(S.in) + (size_t)c0 * RHS_CHUNK;
+        auto issue = [&](int c, int s) {  // lane 0: chunk c into stage s
+          mbar_expect_tx(&full[s], D.chunk_bytes + RHS_CHUNK);
+          tma_load_1d(rstage + (size_t)s * D.chunk_bytes, rec + (size_t)c * D.chunk_bytes, D.chunk_bytes, &full[s]);
+          tma_load_1d(vstage + (size_t)s * RHS_CHUNK, in + (size_t)c * RHS_CHUNK, RHS_CHUNK, &full[s]);
+        };
+        const int lr = lane / LPR, p = lane - lr * LPR;  // row of the step, component (LPR > 1)
+        const int st0 = st, ph0 = ph;
+        int issued = min(NS, nch);
+        if (lane == 0)
+          for (int c = 0, s = st; c < issued; ++c) {
+            issue(c, s);
+            if (++s == NS) s = 0;
+          }
+        T* out = reinterpret_cast<T*>(S.out) + p;
+        T* xch = reinterpret_cast<T*>(S.xch) + p;
+        // one step's data, loaded a step ahead of its use; the addresses taken
+        // from its metadata are worked out a step ahead too (the empty asm
+        // statements keep them there), so that after the __syncwarp only the
+        // loads themselves are left on the chain
+        int4 meta[MC];
+        Vec<T, PER16> val[2][VC];
+        T t[2][LPR == 1 ? B : 1];
+        unsigned cd[2][NE];
+        int o[2], xs[2];
+        T *op[2], *xp[2];
+        auto load = [&](int k, const unsigned char* sp, const unsigned char* vp) {
+#pragma unroll
+          for (int j = 0; j < MC; ++j) meta[j] = *reinterpret_cast<const int4*>(sp + j * 512);
+#pragma unroll
+          for (int j = 0; j < VC; ++j) val[k][j] = *reinterpret_cast<const Vec<T, PER16>*>(sp + (MC + j) * 512);
+          const T* rh = reinterpret_cast<const T*>(vp);
+          if constexpr (LPR == 1) {
+#pragma unroll
+            for (int d = 0; d < B; ++d) t[k][d] = rh[lane * B + d];
+          } else {
+            t[k][0] = rh[lane];
+          }
+        };
+        auto decode = [&](int k) {
+          auto mint = [&](int i) -> int {
+            return (i & 3) == 0 ? meta[i / 4].x : (i & 3) == 1 ? meta[i / 4].y : (i & 3) == 2 ? meta[i / 4].z : meta[i / 4].w;
+          };
+#pragma unroll
+          for (int e = 0; e < NE; ++e) {
+            cd[k][e] = (e & 1) ? (unsigned)mint(e / 2) >> 16 : (unsigned)mint(e / 2) & 0xffffu;
+            asm volatile("" : "+r"(cd[k][e]));
+          }
+          o[k] = mint((NE + 1) / 2);
+          xs[k] = mint((NE + 1) / 2 + 1);
+          op[k] = out + (long long)o[k] * B;
+          xp[k] = xch + (long long)xs[k] * BP;
+          asm volatile("" : "+l"(op[k]), "+l"(xp[k]));
+        };
+        T* const ring0 = reinterpret_cast<T*>(region + kStripZero) + lr * BP;
+        bool abort = !__all_sync(0xffffffffu, mbar_wait(&full[st], (unsigned)ph, a.err, kSiteFull, -1, r));
+        int waited = abort ? 0 : 1, have = 0;
+        const unsigned char* sp = rstage + (size_t)st * D.chunk_bytes + kStripHdr + lane * 16;
+        const unsigned char* vp = vstage + (size_t)st * RHS_CHUNK;
+        if (!abort) {
+          load(0, sp, vp);
+          decode(0);
+        }
+        for (int c = 0; c < nch && !abort; ++c) {
+          int need[CH];
+#pragma unroll
+          for (int j = G - 1; j < CH; j += G) need[j] = reinterpret_cast<const int*>(sp - kStripHdr - lane * 16)[j];
+          T* rg = ring0 + (c * CH % kStripRing) * RW * BP;
+          int st1 = st + 1, ph1 = ph;
+          if (st1 == NS) { st1 = 0; ph1 ^= 1; }
+          const unsigned char* sp1 = rstage + (size_t)st1 * D.chunk_bytes + kStripHdr + lane * 16;
+          const unsigned char* vp1 = vstage + (size_t)st1 * RHS_CHUNK;
+#pragma unroll
+          for (int j = 0; j < CH; ++j) {
+            if (j % G == 0 && need[j + G - 1] > have) {  // every lane reads the same count
+              long long t0 = 0;
+              for (unsigned n = 1; (have = ld_acquire_s(delivered)) < need[j + G - 1]; ++n) {
+                if ((n & 255) == 0) {
+                  if (n == 256) t0 = clock64();
+                  const bool late = clock64() - t0 > kWaitCycles;
+                  if (late && lane == 0) record_fail(a.err, kErrTimeout, kSitePoll, -1, r);
+                  if (__any_sync(0xffffffffu, late || ld_relaxed_int(a.err) != 0)) {
+                    abort = true;
+                    break;
+                  }
+                }
+              }
+              have = __shfl_sync(0xffffffffu, have, 0);
+              if (abort) break;
+            }
+            constexpr int K2 = 2;
+            const int k = j % K2;
+            auto A = [&](int i) -> T { return val[k][i / PER16].v[i % PER16]; };
+            // dependency values
+            Vec<T, BP> x[NE];
+#pragma unroll
+            for (int e = 0; e < NE; ++e) {
+              x[e] = *reinterpret_cast<const Vec<T, BP>*>(reinterpret_cast<const float*>(smem) + cd[k][e]);
+            }
+            // the next step's data
+            const bool more = j + 1 < CH || c + 1 < nch;
+            if (j + 1 < CH) {
+              load((j + 1) % K2, sp + (j + 1) * D.step_bytes, vp + (j + 1) * D.rhs_bytes);
+            } else if (c + 1 < nch) {
+              if (!__all_sync(0xffffffffu, mbar_wait(&full[st1], (unsigned)ph1, a.err, kSiteFull, -1, r))) {
+                abort = true;
+                break;
+              }
+              ++waited;
+              load(0, sp1, vp1);
+            }
+            // the rows
+            if constexpr (LPR == 1) {
+              T acc[B];
+#pragma unroll
+              for (int d = 0; d < B; ++d) acc[d] = t[k][d];
+#pragma unroll
+              for (int e = 0; e < NE; ++e)
+#pragma unroll
+                for (int d = 0; d < B; ++d)
+#pragma unroll
+                  for (int q = 0; q < B; ++q) acc[d] -= A(e * EV + d * B + q) * x[e].v[q];
+              Vec<T, BP> y;
+#pragma unroll
+              for (int d = 0; d < B; ++d) {
+                if constexpr (FWD) {
+                  T u = A(NE * EV + d * B) * acc[0];
+#pragma unroll
+                  for (int q = 1; q < B; ++q) u += A(NE * EV + d * B + q) * acc[q];
+                  y.v[d] = u;
+                } else {
+                  y.v[d] = acc[d];
+                }
+              }
+              *reinterpret_cast<Vec<T, BP>*>(rg + j * RW * BP) = y;
+              if (more) decode((j + 1) % K2);
+              xstore(xs[k], xp[k], y);
+              ostore(o[k], op[k], y);
+            } else {
+              T acc = t[k][0];
+#pragma unroll
+              for (int e = 0; e < NE; ++e)
+#pragma unroll
+                for (int q = 0; q < B; ++q) acc -= A(e * EV + q) * x[e].v[q];
+              if constexpr (FWD) {
+                const int l0 = lane - p;
+                T y = A(NE * EV) * __shfl_sync(0xffffffffu, acc, l0);
+#pragma unroll
+                for (int q = 1; q < B; ++q) {
+                  const T tq = __shfl_sync(0xffffffffu, acc, l0 + q);
+                  y += A(NE * EV + q) * tq;
+                }
+                acc = y;
+              }
+              if (lr < RW) rg[j * RW * BP + p] = acc;
+              const Vec<T, 1> y1{{acc}};
+              if (more) decode((j + 1) % K2);
+              xstore(xs[k], xp[k], y1);
+              ostore(o[k], op[k], y1);
+            }
+            __syncwarp();
+          }
+          if (abort) break;
+          // the chunk is through: its stage takes the next copy
+          if (lane == 0) {
+            st_release_s(consumed, (c + 1) * CH);
+            if (issued < nch) issue(issued, st);
+          }
+          if (issued < nch) ++issued;
+          st = st1;
+          ph = ph1;
+          sp = sp1;
+          vp = vp1;
+        }
+        if (abort && lane == 0) {  // copies in flight land before the CTA leaves (bounded)
+          record_fail(a.err, kErrTimeout, kSiteRange, -1, r);
+          for (int k = waited; k < issued; ++k) mbar_drain(&full[(st0 + k) % NS], (unsigned)(ph0 ^ ((st0 + k) / NS & 1)));
+        }
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) s_stop = ld_relaxed_int(a.err) != 0;
+    __syncthreads();
+    if (s_stop) break;
+  }
+}
+
+// ------------------------------------------------------------------ records
+
+__global__ void k_strip_meta(int CH, int MC, int step_bytes, int chunk_bytes, const int* __restrict__ meta,
+                             const int* __restrict__ need, unsigned char* rec) {
+  unsigned char* ck = rec + (size_t)blockIdx.x * chunk_bytes;
+  if (threadIdx.x < kStripHdr / 4)
+    reinterpret_cast<int*>(ck)[threadIdx.x] = (int)threadIdx.x < CH ? need[(size_t)blockIdx.x * CH + threadIdx.x] : 0;
+  const int per = MC * 32;  // pieces per step
+  const int4* m = reinterpret_cast<const int4*>(meta) + (size_t)blockIdx.x * CH * per;
+  for (int i = threadIdx.x; i < CH * per; i += blockDim.x)
+    reinterpret_cast<int4*>(ck + kStripHdr + (size_t)(i / per) * step_bytes)[i % per] = m[i];
+}
+
+// one block per step: value k of lane l in piece k / (16 / sizeof(T))
+template <typename T, int B, bool FWD>
+__global__ void k_strip_pack(StripPackArgs a) {
+  constexpr int SZ = (int)sizeof(T), PER16 = 16 / SZ, LPR = strip_lpr(B, SZ), BS = B * B;
+  constexpr int EV = B * (LPR == 1 ? B : 1);
+  const long long s = blockIdx.x;
+  const int RW = a.d.RW, ne = a.ne;
+  T* v = reinterpret_cast<T*>(a.rec + (size_t)(s / a.d.CH) * a.d.chunk_bytes + kStripHdr +
+                              (size_t)(s % a.d.CH) * a.d.step_bytes + (size_t)a.d.MC * 512);
+  for (int i = threadIdx.x; i < a.d.VC * 32 * PER16; i += blockDim.x) {
+    const int lane = (i / PER16) & 31, k = (i / PER16 / 32) * PER16 + i % PER16;
+    const int l = lane / LPR, p = lane - l * LPR, e = k / EV, q = k - e * EV;
+    double x = 0.0;
+    if (l < RW) {
+      const int m = LPR == 1 ? q : p * B + q;
+      if (e < ne) {
+        const int c = a.ent_slot[((size_t)s * RW + l) * ne + e];
+        if (c >= 0) x = a.foffd[(size_t)c * BS + m];
+      } else if (FWD && e == ne) {
+        const int row = a.step_rows[(size_t)s * RW + l];
+        if (row >= 0) x = a.fdiag[(size_t)row * BS + m];
+      }
+    }
+    v[i] = (T)x;
+  }
+}
+
+// ------------------------------------------------------------------ launchers
+
+cudaError_t launch_strip_meta(const StripDims& d, int nchunks, const int* meta, const int* need, unsigned char* rec,
+                              cudaStream_t st) {
+  if (nchunks <= 0) return cudaSuccess;
+  k_strip_meta<<<nchunks, 128, 0, st>>>(d.CH, d.MC, d.step_bytes, d.chunk_bytes, meta, need, rec);
+  return cudaGetLastError();
+}
+
+template <typename T, bool FWD>
+static cudaError_t pack_t(const StripPackArgs& a, cudaStream_t st) {
+  if (a.nsteps <= 0) return cudaSuccess;
+  switch (a.b) {
+    case 1: k_strip_pack<T, 1, FWD><<<(unsigned)a.nsteps, 128, 0, st>>>(a); break;
+    case 2: k_strip_pack<T, 2, FWD><<<(unsigned)a.nsteps, 128, 0, st>>>(a); break;
+    case 3: k_strip_pack<T, 3, FWD><<<(unsigned)a.nsteps, 128, 0, st>>>(a); break;
+    default: return cudaErrorInvalidValue;
+  }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_strip_pack(bool forward, bool fp32, const StripPackArgs& a, cudaStream_t st) {
+  if (fp32) return forward ? pack_t<float, true>(a, st) : pack_t<float, false>(a, st);
+  return forward ? pack_t<double, true>(a, st) : pack_t<double, false>(a, st);
+}
+
+// calls f(kernel) for the instance of (fp32, b, forward, ne)
+template <typename F>
+static cudaError_t with_kernel(bool fp32, int b, bool forward, int ne, F&& f) {
+#define DFG_STRIP_NE(T, B, FWD)                   switch (ne) {                                     case 3: return f(k_strip<T, B, FWD, 3>);        case 4: return f(k_strip<T, B, FWD, 4>);        case 7: return f(k_strip<T, B, FWD, 7>);        case 16: return f(k_strip<T, B, FWD, 16>);      default: return cudaErrorInvalidValue;        }
+#define DFG_STRIP_B(B)                                                                    if (fp32) {                                                                               if (forward) { DFG_STRIP_NE(float, B, true) } else { DFG_STRIP_NE(float, B, false) }   } else {                                                                                  if (forward) { DFG_STRIP_NE(double, B, true) } else { DFG_STRIP_NE(double, B, false) }   }
+  switch (b) {
+    case 1: DFG_STRIP_B(1)
+    case 2: DFG_STRIP_B(2)
+    case 3: DFG_STRIP_B(3)
+    default: return cudaErrorInvalidValue;
+  }
+#undef DFG_STRIP_B
+#undef DFG_STRIP_NE
+}
+
+cudaError_t launch_strip(bool forward, bool fp32, int b, const StripArgs& a, int grid, size_t smem, cudaStream_t st,
+                         bool dep) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(64 * a.W);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = dep ? 1 : 0;
+  return with_kernel(fp32, b, forward, a.ne, [&](auto k) { return cudaLaunchKernelEx(&cfg, k, a); });
+}
+
+cudaError_t strip_set_smem_limits(size_t max_smem) {
+  for (int fp32 = 0; fp32 < 2; ++fp32)
+    for (int b = 1; b <= 3; ++b)
+      for (int fwd = 0; fwd < 2; ++fwd)
+        for (int ne : {3, 4, 7, 16}) {
+          const cudaError_t e = with_kernel(fp32, b, fwd, ne, [&](auto k) {
+            return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem);
+          });
+          if (e != cudaSuccess) return e;
+        }
+  return cudaSuccess;
+}
+
+}  // namespace dfg

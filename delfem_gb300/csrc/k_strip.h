@@ -1,0 +1,144 @@
+// k_strip.h -- plan and launch interface of the strip sweeps (k_strip.cu,
+// plans in strip.cpp).
+#pragma once
+#include <cuda_runtime.h>
+
+#include <cstddef>
+#include <vector>
+
+namespace dfg {
+
+// A strip is a run of consecutive rows (in sweep order) whose rows, grouped
+// by their dependency level inside the strip, number at most RW per level:
+// up to RW grid lines of a structured mesh.  One warp sweeps a strip, one
+// level ("step") at a time.
+//
+// Shapes that follow from the block size, the element size, the direction and
+// the entry class (entries per row: 3, 4, 7 or 16).
+struct StripDims {
+  int LPR;     // lanes per row: 1, or b (lane = one component of a row)
+  int RW;      // rows per step
+  int MC;      // 16-byte pieces of metadata per lane and step
+  int VC;      // 16-byte pieces of factor values per lane and step
+  int CH;      // steps per chunk (the unit copied into shared memory)
+  int VS;      // bytes of one row's value in the ring, the mailbox and the exchange buffer
+  int step_bytes, rhs_bytes, chunk_bytes;
+};
+constexpr int kStripHdr = 32;    // bytes before a chunk's steps: CH counts of mailbox items needed
+constexpr int kStripRing = 32;   // ring depth in steps
+constexpr int kStripZero = 32;   // zero bytes at the start of a warp's value region (padding entries)
+constexpr int kStripMaxWarps = 4;
+
+// Lanes per row.  An FP64 step costs 64 cycles of its scheduler per
+// warp-wide FMA whatever the number of active lanes, and a 3x3 row 63 FMAs in
+// one lane: there each component of a row takes its own lane, which divides
+// the step's chain by b.  FP32 2x2 rows stay in one lane (16 FMAs): two lanes
+// per row would halve the rows of a strip and double the hand-offs between
+// strips.
+__host__ __device__ constexpr int strip_lpr(int b, int elem) { return b == 3 ? 3 : (b == 2 && elem == 8) ? 2 : 1; }
+__host__ __device__ constexpr StripDims strip_dims(int b, int elem, bool forward, int ne) {
+  StripDims d{};
+  d.LPR = strip_lpr(b, elem);
+  d.RW = 32 / d.LPR;
+  d.MC = ((ne + 1) / 2 + 2 + 3) / 4;
+  const int per_lane = (ne + (forward ? 1 : 0)) * b * (d.LPR == 1 ? b : 1);
+  d.VC = (per_lane * elem + 15) / 16;
+  d.VS = (b == 3 ? 4 : b) * elem;
+  d.step_bytes = 512 * (d.MC + d.VC);
+  d.rhs_bytes = d.RW * b * elem;
+  d.CH = d.step_bytes <= 2048 ? 8 : d.step_bytes <= 6144 ? 4 : 2;
+  d.chunk_bytes = kStripHdr + d.CH * d.step_bytes;
+  return d;
+}
+// entry class of rows with at most `maxe` entries; 0 = too many
+inline int strip_class(int maxe) { return maxe <= 3 ? 3 : maxe <= 4 ? 4 : maxe <= 7 ? 7 : maxe <= 16 ? 16 : 0; }
+// mailbox slots per warp: enough for the items of several chunks, 8-16 KB
+__host__ __device__ constexpr int strip_mailbox(int VS) { return VS <= 8 ? 1024 : 512; }
+
+// Steps are numbered with every strip padded to whole chunks: step s lies in
+// chunk s / CH.  pos[row] = s * RW + row's place in the step is the row's
+// place in the sweep's "step order", the order of its input.
+struct StripPlan {
+  bool forward = true;
+  int n = 0, b = 1, elem = 8, ne = 0, nstrips = 0, nchunks = 0, nexport = 0;
+  StripDims d{};
+  std::vector<int> strip_chunk;  // nstrips + 1: first chunk
+  std::vector<int> strip_steps;  // nstrips: steps that hold rows
+  std::vector<int> item_ptr;     // nstrips + 1
+  std::vector<int> items;        // per item {exchange slot, step at which its mailbox slot is free}
+  std::vector<int> pos;          // n
+  std::vector<int> need;         // nchunks * CH: mailbox items a step needs delivered
+  std::vector<int> step_rows;    // nchunks * CH * RW, -1 = empty
+  std::vector<int> ent_slot;     // nchunks * CH * RW * ne: CRS slot of the block, -1 = padding
+  std::vector<int> codes;        // same shape: byte offset into the warp's value region
+  std::vector<int> exports;      // nchunks * CH * RW: exchange slot of the row, -1 = none
+  long long steps() const { return (long long)nchunks * d.CH; }
+};
+__host__ __device__ constexpr size_t strip_up128(size_t v) { return (v + 127) / 128 * 128; }
+// A warp's value region: zero bytes, ring, mailbox.
+__host__ __device__ constexpr size_t strip_region_bytes(const StripDims& d) {
+  return strip_up128(kStripZero + (size_t)kStripRing * d.RW * d.VS + (size_t)strip_mailbox(d.VS) * d.VS);
+}
+__host__ __device__ constexpr size_t strip_stage_bytes(const StripDims& d, int NS) {
+  return strip_up128((size_t)NS * (d.chunk_bytes + d.CH * d.rhs_bytes) + 16);
+}
+// Shared memory: the chunk barriers and two progress words of every warp, then
+// per warp its stages and its region.
+__host__ __device__ constexpr size_t strip_stage_offset(const StripDims& d, int W, int NS, int w) {
+  return strip_up128((size_t)W * NS * 8 + (size_t)W * 16) + w * (strip_stage_bytes(d, NS) + strip_region_bytes(d));
+}
+__host__ __device__ constexpr size_t strip_region_offset(const StripDims& d, int W, int NS, int w) {
+  return strip_stage_offset(d, W, NS, w) + strip_stage_bytes(d, NS);
+}
+inline size_t strip_smem_bytes(const StripDims& d, int W, int NS) { return strip_stage_offset(d, W, NS, W); }
+// False when the rows do not fit the sweep: more than 16 entries in a row, or
+// more dependencies on other strips within a chunk than the mailbox holds.
+bool strip_plan(int n, int b, int elem, const int* rowptr, const int* colind, const int* diaind, bool forward,
+                StripPlan& P);
+// Metadata of every step and lane as the records hold it ([step][piece][lane]
+// of 4 ints): ne 16-bit codes (offset / 4 from the start of the CTA's dynamic
+// shared memory, for W warps of NS stages each), then the output position (-1:
+// empty lane) and the exchange slot (-1: none).  out_pos[row]: where the row's
+// result goes.
+std::vector<int> strip_meta(const StripPlan& P, const int* out_pos, int W, int NS);
+
+// One solve's sweep.
+struct StripSlot {
+  const unsigned char* rec;  // chunks
+  const int* strip_chunk;
+  const int* item_ptr;
+  const int2* items;
+  const void* in;            // right-hand sides in step order
+  void* out;
+  void* xch;                 // exchange buffer, sentinel-filled before the sweep
+  const int* done;           // optional: nonzero = skip
+  int nstrips;
+};
+struct StripArgs {
+  StripSlot one;
+  int* ticket;   // 0 at launch
+  int* err;      // device error word
+  int ne;        // entry class
+  int W;         // strips (compute warps) per CTA
+  int NS;        // chunk stages per warp
+};
+cudaError_t launch_strip(bool forward, bool fp32, int b, const StripArgs& a, int grid, size_t smem, cudaStream_t st,
+                         bool dep);
+cudaError_t strip_set_smem_limits(size_t max_smem);
+// places the metadata and the item counts into the records (once per plan)
+cudaError_t launch_strip_meta(const StripDims& d, int nchunks, const int* meta, const int* need, unsigned char* rec,
+                              cudaStream_t st);
+// fills the records' values from the factor
+struct StripPackArgs {
+  StripDims d;
+  int ne, b;
+  long long nsteps;
+  unsigned char* rec;
+  const int* ent_slot;
+  const int* step_rows;
+  const double* fdiag;
+  const double* foffd;
+};
+cudaError_t launch_strip_pack(bool forward, bool fp32, const StripPackArgs& a, cudaStream_t st);
+
+}  // namespace dfg
