@@ -12,22 +12,23 @@
 // memory ahead of it:
 //   * the step records (dependency codes, factor blocks, output positions) and
 //     the right-hand sides, both contiguous in step order, by two TMA bulk
-//     copies per chunk of steps, issued by the warp itself NS chunks ahead (it
-//     frees a stage by finishing it, so no barrier with a producer);
+//     copies per chunk of steps, NS chunks ahead, from a loader warp (issuing
+//     them takes 230 cycles, which the compute warp paid per chunk before);
 //   * the values of other strips by a receiver warp beside each compute warp.
 //     A row that another strip needs is also written to an exchange buffer in
 //     global memory that was filled with a NaN sentinel; the receiver's lanes
-//     poll the strip's items, listed in the order of first use, four each in
+//     poll the strip's items, listed in the order of first use, a few each in
 //     flight, and put them into the warp's mailbox (a ring of slots) as they
 //     arrive.  `delivered` counts the arrived prefix; a step says how many
 //     items it needs, one compare when they are there.
 // Measured on GB300, FP32, per sweep (forward / backward): the 1000x500
-// cantilever 0.21 / 0.16 ms (ranged kernel 1.09 / 1.10), Poisson on 301x257
-// cells 63 / 62 us (one CTA per sweep 200 / 196), elasticity on 56^3 cells 136 /
-// 127 us (a launch per level 345 / 306).  FP64: the cantilever 0.70 / 0.51 ms
-// (2.36 / 2.08), Poisson on 128x128 cells 71 / 63 us (133 / 123).  Inside one
-// strip a level costs 165 cycles (1x1 blocks, FP32) to 820 (2x2, FP64); a
-// hand-off between strips about 3,000, of which the L2 takes 600-900.
+// cantilever 0.15 / 0.14 ms (ranged kernel 1.09 / 1.10), Poisson on 301x257
+// cells 49 / 46 us (one CTA per sweep 200 / 196), elasticity on 56^3 cells 107 /
+// 100 us (a launch per level 345 / 306).  FP64: the cantilever 0.65 / 0.50 ms
+// (2.36 / 2.08), Poisson on 128x128 cells 69 / 59 us (133 / 123).  Inside one
+// strip a level costs 115 (1x1 blocks) to 400 (3x3, 7 entries) cycles in FP32
+// and 420 to 2,100 in FP64, where each warp-wide FMA takes its scheduler 64; a
+// hand-off between strips costs 1,500 to 3,000, of which the L2 takes 600-900.
 //
 // Strips are claimed in order, W per CTA, through a ticket, so a strip only
 // waits on strips already running, whatever the number of resident CTAs.
@@ -119,7 +120,10 @@ __device__ __forceinline__ void ostore(int on, float* p, const Vec<float, 2>& y)
 
 // The receiver of one strip: polls its items in the exchange buffer and
 // delivers them to the mailbox in order.  Two sets of H batches of 32 items are
-// in flight; a set that is through makes room for the next one.
+// in flight; a set that is through makes room for the next one.  More in flight
+// slow everyone's polls down (3D elasticity, 56^3 FP64: 251 us per sweep with
+// H = 1, 265 with 2, 309 with 4), fewer starve short steps (3D Poisson, 44^3
+// FP32: 47, 41 and 45 us).
 template <typename T, int B, int H>
 __device__ __forceinline__ void receive(const StripSlot& S, int r, unsigned char* mail, int* delivered,
                                         const int* consumed, int* err, int lane) {
@@ -138,6 +142,7 @@ __device__ __forceinline__ void receive(const StripSlot& S, int r, unsigned char
 #pragma unroll
   for (int u = 0; u < H; ++u) nxt[u] = item((U + u) * 32 + lane);
   int base = 0;
+  bool started = false;  // until the first item is there it is polled alone: a strip far from the front leaves the L2 to the others
   long long t0 = clock64();
   for (unsigned n = 1; base < cnt; ++n) {
     if ((n & 63) == 0) {
@@ -153,7 +158,7 @@ __device__ __forceinline__ void receive(const StripSlot& S, int r, unsigned char
     for (int u = 0; u < U; ++u) {
 #pragma unroll
       for (int d = 0; d < BP; ++d) v[u].v[d] = sentinel_value<T>();
-      xload(!(got >> u & 1) && base + u * 32 + lane < cnt && it[u].y <= done_steps, xch + (size_t)it[u].x * BP, v[u]);
+      xload(!(got >> u & 1) && base + u * 32 + lane < cnt && it[u].y <= done_steps && (started || (u == 0 && lane == 0)), xch + (size_t)it[u].x * BP, v[u]);
     }
     const unsigned had = got;
 #pragma unroll
@@ -166,6 +171,7 @@ __device__ __forceinline__ void receive(const StripSlot& S, int r, unsigned char
     }
     if (!__any_sync(0xffffffffu, got != had)) continue;
     t0 = clock64();
+    started = true;
     // the delivered prefix over the batches in flight
     int pre = base;
     bool whole = true;
@@ -193,7 +199,7 @@ __device__ __forceinline__ void receive(const StripSlot& S, int r, unsigned char
 }
 
 template <typename T, int B, bool FWD, int NE>
-__global__ void __launch_bounds__(2 * kStripMaxWarps * 32) k_strip(StripArgs a) {
+__global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32) k_strip(StripArgs a) {
   constexpr int SZ = (int)sizeof(T);
   constexpr StripDims D = strip_dims(B, SZ, FWD, NE);
   constexpr int LPR = D.LPR, RW = D.RW, MC = D.MC, VC = D.VC, CH = D.CH, VS = D.VS;
@@ -204,13 +210,16 @@ __global__ void __launch_bounds__(2 * kStripMaxWarps * 32) k_strip(StripArgs a) 
   // steps per test of the mailbox: short steps share one (a test is a branch,
   // about 10 cycles, and waiting for the last of four steps' items costs a
   // hand-off three steps)
+  // values are loaded a step ahead where two sets of them fit the registers
+  constexpr int VB = VC <= 8 ? 2 : 1;
+  constexpr int HB = B == 3 ? 1 : 2;
   constexpr int G = NE <= 4 && CH >= 4 ? 4 : 1;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ int s_ticket, s_stop;
   const int W = a.W, NS = a.NS;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool compute = warp < W;
-  const int w = compute ? warp : warp - W;
+  const bool compute = warp < W, load_warp = warp == 2 * W;
+  const int w = compute ? warp : load_warp ? min(lane, W - 1) : warp - W;  // (the loader's lane w serves warp w)
   uint64_t* full = reinterpret_cast<uint64_t*>(smem) + w * NS;
   int* delivered = reinterpret_cast<int*>(smem + (size_t)W * NS * 8) + w * 4;
   int* consumed = delivered + 1;
@@ -225,8 +234,9 @@ __global__ void __launch_bounds__(2 * kStripMaxWarps * 32) k_strip(StripArgs a) 
   pdl_enter();
   if (a.one.done && *a.one.done) return;
   const StripSlot& S = a.one;
-  int st = 0, ph = 0;  // stage and phase of the next chunk this warp takes
+  int st = 0, ph = 0;  // stage and phase of the strip's next chunk (compute warps and loader alike)
   for (;;) {
+    int issued = 0;  // loader: chunks of the strip issued
     if (compute && lane == 0) {
       *delivered = 0;
       *consumed = 0;
@@ -235,26 +245,37 @@ __global__ void __launch_bounds__(2 * kStripMaxWarps * 32) k_strip(StripArgs a) 
     __syncthreads();
     const int r = s_ticket * W + w;
     if (s_ticket * W >= S.nstrips) break;
-    if (r < S.nstrips) {
-      if (!compute) {
-        receive<T, B, RW == 32 ? 4 : 2>(S, r, region + kStripZero + kStripRing * RW * VS, delivered, consumed, a.err, lane);
-      } else {
-        const int c0 = S.strip_chunk[r], nch = S.strip_chunk[r + 1] - c0;
-        const unsigned char* rec = S.rec + (size_t)c0 * D.chunk_bytes;
-        const unsigned char* in = reinterpret_cast<const unsigned char*>(S.in) + (size_t)c0 * RHS_CHUNK;
-        auto issue = [&](int c, int s) {  // lane 0: chunk c into stage s
-          mbar_expect_tx(&full[s], D.chunk_bytes + RHS_CHUNK);
-          tma_load_1d(rstage + (size_t)s * D.chunk_bytes, rec + (size_t)c * D.chunk_bytes, D.chunk_bytes, &full[s]);
-          tma_load_1d(vstage + (size_t)s * RHS_CHUNK, in + (size_t)c * RHS_CHUNK, RHS_CHUNK, &full[s]);
-        };
-        const int lr = lane / LPR, p = lane - lr * LPR;  // row of the step, component (LPR > 1)
-        const int st0 = st, ph0 = ph;
-        int issued = min(NS, nch);
-        if (lane == 0)
-          for (int c = 0, s = st; c < issued; ++c) {
-            issue(c, s);
-            if (++s == NS) s = 0;
+    if (load_warp) {
+      // -------------------------------------------------------------- loader
+      // lane w keeps warp w's stages filled: a chunk's records and its
+      // right-hand sides, NS chunks ahead of the chunks the warp has finished
+      const bool on = lane < W && r < S.nstrips;
+      const int c0 = on ? S.strip_chunk[r] : 0, nch = on ? S.strip_chunk[r + 1] - c0 : 0;
+      const unsigned char* rec = S.rec + (size_t)c0 * D.chunk_bytes;
+      const unsigned char* in = reinterpret_cast<const unsigned char*>(S.in) + (size_t)c0 * RHS_CHUNK;
+      bool failing = false;
+      for (unsigned n = 1; __any_sync(0xffffffffu, issued < nch && !failing); ++n) {
+        if (issued < nch && !failing) {
+          const int done = ld_acquire_s(consumed) / CH;
+          for (; issued < min(nch, done + NS); ++issued) {
+            const int s = (st + issued) % NS;
+            mbar_expect_tx(&full[s], D.chunk_bytes + RHS_CHUNK);
+            tma_load_1d(rstage + (size_t)s * D.chunk_bytes, rec, D.chunk_bytes, &full[s]);
+            tma_load_1d(vstage + (size_t)s * RHS_CHUNK, in, RHS_CHUNK, &full[s]);
+            rec += D.chunk_bytes;
+            in += RHS_CHUNK;
           }
+          if ((n & 63) == 0) failing = ld_relaxed_int(a.err) != 0;
+        }
+        __nanosleep(64);
+      }
+    } else if (r < S.nstrips) {
+      if (!compute) {
+        receive<T, B, HB>(S, r, region + kStripZero + kStripRing * RW * VS, delivered, consumed, a.err, lane);
+      } else {
+        // ------------------------------------------------------------- compute
+        const int c0 = S.strip_chunk[r], nch = S.strip_chunk[r + 1] - c0;
+        const int lr = lane / LPR, p = lane - lr * LPR;  // row of the step, component (LPR > 1)
         T* out = reinterpret_cast<T*>(S.out) + p;
         T* xch = reinterpret_cast<T*>(S.xch) + p;
         // one step's data, loaded a step ahead of its use; the addresses taken
@@ -262,7 +283,7 @@ __global__ void __launch_bounds__(2 * kStripMaxWarps * 32) k_strip(StripArgs a) 
         // statements keep them there), so that after the __syncwarp only the
         // loads themselves are left on the chain
         int4 meta[MC];
-        Vec<T, PER16> val[2][VC];
+        Vec<T, PER16> val[VB][VC];
         T t[2][LPR == 1 ? B : 1];
         unsigned cd[2][NE];
         int o[2], xs[2];
@@ -271,7 +292,8 @@ __global__ void __launch_bounds__(2 * kStripMaxWarps * 32) k_strip(StripArgs a) 
 #pragma unroll
           for (int j = 0; j < MC; ++j) meta[j] = *reinterpret_cast<const int4*>(sp + j * 512);
 #pragma unroll
-          for (int j = 0; j < VC; ++j) val[k][j] = *reinterpret_cast<const Vec<T, PER16>*>(sp + (MC + j) * 512);
+          for (int j = 0; j < VC; ++j)
+            if (VB == 2) val[k % VB][j] = *reinterpret_cast<const Vec<T, PER16>*>(sp + (MC + j) * 512);
           const T* rh = reinterpret_cast<const T*>(vp);
           if constexpr (LPR == 1) {
 #pragma unroll
@@ -296,44 +318,60 @@ __global__ void __launch_bounds__(2 * kStripMaxWarps * 32) k_strip(StripArgs a) 
           asm volatile("" : "+l"(op[k]), "+l"(xp[k]));
         };
         T* const ring0 = reinterpret_cast<T*>(region + kStripZero) + lr * BP;
-        bool abort = !__all_sync(0xffffffffu, mbar_wait(&full[st], (unsigned)ph, a.err, kSiteFull, -1, r));
-        int waited = abort ? 0 : 1, have = 0;
-        const unsigned char* sp = rstage + (size_t)st * D.chunk_bytes + kStripHdr + lane * 16;
-        const unsigned char* vp = vstage + (size_t)st * RHS_CHUNK;
+        bool abort = false;
+        // waits until the progress word reaches `want`; its last value
+        auto wait_for = [&](const int* word, int want, int site) -> int {
+          int v;
+          long long t0 = 0;
+          for (unsigned n = 1; !__all_sync(0xffffffffu, (v = ld_acquire_s(word)) >= want); ++n) {
+            if ((n & 255) == 0) {
+              if (n == 256) t0 = clock64();
+              const bool late = clock64() - t0 > kWaitCycles;
+              if (late && lane == 0) record_fail(a.err, kErrTimeout, site, -1, r);
+              if (__any_sync(0xffffffffu, late || ld_relaxed_int(a.err) != 0)) {
+                abort = true;
+                break;
+              }
+            }
+          }
+          return __shfl_sync(0xffffffffu, v, 0);
+        };
+        abort = !__all_sync(0xffffffffu, mbar_wait(&full[st], (unsigned)ph, a.err, kSiteFull, -1, r));
+        int have = 0;
+        const unsigned char *const sp0 = rstage + kStripHdr + lane * 16, *const vp0 = vstage;
+        const unsigned char *sp = sp0 + (size_t)st * D.chunk_bytes, *vp = vp0 + (size_t)st * RHS_CHUNK;
+        int need[CH];  // (one in G is used)
+        auto load_need = [&](const unsigned char* s) {
+#pragma unroll
+          for (int j = G - 1; j < CH; j += G) need[j] = reinterpret_cast<const int*>(s - kStripHdr - lane * 16)[j];
+        };
         if (!abort) {
           load(0, sp, vp);
           decode(0);
+          load_need(sp);
         }
+        T* rg = ring0;
         for (int c = 0; c < nch && !abort; ++c) {
-          int need[CH];
-#pragma unroll
-          for (int j = G - 1; j < CH; j += G) need[j] = reinterpret_cast<const int*>(sp - kStripHdr - lane * 16)[j];
-          T* rg = ring0 + (c * CH % kStripRing) * RW * BP;
-          int st1 = st + 1, ph1 = ph;
-          if (st1 == NS) { st1 = 0; ph1 ^= 1; }
-          const unsigned char* sp1 = rstage + (size_t)st1 * D.chunk_bytes + kStripHdr + lane * 16;
-          const unsigned char* vp1 = vstage + (size_t)st1 * RHS_CHUNK;
+          if (++st == NS) { st = 0; ph ^= 1; }
+          // the test for the next chunk takes about 100 cycles: asked for here,
+          // looked at in the last step
+          const bool landed = c + 1 < nch && mbar_test_wait(&full[st], (unsigned)ph);
+          const unsigned char* sp1 = st == 0 ? sp0 : sp + D.chunk_bytes;
+          const unsigned char* vp1 = st == 0 ? vp0 : vp + RHS_CHUNK;
 #pragma unroll
           for (int j = 0; j < CH; ++j) {
-            if (j % G == 0 && need[j + G - 1] > have) {  // every lane reads the same count
-              long long t0 = 0;
-              for (unsigned n = 1; (have = ld_acquire_s(delivered)) < need[j + G - 1]; ++n) {
-                if ((n & 255) == 0) {
-                  if (n == 256) t0 = clock64();
-                  const bool late = clock64() - t0 > kWaitCycles;
-                  if (late && lane == 0) record_fail(a.err, kErrTimeout, kSitePoll, -1, r);
-                  if (__any_sync(0xffffffffu, late || ld_relaxed_int(a.err) != 0)) {
-                    abort = true;
-                    break;
-                  }
-                }
-              }
-              have = __shfl_sync(0xffffffffu, have, 0);
+            if (j % G == 0 && need[j + G - 1] > have) {
+              have = wait_for(delivered, need[j + G - 1], kSitePoll);
               if (abort) break;
             }
             constexpr int K2 = 2;
             const int k = j % K2;
-            auto A = [&](int i) -> T { return val[k][i / PER16].v[i % PER16]; };
+            if (VB == 1) {
+#pragma unroll
+              for (int v = 0; v < VC; ++v)
+                val[0][v] = *reinterpret_cast<const Vec<T, PER16>*>(sp + j * D.step_bytes + (MC + v) * 512);
+            }
+            auto A = [&](int i) -> T { return val[k % VB][i / PER16].v[i % PER16]; };
             // dependency values
             Vec<T, BP> x[NE];
 #pragma unroll
@@ -345,13 +383,15 @@ __global__ void __launch_bounds__(2 * kStripMaxWarps * 32) k_strip(StripArgs a) 
             if (j + 1 < CH) {
               load((j + 1) % K2, sp + (j + 1) * D.step_bytes, vp + (j + 1) * D.rhs_bytes);
             } else if (c + 1 < nch) {
-              if (!__all_sync(0xffffffffu, mbar_wait(&full[st1], (unsigned)ph1, a.err, kSiteFull, -1, r))) {
+              if (!__all_sync(0xffffffffu, landed) &&
+                  !__all_sync(0xffffffffu, mbar_wait(&full[st], (unsigned)ph, a.err, kSiteFull, -1, r))) {
                 abort = true;
                 break;
               }
-              ++waited;
               load(0, sp1, vp1);
+              load_need(sp1);
             }
+            if (SZ == 8 && more) decode((j + 1) % K2);
             // the rows
             if constexpr (LPR == 1) {
               T acc[B];
@@ -376,7 +416,7 @@ __global__ void __launch_bounds__(2 * kStripMaxWarps * 32) k_strip(StripArgs a) 
                 }
               }
               *reinterpret_cast<Vec<T, BP>*>(rg + j * RW * BP) = y;
-              if (more) decode((j + 1) % K2);
+              if (SZ == 4 && more) decode((j + 1) % K2);
               xstore(xs[k], xp[k], y);
               ostore(o[k], op[k], y);
             } else {
@@ -397,34 +437,34 @@ __global__ void __launch_bounds__(2 * kStripMaxWarps * 32) k_strip(StripArgs a) 
               }
               if (lr < RW) rg[j * RW * BP + p] = acc;
               const Vec<T, 1> y1{{acc}};
-              if (more) decode((j + 1) % K2);
+              if (SZ == 4 && more) decode((j + 1) % K2);
               xstore(xs[k], xp[k], y1);
               ostore(o[k], op[k], y1);
             }
             __syncwarp();
           }
           if (abort) break;
-          // the chunk is through: its stage takes the next copy
-          if (lane == 0) {
-            st_release_s(consumed, (c + 1) * CH);
-            if (issued < nch) issue(issued, st);
-          }
-          if (issued < nch) ++issued;
-          st = st1;
-          ph = ph1;
+          if (lane == 0) st_release_s(consumed, (c + 1) * CH);  // the chunk's stage is free
           sp = sp1;
           vp = vp1;
+          rg = (c + 1) * CH % kStripRing == 0 ? ring0 : rg + CH * RW * BP;
         }
-        if (abort && lane == 0) {  // copies in flight land before the CTA leaves (bounded)
-          record_fail(a.err, kErrTimeout, kSiteRange, -1, r);
-          for (int k = waited; k < issued; ++k) mbar_drain(&full[(st0 + k) % NS], (unsigned)(ph0 ^ ((st0 + k) / NS & 1)));
-        }
+        if (abort && lane == 0) record_fail(a.err, kErrTimeout, kSiteRange, -1, r);
       }
     }
     __syncthreads();
     if (threadIdx.x == 0) s_stop = ld_relaxed_int(a.err) != 0;
     __syncthreads();
-    if (s_stop) break;
+    if (s_stop) {  // copies in flight land before the CTA leaves (bounded)
+      for (int k = ld_acquire_s(consumed) / CH; k < issued; ++k)
+        mbar_drain(&full[(st + k) % NS], (unsigned)(ph ^ ((st + k) / NS & 1)));
+      break;
+    }
+    if (load_warp && r < S.nstrips) {
+      const int nch = S.strip_chunk[r + 1] - S.strip_chunk[r];
+      ph ^= (st + nch) / NS & 1;
+      st = (st + nch) % NS;
+    }
   }
 }
 
@@ -513,7 +553,7 @@ cudaError_t launch_strip(bool forward, bool fp32, int b, const StripArgs& a, int
                          bool dep) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(64 * a.W);
+  cfg.blockDim = dim3(32 * (2 * a.W + 1));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];

@@ -8,10 +8,11 @@
 
 namespace dfg {
 
-// A strip is a run of consecutive rows (in sweep order) whose rows, grouped
-// by their dependency level inside the strip, number at most RW per level:
-// up to RW grid lines of a structured mesh.  One warp sweeps a strip, one
-// level ("step") at a time.
+// A strip is a set of rows that, grouped by their dependency level inside the
+// strip, number at most RW per level, and whose other dependencies lie in
+// earlier strips: up to RW consecutive grid lines of a structured 2D mesh, a
+// tile of neighbouring lines of neighbouring planes of a 3D one.  One warp
+// sweeps a strip, one level ("step") at a time.
 //
 // Shapes that follow from the block size, the element size, the direction and
 // the entry class (entries per row: 3, 4, 7 or 16).
@@ -46,7 +47,7 @@ __host__ __device__ constexpr StripDims strip_dims(int b, int elem, bool forward
   d.VS = (b == 3 ? 4 : b) * elem;
   d.step_bytes = 512 * (d.MC + d.VC);
   d.rhs_bytes = d.RW * b * elem;
-  d.CH = d.step_bytes <= 2048 ? 8 : d.step_bytes <= 6144 ? 4 : 2;
+  d.CH = d.step_bytes <= 2560 ? 8 : d.step_bytes <= 6144 ? 4 : 2;
   d.chunk_bytes = kStripHdr + d.CH * d.step_bytes;
   return d;
 }

@@ -1,11 +1,139 @@
 // strip.cpp -- host-side plans of the strip sweeps (k_strip.cu): rows into
 // strips and steps, dependencies into ring and mailbox references.
 #include <algorithm>
-#include <cstring>
+#include <cstdlib>
 
 #include "k_strip.h"
 
 namespace dfg {
+
+namespace {
+
+// The rows of a sweep: position p of the sweep order is row p forward, row
+// n-1-p backward; a row's entries point to earlier positions.
+struct Rows {
+  int n;
+  bool forward;
+  const int *rowptr, *colind, *diaind;
+  const int* glev;  // dependency level in the whole sweep
+  int row(int p) const { return forward ? p : n - 1 - p; }
+  int pos(int row) const { return forward ? row : n - 1 - row; }
+  int first(int row) const { return forward ? rowptr[row] : diaind[row]; }
+  int end(int row) const { return forward ? diaind[row] : rowptr[row + 1]; }
+};
+
+// Rows share a step by their level inside the strip.  A row whose level in the
+// whole sweep says that it could run this much earlier, or only this much
+// later, than the rows it would share a step with does not join them.
+constexpr int kDrift = 4;
+
+// Strips of consecutive rows: the row that would be the RW+1st of a level
+// starts the next strip (in a structured mesh the first row of grid line
+// RW+1), and so does a row that has drifted.
+void run_strips(const Rows& R, int RW, std::vector<int>& strip, std::vector<int>& lev, std::vector<int>& lane,
+                std::vector<int>& steps) {
+  steps.clear();
+  std::vector<int> cnt;
+  for (int p = 0; p < R.n;) {
+    const int p0 = p, g0 = R.glev[R.row(p0)];
+    cnt.clear();
+    for (; p < R.n; ++p) {
+      const int row = R.row(p);
+      int lv = 0;
+      for (int c = R.first(row); c < R.end(row); ++c)
+        if (R.pos(R.colind[c]) >= p0) lv = std::max(lv, lev[R.colind[c]] + 1);
+      const int drift = R.glev[row] - lv - g0;
+      if (drift > kDrift || drift < -kDrift) break;
+      if (lv < (int)cnt.size() && cnt[lv] == RW) break;
+      if (lv >= (int)cnt.size()) cnt.resize(lv + 1, 0);
+      lev[row] = lv;
+      lane[row] = cnt[lv]++;
+      strip[row] = (int)steps.size();
+    }
+    steps.push_back((int)cnt.size());
+  }
+}
+
+// Strips that are tiles of grid lines: by neighbouring lines of bz
+// neighbouring planes, by * bz <= RW.  A plane of a 3D mesh handed on plane by
+// plane costs a hand-off per plane; with tiles a dependency chain changes
+// strips once per bz planes and once per by lines.  Lines and planes are read
+// off the dependencies: a row that does not depend on the row before it starts
+// a line, a line none of whose rows depends on the line before it starts a
+// plane.  False when there are no planes, when tiles would not cut the
+// hand-offs, or when some dependency does not respect the tiles' order.
+bool tile_strips(const Rows& R, int RW, std::vector<int>& strip, std::vector<int>& lev, std::vector<int>& lane,
+                 std::vector<int>& steps) {
+  const int n = R.n;
+  std::vector<int> line(n), plane, y;  // line of a position; plane and place in it of a line
+  int nl = 0;
+  bool linked = false;  // the current line depends on the line before it
+  auto close_line = [&] {
+    if (plane.empty() || !linked) {
+      plane.push_back(plane.empty() ? 0 : plane.back() + 1);
+      y.push_back(0);
+    } else {
+      plane.push_back(plane.back());
+      y.push_back(y.back() + 1);
+    }
+    linked = false;
+  };
+  for (int p = 0; p < n; ++p) {
+    const int row = R.row(p);
+    bool next = p > 0;
+    for (int c = R.first(row); c < R.end(row); ++c) next &= R.pos(R.colind[c]) != p - 1;
+    if (next) {
+      close_line();
+      ++nl;
+    }
+    line[p] = nl;
+    for (int c = R.first(row); c < R.end(row); ++c) linked |= line[R.pos(R.colind[c])] == nl - 1;
+  }
+  close_line();
+  ++nl;
+  const int nz = plane.back() + 1;
+  int ny = 0;
+  for (int l = 0; l < nl; ++l) ny = std::max(ny, y[l] + 1);
+  if (nz < 2 || ny < 2) return false;
+  int by = 1, bz = 1, hops = ny + nz;
+  for (int a = 1; a <= std::min(RW, ny); ++a) {
+    const int c = std::min(RW / a, nz), h = (ny + a - 1) / a + (nz + c - 1) / c;
+    if (h < hops || (h == hops && std::abs(a - c) < std::abs(by - bz))) { by = a; bz = c; hops = h; }
+  }
+  if (hops >= nz + (ny + RW - 1) / RW) return false;
+  const int ty = (ny + by - 1) / by, nt = ty * ((nz + bz - 1) / bz);
+  std::vector<std::vector<int>> cnt(nt);
+  std::vector<int> g0(nt, -1);
+  for (int p = 0; p < n; ++p) {
+    const int row = R.row(p), t = plane[line[p]] / bz * ty + y[line[p]] / by;
+    int lv = 0;
+    for (int c = R.first(row); c < R.end(row); ++c) {
+      const int k = R.colind[c];
+      if (strip[k] > t) return false;
+      if (strip[k] == t) lv = std::max(lv, lev[k] + 1);
+    }
+    if (g0[t] < 0) g0[t] = R.glev[row];
+    const int drift = R.glev[row] - lv - g0[t];
+    if (drift > kDrift || drift < -kDrift) return false;
+    if (lv >= (int)cnt[t].size()) cnt[t].resize(lv + 1, 0);
+    if (cnt[t][lv] == RW) return false;
+    lev[row] = lv;
+    lane[row] = cnt[t][lv]++;
+    strip[row] = t;
+  }
+  // tiles without rows (the last planes may be short) are dropped
+  std::vector<int> id(nt, -1);
+  steps.clear();
+  for (int t = 0; t < nt; ++t)
+    if (!cnt[t].empty()) {
+      id[t] = (int)steps.size();
+      steps.push_back((int)cnt[t].size());
+    }
+  for (int i = 0; i < n; ++i) strip[i] = id[strip[i]];
+  return true;
+}
+
+}  // namespace
 
 bool strip_plan(int n, int b, int elem, const int* rowptr, const int* colind, const int* diaind, bool forward,
                 StripPlan& P) {
@@ -24,46 +152,21 @@ bool strip_plan(int n, int b, int elem, const int* rowptr, const int* colind, co
   P.d = strip_dims(b, elem, forward, P.ne);
   const int RW = P.d.RW, CH = P.d.CH, ne = P.ne;
 
-  // strips: rows in order, each at its dependency level inside the strip.  The
-  // row that would be the RW+1st of a level starts the next strip (in a
-  // structured mesh the first row of grid line RW+1), and so does a row whose
-  // level in the whole sweep says that it could run much earlier or only much
-  // later than the rows it would share a step with: the first row of the next
-  // plane of a 3D mesh, which would otherwise wait for the last lines of this
-  // one, plane after plane.
-  constexpr int kDrift = 4;
-  std::vector<int> lev(n), lane(n), strip(n), cnt, glev(n);
+  // level of every row in the whole sweep
+  std::vector<int> glev(n), lev(n), lane(n), strip(n);
   for (int p = 0; p < n; ++p) {
     const int row = row_of(p);
     int lv = 0;
     for (int c = first(row); c < end(row); ++c) lv = std::max(lv, glev[colind[c]] + 1);
     glev[row] = lv;
   }
+  const Rows R{n, forward, rowptr, colind, diaind, glev.data()};
+  std::vector<int> steps;
+  if (!tile_strips(R, RW, strip, lev, lane, steps)) run_strips(R, RW, strip, lev, lane, steps);
+  P.nstrips = (int)steps.size();
+  P.strip_steps = steps;
   P.strip_chunk.push_back(0);
-  for (int p = 0; p < n;) {
-    const int p0 = p;
-    cnt.clear();
-    for (; p < n; ++p) {
-      const int row = row_of(p);
-      int lv = 0;
-      for (int c = first(row); c < end(row); ++c) {
-        const int k = colind[c];
-        if ((forward ? k : n - 1 - k) >= p0) lv = std::max(lv, lev[k] + 1);
-      }
-      const int drift = glev[row] - lv - glev[row_of(p0)];
-      if (drift > kDrift || drift < -kDrift) break;
-      if (lv >= (int)cnt.size()) cnt.resize(lv + 1, 0);
-      if (cnt[lv] == RW) break;
-      lev[row] = lv;
-      lane[row] = cnt[lv]++;
-      strip[row] = P.nstrips;
-    }
-    // a level opened by the row that broke the strip is empty: drop it
-    while (!cnt.empty() && cnt.back() == 0) cnt.pop_back();
-    P.strip_steps.push_back((int)cnt.size());
-    P.strip_chunk.push_back(P.strip_chunk.back() + ((int)cnt.size() + CH - 1) / CH);
-    ++P.nstrips;
-  }
+  for (int r = 0; r < P.nstrips; ++r) P.strip_chunk.push_back(P.strip_chunk.back() + (steps[r] + CH - 1) / CH);
   P.nchunks = P.strip_chunk.back();
   const size_t nsteps = (size_t)P.steps();
   P.pos.resize(n);
