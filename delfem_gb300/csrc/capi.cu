@@ -1607,6 +1607,9 @@ extern "C" int dfg_precond_set_linear_system(dfg_precond prec, dfg_system sys) {
     dalloc(ctx, prec->foffd, (size_t)std::max<long long>(prec->nnz, 1) * bs * 8);
     prec->lev_fwd = build_levels(sys->n, F.rowptr, F.colind, F.diaind, true);
     upload(ctx, prec->lev_rows, prec->lev_fwd.rows.data(), std::max<size_t>(prec->lev_fwd.rows.size(), 1));
+    prec->ilu = ilu_plan(sys->b, prec->lev_fwd.ptr, prec->lev_fwd.rows, F.rowptr, F.colind, F.diaind);
+    upload(ctx, prec->ilu_units, prec->ilu.units.data(), prec->ilu.units.size());
+    dalloc(ctx, prec->ilu_sync, kIluSync * 4);
     // strips where the rows fit them, unless both directions together are
     // faster level-scheduled
     prec->fwd = SweepDev{};
@@ -1642,29 +1645,59 @@ extern "C" int dfg_precond_set_value(dfg_precond prec, dfg_system sys) {
     dfg_ctx ctx_ = ctx;
     REQUIRE(prec->symbolic && prec->sys == sys, DFG_NOT_READY, "dfg_precond_set_linear_system must come first");
     const size_t bs = (size_t)sys->b * sys->b;
-    // SetValue_Initialize: copy A into the factor storage (zero at fill-in)
-    CK(cudaMemcpyAsync(prec->fdiag.p, sys->diag.p, (size_t)sys->n * bs * 8, cudaMemcpyDeviceToDevice, ctx->stream));
+    const FactorPattern F = factor_pattern(prec);
+    const Levels& L = prec->lev_fwd;
+    const bool one_launch = prec->ilu.warp_bytes > 0;
+    // SetValue_Initialize: A on the factor's pattern, zero at fill-in.  The
+    // one-launch factorisation reads it where it is (with fill-in: from a
+    // buffer of its own), the level-by-level one works in the factor's storage.
+    const long long nval = prec->nnz * (long long)bs;
     if (prec->own_pattern) {
-      CK(cudaMemsetAsync(prec->foffd.p, 0, (size_t)prec->nnz * bs * 8, ctx->stream));
-      CK(launch_factor_init(sys->b, sys->nnz, prec->a2f.as<int>(), sys->offd.as<double>(), prec->foffd.as<double>(),
+      DBuf& dst = one_launch ? prec->ilu_src : prec->foffd;
+      dalloc(ctx, dst, (size_t)nval * 8);
+      CK(cudaMemsetAsync(dst.p, 0, (size_t)nval * 8, ctx->stream));
+      CK(launch_factor_init(sys->b, sys->nnz, prec->a2f.as<int>(), sys->offd.as<double>(), dst.as<double>(),
                             ctx->stream));
       launched(ctx);
-    } else if (sys->nnz) {
-      CK(cudaMemcpyAsync(prec->foffd.p, sys->offd.p, (size_t)sys->nnz * bs * 8, cudaMemcpyDeviceToDevice, ctx->stream));
+    } else if (!one_launch && sys->nnz) {
+      CK(cudaMemcpyAsync(prec->foffd.p, sys->offd.p, (size_t)nval * 8, cudaMemcpyDeviceToDevice, ctx->stream));
     }
-    const FactorPattern F = factor_pattern(prec);
-    Scratch sc = scratch_of(ctx);
-    int* nsing = sc.tickets + 8;
-    CK(cudaMemsetAsync(nsing, 0, sizeof(int), ctx->stream));
-    const Levels& L = prec->lev_fwd;
-    const int nl = (int)L.ptr.size() - 1;
-    for (int l = 0; l < nl; ++l)
-      CK(launch_ilu_level(sys->b, prec->lev_rows.as<int>() + L.ptr[l], L.ptr[l + 1] - L.ptr[l], F.d_rowptr,
-                          F.d_colind, F.d_diaind, prec->fdiag.as<double>(), prec->foffd.as<double>(), nsing,
-                          ctx->stream, l > 0));
-    launched(ctx, nl);
-    int h_nsing = 0;
-    CK(cudaMemcpyAsync(&h_nsing, nsing, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    if (one_launch) {
+      CK(fill_sentinel(nval, prec->foffd.p, false, ctx->stream));
+      launched(ctx);
+    } else {
+      CK(cudaMemcpyAsync(prec->fdiag.p, sys->diag.p, (size_t)sys->n * bs * 8, cudaMemcpyDeviceToDevice, ctx->stream));
+    }
+    int* sync = prec->ilu_sync.as<int>();
+    CK(cudaMemsetAsync(sync, 0, kIluSync * 4, ctx->stream));
+    if (one_launch) {
+      IluArgs a{};
+      a.units = prec->ilu_units.as<int2>();
+      a.nunits = (int)prec->ilu.units.size();
+      a.rows = prec->lev_rows.as<int>();
+      a.rowptr = F.d_rowptr;
+      a.colind = F.d_colind;
+      a.diaind = F.d_diaind;
+      a.adiag = sys->diag.as<double>();
+      a.aoffd = prec->own_pattern ? prec->ilu_src.as<double>() : sys->offd.as<double>();
+      a.fdiag = prec->fdiag.as<double>();
+      a.foffd = prec->foffd.as<double>();
+      a.sync = sync;
+      a.maxrow = prec->ilu.maxrow;
+      a.maxlow = prec->ilu.maxlow;
+      a.maxu = prec->ilu.maxu;
+      CK(launch_ilu(sys->b, prec->ilu, a, ctx->nsm, ctx->stream));
+      launched(ctx, 1);
+    } else {
+      const int nl = (int)L.ptr.size() - 1;
+      for (int l = 0; l < nl; ++l)
+        CK(launch_ilu_level(sys->b, prec->lev_rows.as<int>() + L.ptr[l], L.ptr[l + 1] - L.ptr[l], F.d_rowptr,
+                            F.d_colind, F.d_diaind, prec->fdiag.as<double>(), prec->foffd.as<double>(), sync + 1,
+                            ctx->stream, l > 0));
+      launched(ctx, nl);
+    }
+    int h_sync[kIluSync] = {};
+    CK(cudaMemcpyAsync(h_sync, sync, sizeof(h_sync), cudaMemcpyDeviceToHost, ctx->stream));
     if (prec->strips) {
       pack_strips(ctx, prec, false);
     } else {
@@ -1672,10 +1705,15 @@ extern "C" int dfg_precond_set_value(dfg_precond prec, dfg_system sys) {
       pack_sweep(ctx, prec, prec->bwd, false);
     }
     CK(cudaStreamSynchronize(ctx->stream));
-    prec->numeric = true;
     prec->numeric32 = false;
-    if (h_nsing > 10) {
-      set_err(ctx, "ILU: " + std::to_string(h_nsing) + " singular pivots (more than 10)");
+    if (h_sync[4] != 0) {
+      prec->numeric = false;
+      set_err(ctx, "a wait of the ILU factorisation timed out (row " + std::to_string(h_sync[7]) + ")");
+      return DFG_TIMEOUT;
+    }
+    prec->numeric = true;
+    if (h_sync[1] > 10) {
+      set_err(ctx, "ILU: " + std::to_string(h_sync[1]) + " singular pivots (more than 10)");
       return DFG_SINGULAR_PIVOT;
     }
     return DFG_OK;

@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "../../include/dfg.h"
+#include "k_ilu.h"
 #include "k_strip.h"
 #include "k_sweep.h"
 
@@ -291,6 +292,8 @@ struct dfg_precond_s {
   dfg::DBuf fdiag, foffd;          // factor, reference layout (FP64)
   dfg::Levels lev_fwd;
   dfg::DBuf lev_rows;
+  dfg::IluPlan ilu;                       // one-launch factorisation (units on the device)
+  dfg::DBuf ilu_units, ilu_sync, ilu_src;  // ilu_src: A on a pattern with fill-in
   dfg::SweepDev fwd, bwd;
   bool strips = false;             // both directions sweep in strips (fwd, bwd then unused)
   dfg::StripDev strip[2][2];       // [forward, backward][FP64, FP32]

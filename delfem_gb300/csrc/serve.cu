@@ -164,6 +164,7 @@ struct Req {
   GatherMap gm;
   SellMap sell;
   Levels lev;
+  IluPlan ilu;
   SweepPlan pf, pb;
   std::vector<unsigned char> hf, hb;
   std::vector<long long> of, ob;
@@ -183,7 +184,7 @@ struct Req {
   size_t o_recf, o_offf, o_rsf, o_recb, o_offb, o_rsb, o_st, o_cnt;
   size_t o_chf = 0, o_chb = 0, o_posf = 0, o_rperm = 0;
   size_t t_rowptr, t_colind, t_diag, t_offd, t_ssrc;
-  size_t t_coords, t_conn, t_coef, t_bc, t_load, t_em, t_er, t_sp, t_ss, t_rp, t_rs, t_dia, t_lev, t_fd, t_fo;
+  size_t t_coords, t_conn, t_coef, t_bc, t_load, t_em, t_er, t_sp, t_ss, t_rp, t_rs, t_dia, t_lev, t_units, t_fd, t_fo;
   size_t t_eof, t_esf, t_srf, t_eob, t_esb, t_srb;
   size_t pbase = 0, tbase = 0;
   bool have_p = false, have_t = false;
@@ -352,6 +353,7 @@ bool symbolic(dfg_server_s* S, Req* r) {
     return false;
   }
   r->lev = build_levels(n, r->rowptr.data(), r->colind.data(), r->diaind.data(), true);
+  r->ilu = ilu_plan(r->b, r->lev.ptr, r->lev.rows, r->rowptr.data(), r->colind.data(), r->diaind.data());
   r->sell = build_sell(n, r->rowptr.data(), r->colind.data());
   const int elem = S->fp32 ? 4 : 8;
   r->maxe = 0;
@@ -465,6 +467,7 @@ bool symbolic(dfg_server_s* S, Req* r) {
   r->t_rs = T.add(std::max<size_t>(r->gm.res_src.size(), 1) * 4);
   r->t_dia = T.add((size_t)n * 4);
   r->t_lev = T.add(std::max<size_t>(r->lev.rows.size(), 1) * 4);
+  r->t_units = T.add(std::max<size_t>(r->ilu.units.size(), 1) * sizeof(int2));
   r->t_fd = T.add((size_t)n * bs * 8);
   r->t_fo = T.add(Z * bs * 8);
   r->t_eof = T.add(r->pf.ent_off.size() * 8);
@@ -491,7 +494,7 @@ void up(dfg_server_s* S, cudaStream_t st, size_t base, size_t off, const std::ve
 SrvSlot slot_of(dfg_server_s* S, Req* r);
 
 // Device work of one admission on an admission lane's stream; returns the
-// ILU singular-pivot count.
+// ILU singular-pivot count, -1 when a wait of the factorisation gave up.
 int admit_device(dfg_server_s* S, Req* r, dfg_server_s::AdmLane& lane) {
   const size_t pb = r->pbase, tb = r->tbase;
   const int n = r->n, b = r->b;
@@ -515,6 +518,7 @@ int admit_device(dfg_server_s* S, Req* r, dfg_server_s::AdmLane& lane) {
   up(S, st, tb, r->t_rs, r->gm.res_src);
   up(S, st, tb, r->t_dia, r->diaind);
   up(S, st, tb, r->t_lev, r->lev.rows);
+  up(S, st, tb, r->t_units, r->ilu.units);
   up(S, st, pb, r->o_recf, r->hf);
   up(S, st, pb, r->o_offf, r->of);
   up(S, st, pb, r->o_rsf, r->pf.range_steps);
@@ -582,18 +586,28 @@ int admit_device(dfg_server_s* S, Req* r, dfg_server_s::AdmLane& lane) {
   bc.res = rhs;
   SCK(launch_bc(bc, st));
   nl += 2;
-  // ILU(0): SetValue_Initialize (copy), then the levels
+  // ILU(0): all levels in one launch, or (rows too wide for it)
+  // SetValue_Initialize (copy) and a launch per level
   double* fd = at<double>(S, tb, r->t_fd);
   double* fo = at<double>(S, tb, r->t_fo);
-  SCK(cudaMemcpyAsync(fd, diag, n * bs * 8, cudaMemcpyDeviceToDevice, st));
-  if (r->nnz) SCK(cudaMemcpyAsync(fo, offd, r->nnz * bs * 8, cudaMemcpyDeviceToDevice, st));
-  int* nsing = reinterpret_cast<int*>(lane.d_red + kRedGrid + 16);
-  SCK(cudaMemsetAsync(nsing, 0, sizeof(int), st));
-  const int nlev = (int)r->lev.ptr.size() - 1;
-  for (int l = 0; l < nlev; ++l)
-    SCK(launch_ilu_level(b, at<int>(S, tb, r->t_lev) + r->lev.ptr[l], r->lev.ptr[l + 1] - r->lev.ptr[l],
-                         bc.rowptr, bc.colind, at<int>(S, tb, r->t_dia), fd, fo, nsing, st, l > 0));
-  nl += nlev;
+  int* sync = reinterpret_cast<int*>(lane.d_red + kRedGrid + 16);
+  SCK(cudaMemsetAsync(sync, 0, kIluSync * sizeof(int), st));
+  if (r->ilu.warp_bytes > 0) {
+    SCK(fill_sentinel(r->nnz * (long long)bs, fo, false, st));
+    const IluArgs ia{at<int2>(S, tb, r->t_units), (int)r->ilu.units.size(), at<int>(S, tb, r->t_lev), bc.rowptr,
+                     bc.colind, at<int>(S, tb, r->t_dia), diag, offd, fd, fo, sync, r->ilu.maxrow, r->ilu.maxlow,
+                     r->ilu.maxu};
+    SCK(launch_ilu(b, r->ilu, ia, S->nsm, st));
+    nl += 2;
+  } else {
+    SCK(cudaMemcpyAsync(fd, diag, n * bs * 8, cudaMemcpyDeviceToDevice, st));
+    if (r->nnz) SCK(cudaMemcpyAsync(fo, offd, r->nnz * bs * 8, cudaMemcpyDeviceToDevice, st));
+    const int nlev = (int)r->lev.ptr.size() - 1;
+    for (int l = 0; l < nlev; ++l)
+      SCK(launch_ilu_level(b, at<int>(S, tb, r->t_lev) + r->lev.ptr[l], r->lev.ptr[l + 1] - r->lev.ptr[l],
+                           bc.rowptr, bc.colind, at<int>(S, tb, r->t_dia), fd, fo, sync + 1, st, l > 0));
+    nl += nlev;
+  }
   // the matrix into its sliced-ELL copy (the only copy that stays resident;
   // the mixed form keeps an FP32 one beside it)
   SCK(sell_pack(r->sell.nslices, b, at<long long>(S, pb, r->o_sptr), at<int>(S, tb, r->t_ssrc), diag, offd,
@@ -636,13 +650,13 @@ int admit_device(dfg_server_s* S, Req* r, dfg_server_s::AdmLane& lane) {
   SCK(api_dot(m, rhs, rhs, red, st));
   SCK(srv_init_state(at<PcgState>(S, pb, r->o_st), red.result, S->tol, S->maxit, S->mixed ? kMixedDelta2 : 0.0, st));
   nl += 3;
-  SCK(cudaMemcpyAsync(lane.h_nsing, nsing, sizeof(int), cudaMemcpyDeviceToHost, st));
+  SCK(cudaMemcpyAsync(lane.h_nsing, sync, kIluSync * sizeof(int), cudaMemcpyDeviceToHost, st));
   SCK(cudaStreamSynchronize(st));
   {
     std::lock_guard<std::mutex> lk(S->mu);
     S->launches += nl;
   }
-  return *lane.h_nsing;
+  return lane.h_nsing[4] != 0 ? -1 : lane.h_nsing[1];
 }
 
 void finish_locked(dfg_server_s* S, Req* r) {
@@ -651,7 +665,7 @@ void finish_locked(dfg_server_s* S, Req* r) {
   // host set-up data is no longer needed
   r->coords = {}; r->coef = {}; r->load = {}; r->conn = {}; r->bcflag = {};
   r->rowptr = {}; r->colind = {}; r->diaind = {};
-  r->gm = GatherMap{}; r->sell = SellMap{}; r->lev = Levels{}; r->pf = SweepPlan{}; r->pb = SweepPlan{};
+  r->gm = GatherMap{}; r->sell = SellMap{}; r->lev = Levels{}; r->ilu = IluPlan{}; r->pf = SweepPlan{}; r->pb = SweepPlan{};
   r->hf = {}; r->hb = {}; r->of = {}; r->ob = {};
   r->chf = {}; r->chb = {}; r->posf = {};
   ++S->n_finished;
@@ -780,6 +794,13 @@ void admission_thread(dfg_server_s* S, int li) {
     if (S->fatal != DFG_OK) {  // the serving loop has stopped
       r->status = S->fatal;
       r->error = S->fatal_msg;
+      release_locked(S, r);
+      finish_locked(S, r);
+      continue;
+    }
+    if (nsing < 0) {
+      r->status = DFG_TIMEOUT;
+      r->error = "ILU(0): a wait of the factorisation gave up (row " + std::to_string(lane.h_nsing[7]) + ")";
       release_locked(S, r);
       finish_locked(S, r);
       continue;
