@@ -161,6 +161,13 @@ __global__ void k_ilu_level(const int* __restrict__ rows, int cnt, const int* __
 // units claimed earlier, by warps that are running, so nothing depends on how
 // many CTAs are resident; every wait is bounded.
 //
+// Measured on GB300, SetValue as a whole, a thread per row and a launch per
+// level -> this kernel: 1x1 blocks 128x128 cells 1.92 -> 0.48 ms, 300x300 4.65 ->
+// 1.08; 2x2 200x100 4.77 -> 0.71, 401x199 9.46 -> 1.42, ILU(1) 161x83 7.88 ->
+// 0.83; 3x3 24^3 9.7 -> 0.70, 56^3 25.6 -> 2.7 ms.  (Counters of finished units
+// with release and acquire instead of the sentinel: 1.27, 3.36, 1.56, 3.34,
+// 1.48, 1.09 and 8.3 ms.)  What bounds it now: the FP64 chain of a row per
+// level in narrow levels (1.9 us per level, 1x1), the FP64 pipes in wide ones.
 template <int B>
 struct IluLanes;
 template <> struct IluLanes<1> { static constexpr int G = 8, J = 8; };
@@ -380,6 +387,7 @@ static cudaError_t launch_ilu_b(const IluPlan& P, const IluArgs& a, int nsm, cud
   // enough warps for three levels' units (those of the next levels load while
   // they wait), at most per_sm CTAs, one warp per scheduler each: with more the
   // units of a wide level pile up on some of the schedulers
+  // (3x3, 56^3: 8.3 ms with ten CTAs per SM, 2.7 with two and the sentinel)
   constexpr int per_sm = 2;
   const int grid = std::max(1, std::min((3 * P.max_level_units + kIluWarps - 1) / kIluWarps, nsm * per_sm));
   k_ilu<B><<<grid, kIluWarps * 32, smem, st>>>(a, P.warp_bytes / (32 / IluLanes<B>::G));

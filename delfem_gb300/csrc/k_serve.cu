@@ -136,6 +136,14 @@ __device__ __forceinline__ void put_sweep_input(const SrvSlot& S, long long k, d
   }
 }
 
+// The share of chunk c in the sentinel fill of the slot's exchange buffers.
+template <typename Z>
+__device__ __forceinline__ void fill_xch(const SrvSlot& S, int c) {
+  const long long k = c - S.chunk0, e1 = S.nx * (k + 1) / S.nchunks;
+  for (long long e = S.nx * k / S.nchunks + threadIdx.x; e < e1; e += kSrvTpb)
+    reinterpret_cast<Z*>(S.xch)[e] = sentinel_value<Z>();
+}
+
 // element range [e0, e1) of chunk c of slot S
 __device__ __forceinline__ void chunk_elems(const SrvSlot& S, int c, long long& e0, long long& e1) {
   const long long row0 = (long long)(c - S.chunk0) * kSrvRows;
@@ -280,6 +288,7 @@ __global__ void __launch_bounds__(kSrvTpb, kSrvVecBlocks) k_srv_update_rx(const 
       }
       put_sweep_input<Z>(S, k, r);
     }
+    fill_xch<Z>(T->slot[si], c);
     publish(part, c, partials);
   }
 }
@@ -503,6 +512,7 @@ __global__ void __launch_bounds__(kSrvTpb, kSrvVecBlocks) k_srvm_update_rx(const
         z[k] = sentinel_value<float>();
       }
     }
+    fill_xch<float>(S, c);
     double tot;
     if (slot_sum(part, c, S, partials, &tot) && threadIdx.x == 0) {
       PcgState* st = S.st;

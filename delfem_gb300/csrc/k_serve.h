@@ -41,11 +41,16 @@ struct SrvSlot {
   float* p32;
   float* q32;
   double* d;
-  // one-CTA-per-solve sweeps (k_solo.cu), else nullptr: the forward sweep's
-  // input stored in its step order, rperm[posf[row]*b + c] = r[row*b + c]
-  // (the sweep's element type: FP32 in the FP32 modes)
+  // strip and one-CTA-per-solve sweeps (k_strip.cu, k_solo.cu), else nullptr:
+  // the forward sweep's input stored in its step order,
+  // rperm[posf[row]*b + c] = r[row*b + c] (the sweep's element type: FP32 in
+  // the FP32 modes)
   const int* posf;
   void* rperm;
+  // strip sweeps: the exchange buffers of both directions, nx elements filled
+  // with the sentinel before each iteration's sweeps
+  void* xch;
+  long long nx;
 };
 
 struct SrvTable {

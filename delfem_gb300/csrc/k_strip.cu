@@ -215,7 +215,7 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32) k_strip(StripAr
   constexpr int HB = B == 3 ? 1 : 2;
   constexpr int G = NE <= 4 && CH >= 4 ? 4 : 1;
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ int s_ticket, s_stop;
+  __shared__ int s_group, s_slot, s_stop;
   const int W = a.W, NS = a.NS;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool compute = warp < W, load_warp = warp == 2 * W;
@@ -233,7 +233,6 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32) k_strip(StripAr
   }
   pdl_enter();
   if (a.one.done && *a.one.done) return;
-  const StripSlot& S = a.one;
   int st = 0, ph = 0;  // stage and phase of the strip's next chunk (compute warps and loader alike)
   for (;;) {
     int issued = 0;  // loader: chunks of the strip issued
@@ -241,10 +240,36 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32) k_strip(StripAr
       *delivered = 0;
       *consumed = 0;
     }
-    if (threadIdx.x == 0) s_ticket = atomicAdd(a.ticket, 1);
+    if (threadIdx.x == 0) {
+      int t = atomicAdd(a.ticket, 1), j = 0;
+      if (const StripBatch* bt = a.batch) {
+        const int n = bt->nslots;
+        if (n == 0 || t >= bt->group_start[n]) {
+          t = -1;
+        } else {
+          int lo = 0, hi = n - 1;  // last j with group_start[j] <= t
+          while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (bt->group_start[mid] <= t) lo = mid; else hi = mid - 1;
+          }
+          j = lo;
+          t = ld_relaxed_int(bt->slot[j].done) != 0 ? -2 : t - bt->group_start[j];
+        }
+      } else if (t * W >= a.one.nstrips) {
+        t = -1;
+      }
+      s_group = t;
+      s_slot = j;
+    }
     __syncthreads();
-    const int r = s_ticket * W + w;
-    if (s_ticket * W >= S.nstrips) break;
+    const int group = s_group;
+    const StripSlot S = a.batch ? a.batch->slot[s_slot] : a.one;
+    if (group == -1) break;
+    if (group == -2) {  // a finished solve
+      __syncthreads();
+      continue;
+    }
+    const int r = group * W + w;
     if (load_warp) {
       // -------------------------------------------------------------- loader
       // lane w keeps warp w's stages filled: a chunk's records and its

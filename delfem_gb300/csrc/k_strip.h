@@ -115,8 +115,19 @@ struct StripSlot {
   const int* done;           // optional: nonzero = skip
   int nstrips;
 };
+// Several independent sweeps in one launch (the serving path): a ticket t
+// names group t - group_start[j] (of W strips) of the slot j with
+// group_start[j] <= t < group_start[j + 1]; finished solves' groups are
+// skipped.
+constexpr int kStripMaxSlots = 256;
+struct StripBatch {
+  int nslots;
+  int group_start[kStripMaxSlots + 1];
+  StripSlot slot[kStripMaxSlots];
+};
 struct StripArgs {
   StripSlot one;
+  const StripBatch* batch;  // non-null: batched launch (`one` unused)
   int* ticket;   // 0 at launch
   int* err;      // device error word
   int ne;        // entry class

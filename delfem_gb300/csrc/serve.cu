@@ -54,6 +54,9 @@ namespace {
 using Clock = std::chrono::steady_clock;
 
 constexpr int kClasses = 9;         // block size 1..3 x dependency entries <= 4, 8, 16
+constexpr int kStripNe[] = {3, 4, 7, 16};
+constexpr int kStripClasses = 12;   // block size 1..3 x entry class of the strip sweeps
+constexpr int kStripBit = 2 * kClasses;  // their first bit in Group::graph_mask
 constexpr int kMaxChunks = 1 << 20; // chunk space of one launch (kSrvRows rows each)
 constexpr int kRingSteps = 32;
 constexpr int kServeStages = 3;   // sweep pipeline depth in batched launches
@@ -175,6 +178,16 @@ struct Req {
   // position of every row (where the forward input is stored)
   std::vector<SoloChunk> chf, chb;
   std::vector<int> posf;
+  // strips (k_strip.cu): per direction the plan (less what the packed metadata
+  // holds) and the metadata
+  bool strips = false;
+  StripPlan strip[2];
+  std::vector<int> smeta[2];
+  size_t o_srec[2] = {}, o_schunk[2] = {}, o_sip[2] = {}, o_sit[2] = {}, o_sxch = 0;
+  size_t t_smeta[2] = {}, t_sneed[2] = {}, t_sslot[2] = {}, t_srows[2] = {};
+  long long nxch() const {  // elements of both exchange buffers
+    return ((long long)strip[0].nexport + strip[1].nexport) * (strip[0].d.VS / strip[0].elem);
+  }
   // algorithmic bytes of one launch of each batched kernel for this solve:
   // 0 r.z, 1 p update, 2 SpMV, 3 r/x update, then forward and backward sweep
   double alg[6] = {};
@@ -199,6 +212,10 @@ struct Req {
 inline int class_index(int b, int maxe) { return (b - 1) * 3 + (maxe <= 4 ? 0 : maxe <= 8 ? 1 : 2); }
 inline int class_maxe(int c) { return (c % 3) == 0 ? 4 : (c % 3) == 1 ? 8 : 16; }
 inline int class_b(int c) { return c / 3 + 1; }
+inline int strip_class_index(int b, int ne) { return (b - 1) * 4 + (ne == 3 ? 0 : ne == 4 ? 1 : ne == 7 ? 2 : 3); }
+constexpr int kTickets = kClasses * 4 + kStripClasses * 2;
+// the class whose stream and profile slot a strip class shares
+inline int strip_host_class(int k) { return k / 4 * 3 + (k % 4 <= 1 ? 0 : k % 4 - 1); }
 
 // Device tables, streams and graphs of one size group (see kGroups).
 struct Group {
@@ -208,7 +225,9 @@ struct Group {
   SweepBatch* h_sb = nullptr;
   SoloBatch* d_solo = nullptr;     // kClasses x 2: one-CTA-per-solve sweeps
   SoloBatch* h_solo = nullptr;
-  int* d_tickets = nullptr;        // kClasses x 2 ranged, then kClasses x 2 solo
+  StripBatch* d_strip = nullptr;   // kStripClasses x 2: strip sweeps
+  StripBatch* h_strip = nullptr;
+  int* d_tickets = nullptr;        // kClasses x 2 ranged, kClasses x 2 solo, kStripClasses x 2 strips
   double* d_partials = nullptr;    // kMaxChunks
   unsigned char* d_chunk_slot = nullptr;  // kMaxChunks: each chunk's slot
   unsigned char* h_chunk_slot = nullptr;
@@ -219,7 +238,7 @@ struct Group {
   cudaEvent_t ev_fork = nullptr, ev_done = nullptr, ev_join[kClasses] = {};
   cudaEvent_t ev_prof[2 * DFG_SERVER_NKERNELS] = {};
   cudaGraphExec_t exec = nullptr, exec_prof = nullptr;
-  int graph_mask = -1;             // bits 0..8: ranged classes present; 9..17: solo classes
+  int graph_mask = -1;             // bits 0..8: ranged classes present; 9..17: solo; 18..29: strips
   std::vector<Req*> act;           // table order
   std::deque<Req*> incoming;       // admitted, waiting for a table slot (guarded by the server mutex)
   bool changed = false, in_flight = false, prof = false;
@@ -265,6 +284,9 @@ struct dfg_server_s {
   int solo_grid[kClasses] = {}, solo_ns[kClasses][2] = {}, solo_R[kClasses] = {}, solo_rec_stage[kClasses][2] = {};
   int solo_ch[kClasses][2] = {};
   size_t solo_smem[kClasses][2] = {};
+  // per-class strip sweep shape: grid, stages, shared memory
+  int strip_grid[kStripClasses] = {}, strip_ns[kStripClasses][2] = {};
+  size_t strip_smem[kStripClasses][2] = {};
   int sweeps = 0;  // dfg_server_config::sweeps
 
   // host state
@@ -311,28 +333,40 @@ namespace {
 
 // ---------------------------------------------------------------- symbolic
 
-// Which sweep kernel serves a solve.  One CTA per solve (k_solo.cu) keeps a
-// solve's whole dependency chain on one SM, and the in-flight solves fill
-// the device; the ranged kernel (k_sweep.cu) spreads one solve over many
-// SMs at the price of cross-SM hand-offs (about 0.75 us per dependency level
-// in batched launches).  FP32 sweeps take one CTA, except 3x3-block solves
-// above 100,000 nodes.  Measured on GB300 over bands of the serving streams
-// (FP32 factor, solves/s, ranged -> one CTA).  2D stream: 1x1 blocks
-// 231 -> 295 (2k-20k nodes), 58 -> 84, 19 -> 28, 5.5 -> 7.1 (150k-400k);
-// 2x2 blocks 142 -> 158, 34 -> 40, 13.0 -> 13.7 (60k-150k), 4.65 -> 5.71
-// (150k-250k), 2.07 -> 2.31 (250k-400k).  3D stream: 1x1 blocks
-// 52.8 -> 126.0 (< 40k), 13.9 -> 48.1, 12.8 -> 24.8, 6.1 -> 11.5 (> 300k);
-// 3x3 blocks 18.1 -> 32.9 (< 40k), 7.8 -> 9.0 (40k-120k), but 4.0 -> 2.4
-// (120k-300k) and 2.3 -> 1.1 (> 300k): a wide 3D level of 3x3 blocks is more
-// record bytes than one SM streams in a level's time.  FP64 sweeps stay
-// ranged: on one SM every level waits on a chain of dependent FP64 FMAs (64
-// cycles each on GB300), about twice the ranged kernel's time beyond the
-// smallest solves.
+// Which sweep kernel serves a solve whose rows do not fit strips (rows of
+// more than 16 entries do not get here; scattered numberings do).  One CTA per
+// solve (k_solo.cu) keeps a solve's whole dependency chain on one SM; the
+// ranged kernel (k_sweep.cu) spreads one solve over many SMs at the price of
+// cross-SM hand-offs (about 0.75 us per dependency level).  Measured on GB300
+// over bands of the serving streams (FP32 factor, solves/s, ranged -> one
+// CTA).  2D stream: 1x1 blocks 231 -> 295 (2k-20k nodes) to 5.5 -> 7.1
+// (150k-400k); 2x2 blocks 142 -> 158 to 2.07 -> 2.31.  3D stream: 1x1 blocks
+// 52.8 -> 126.0 (< 40k) to 6.1 -> 11.5 (> 300k); 3x3 blocks 18.1 -> 32.9
+// (< 40k), 7.8 -> 9.0 (40k-120k), but 4.0 -> 2.4 (120k-300k) and 2.3 -> 1.1.
+// FP64 sweeps stay ranged: on one SM every level waits on a chain of dependent
+// FP64 FMAs (64 cycles each on GB300).
 constexpr int kSoloMaxNodes3x3 = 100000;
 bool use_solo(const dfg_server_s* S, const Req* r) {
   if (S->sweeps == 1) return false;
   if (S->sweeps == 2) return true;
   return S->fp32 && (r->b < 3 || r->n <= kSoloMaxNodes3x3);
+}
+
+// Strips (k_strip.cu) serve every solve whose rows fit them, unless the
+// configuration asks for one of the older kinds.  Measured on GB300, the
+// saturated 2D stream (solves/s, the rule above -> strips): FP64 45 -> 63, FP32
+// factor 87 -> 105, FP32 everything 59 -> 84; a batch of 24 requests of 2k-40k
+// nodes, FP32 factor, 257 -> 140 ms.  One strip per CTA and about four CTAs per
+// SM: a launch mixes solves of one strip and of twenty, and any SM can take any
+// strip.
+constexpr int kServeStripWarps = 1;  // strips per CTA
+bool use_strips(const dfg_server_s* S, Req* r, int elem) {
+  if (S->sweeps != 0) return false;
+  for (int dir = 0; dir < 2; ++dir)
+    if (!strip_plan(r->n, r->b, elem, r->rowptr.data(), r->colind.data(), r->diaind.data(), dir == 0, r->strip[dir]) ||
+        S->strip_ns[strip_class_index(r->b, r->strip[dir].ne)][dir] == 0)
+      return false;
+  return true;
 }
 
 // Fills the request's host-side set-up; returns false with r->error on failure.
@@ -365,8 +399,22 @@ bool symbolic(dfg_server_s* S, Req* r) {
   }
   r->cls = class_index(r->b, r->maxe);
   r->group = group_of((long long)n * r->b, S->ngroups);
-  r->solo = use_solo(S, r);
-  if (r->solo) {
+  r->strips = use_strips(S, r, elem);
+  r->solo = !r->strips && use_solo(S, r);
+  if (r->strips) {
+    // the forward sweep writes y where the backward sweep reads it; the
+    // backward sweep writes z in row order
+    std::vector<int> ident(n);
+    for (int i = 0; i < n; ++i) ident[i] = i;
+    for (int dir = 0; dir < 2; ++dir) {
+      StripPlan& P = r->strip[dir];
+      const int k = strip_class_index(r->b, P.ne);
+      r->smeta[dir] = strip_meta(P, dir == 0 ? r->strip[1].pos.data() : ident.data(), kServeStripWarps, S->strip_ns[k][dir]);
+      P.codes = {};
+      P.exports = {};
+    }
+    r->posf = std::move(r->strip[0].pos);
+  } else if (r->solo) {
     const int k = r->cls, R = S->solo_R[k];
     SoloPlan sf = solo_sweep_plan(n, r->b, r->rowptr.data(), r->colind.data(), r->diaind.data(), true, R, elem,
                                   S->solo_rec_stage[k][0], S->solo_ch[k][0]);
@@ -408,8 +456,12 @@ bool symbolic(dfg_server_s* S, Req* r) {
       r->alg[2] = idx + vals * 8 + dm * 16;  // values + CRS-equivalent indices + p read + q write
       r->alg[3] = dm * (16 + 8 + 16 + 8 + 2 * elem + (S->fp32 ? 4 : 0));
     }
-    r->alg[4] = (double)r->hf.size() + dm * 2 * elem;
-    r->alg[5] = (double)r->hb.size() + dm * 2 * elem;
+    auto rec = [&](int dir) {
+      return r->strips ? (double)r->strip[dir].nchunks * r->strip[dir].d.chunk_bytes
+                       : (double)(dir == 0 ? r->hf.size() : r->hb.size());
+    };
+    r->alg[4] = rec(0) + dm * 2 * elem;
+    r->alg[5] = rec(1) + dm * 2 * elem;
   }
   Layout& P = r->P;
   const size_t sblk = (size_t)std::max<long long>(r->sell.ptr.back(), 1);
@@ -429,7 +481,8 @@ bool symbolic(dfg_server_s* S, Req* r) {
   r->o_rd = P.add(m * 8);
   // a solo solve's y is stored in the backward plan's step order (padded
   // steps of 32 rows)
-  const size_t ystore = r->solo ? std::max<size_t>(m, (size_t)r->pb.nsteps * 32 * r->b) : m;
+  const size_t ystore = r->solo ? std::max<size_t>(m, (size_t)r->pb.nsteps * 32 * r->b)
+                        : r->strips ? (size_t)r->strip[1].steps() * r->strip[1].d.RW * r->b : m;
   r->o_y = P.add(ystore * elem + 64);
   r->o_z = P.add(m * elem + 64);
   r->o_r32 = P.add(S->fp32 ? m * 4 + 64 : 16);
@@ -447,7 +500,27 @@ bool symbolic(dfg_server_s* S, Req* r) {
     r->o_posf = P.add((size_t)n * 4);
     r->o_rperm = P.add((size_t)r->pf.nsteps * 32 * r->b * elem + 64);
   }
+  if (r->strips) {
+    for (int dir = 0; dir < 2; ++dir) {
+      const StripPlan& Q = r->strip[dir];
+      r->o_srec[dir] = P.add((size_t)Q.nchunks * Q.d.chunk_bytes);
+      r->o_schunk[dir] = P.add(Q.strip_chunk.size() * 4);
+      r->o_sip[dir] = P.add(Q.item_ptr.size() * 4);
+      r->o_sit[dir] = P.add(Q.items.size() * 4 + 16);
+    }
+    r->o_posf = P.add((size_t)n * 4);
+    r->o_rperm = P.add((size_t)r->strip[0].steps() * r->strip[0].d.rhs_bytes + 64);
+    r->o_sxch = P.add((size_t)r->nxch() * elem + 64);
+  }
   Layout& T = r->T;
+  if (r->strips)
+    for (int dir = 0; dir < 2; ++dir) {
+      const StripPlan& Q = r->strip[dir];
+      r->t_smeta[dir] = T.add(r->smeta[dir].size() * 4);
+      r->t_sneed[dir] = T.add(Q.need.size() * 4);
+      r->t_sslot[dir] = T.add(Q.ent_slot.size() * 4);
+      r->t_srows[dir] = T.add(Q.step_rows.size() * 4);
+    }
   const size_t k = r->nnoel;
   r->t_rowptr = T.add((n + 1) * 4);
   r->t_colind = T.add(Z * 4);
@@ -529,6 +602,24 @@ int admit_device(dfg_server_s* S, Req* r, dfg_server_s::AdmLane& lane) {
     up(S, st, pb, r->o_chf, r->chf);
     up(S, st, pb, r->o_chb, r->chb);
     up(S, st, pb, r->o_posf, r->posf);
+  }
+  if (r->strips) {
+    for (int dir = 0; dir < 2; ++dir) {
+      const StripPlan& Q = r->strip[dir];
+      up(S, st, tb, r->t_smeta[dir], r->smeta[dir]);
+      up(S, st, tb, r->t_sneed[dir], Q.need);
+      up(S, st, tb, r->t_sslot[dir], Q.ent_slot);
+      up(S, st, tb, r->t_srows[dir], Q.step_rows);
+      up(S, st, pb, r->o_schunk[dir], Q.strip_chunk);
+      up(S, st, pb, r->o_sip[dir], Q.item_ptr);
+      up(S, st, pb, r->o_sit[dir], Q.items);
+      SCK(launch_strip_meta(Q.d, Q.nchunks, at<int>(S, tb, r->t_smeta[dir]), at<int>(S, tb, r->t_sneed[dir]),
+                            at<unsigned char>(S, pb, r->o_srec[dir]), st));
+    }
+    up(S, st, pb, r->o_posf, r->posf);
+    // the rows' places only: what lies between them is never used, but copied
+    SCK(cudaMemsetAsync(at<void>(S, pb, r->o_rperm), 0,
+                        (size_t)r->strip[0].steps() * r->strip[0].d.rhs_bytes, st));
   }
   up(S, st, tb, r->t_eof, r->pf.ent_off);
   up(S, st, tb, r->t_esf, r->pf.ent_slot);
@@ -619,7 +710,14 @@ int admit_device(dfg_server_s* S, Req* r, dfg_server_s::AdmLane& lane) {
     ++nl;
   }
   // the factor into the step records
-  for (int dir = 0; dir < 2; ++dir) {
+  for (int dir = 0; dir < 2 && r->strips; ++dir) {
+    const StripPlan& Q = r->strip[dir];
+    const StripPackArgs pa{Q.d, Q.ne, b, Q.steps(), at<unsigned char>(S, pb, r->o_srec[dir]),
+                           at<int>(S, tb, r->t_sslot[dir]), at<int>(S, tb, r->t_srows[dir]), fd, fo};
+    SCK(launch_strip_pack(dir == 0, S->fp32, pa, st));
+    nl += 2;
+  }
+  for (int dir = 0; dir < 2 && !r->strips; ++dir) {
     const SweepPlan& pl = dir == 0 ? r->pf : r->pb;
     PackArgs pa{};
     pa.nsteps = pl.nsteps;
@@ -642,8 +740,12 @@ int admit_device(dfg_server_s* S, Req* r, dfg_server_s::AdmLane& lane) {
     SCK(srv_init_vectors(m, rhs, at<double>(S, pb, r->o_r), at<double>(S, pb, r->o_x), at<double>(S, pb, r->o_p),
                          at<void>(S, pb, r->o_y), at<void>(S, pb, r->o_z),
                          S->fp32 ? at<float>(S, pb, r->o_r32) : nullptr, S->fp32, st));
-  if (r->solo) {  // the first forward input, in the forward plan's step order
+  if (r->solo || r->strips) {  // the first forward input, in the forward plan's step order
     SCK(srv_permute_rhs(slot_of(S, r), S->fp32, st));
+    ++nl;
+  }
+  if (r->strips) {
+    SCK(fill_sentinel(r->nxch(), at<void>(S, pb, r->o_sxch), S->fp32, st));
     ++nl;
   }
   Red red{lane.d_red, reinterpret_cast<unsigned*>(lane.d_red + kRedGrid), lane.d_red + kRedGrid + 8};
@@ -668,6 +770,7 @@ void finish_locked(dfg_server_s* S, Req* r) {
   r->gm = GatherMap{}; r->sell = SellMap{}; r->lev = Levels{}; r->ilu = IluPlan{}; r->pf = SweepPlan{}; r->pb = SweepPlan{};
   r->hf = {}; r->hb = {}; r->of = {}; r->ob = {};
   r->chf = {}; r->chb = {}; r->posf = {};
+  for (int dir = 0; dir < 2; ++dir) { r->strip[dir] = StripPlan{}; r->smeta[dir] = {}; }
   ++S->n_finished;
   S->cv_done.notify_all();
 }
@@ -837,9 +940,13 @@ SrvSlot slot_of(dfg_server_s* S, Req* r) {
   s.r32 = S->fp32 ? at<float>(S, pb, r->o_r32) : nullptr;
   s.st = at<PcgState>(S, pb, r->o_st);
   s.cnt = at<unsigned>(S, pb, r->o_cnt);
-  if (r->solo) {
+  if (r->solo || r->strips) {
     s.posf = at<int>(S, pb, r->o_posf);
     s.rperm = at<void>(S, pb, r->o_rperm);
+  }
+  if (r->strips) {
+    s.xch = at<void>(S, pb, r->o_sxch);
+    s.nx = r->nxch();
   }
   if (S->mixed) {
     s.r = s.p = s.q = nullptr;
@@ -879,6 +986,38 @@ int upload_table(dfg_server_s* S, Group& G) {
       G.h_sb[k * 2 + dir].range_start[0] = 0;
       G.h_solo[k * 2 + dir].nslots = 0;
     }
+  for (int k = 0; k < kStripClasses * 2; ++k) {
+    G.h_strip[k].nslots = 0;
+    G.h_strip[k].group_start[0] = 0;
+  }
+  // strips: longest chains first
+  std::vector<int> order;
+  for (int i = 0; i < (int)act.size(); ++i)
+    if (act[i]->strips) order.push_back(i);
+  std::stable_sort(order.begin(), order.end(),
+                   [&](int x, int y) { return act[x]->strip[0].nchunks > act[y]->strip[0].nchunks; });
+  for (int i : order) {
+    Req* r = act[i];
+    const SrvSlot& sl = T->slot[i];
+    for (int dir = 0; dir < 2; ++dir) {
+      const StripPlan& Q = r->strip[dir];
+      const int k = strip_class_index(r->b, Q.ne);
+      mask |= 1 << (kStripBit + k);
+      StripBatch& B = G.h_strip[k * 2 + dir];
+      const int j = B.nslots++;
+      StripSlot& w = B.slot[j];
+      w.rec = at<unsigned char>(S, r->pbase, r->o_srec[dir]);
+      w.strip_chunk = at<int>(S, r->pbase, r->o_schunk[dir]);
+      w.item_ptr = at<int>(S, r->pbase, r->o_sip[dir]);
+      w.items = at<int2>(S, r->pbase, r->o_sit[dir]);
+      w.in = dir == 0 ? sl.rperm : sl.y;  // both in this sweep's step order
+      w.out = dir == 0 ? sl.y : sl.z;     // y in the backward sweep's step order, z in row order
+      w.xch = static_cast<unsigned char*>(sl.xch) + (dir == 0 ? 0 : (size_t)r->strip[0].nexport * r->strip[0].d.VS);
+      w.done = &sl.st->done;
+      w.nstrips = Q.nstrips;
+      B.group_start[j + 1] = B.group_start[j] + (Q.nstrips + kServeStripWarps - 1) / kServeStripWarps;
+    }
+  }
   // solo sweeps: largest solves first, so the last CTA to start has the
   // least left to do
   std::vector<int> solo_order;
@@ -906,7 +1045,7 @@ int upload_table(dfg_server_s* S, Group& G) {
   }
   for (int i = 0; i < (int)act.size(); ++i) {
     Req* r = act[i];
-    if (r->solo) continue;
+    if (r->solo || r->strips) continue;
     mask |= 1 << r->cls;
     for (int dir = 0; dir < 2; ++dir) {
       SweepBatch& B = G.h_sb[r->cls * 2 + dir];
@@ -928,6 +1067,10 @@ int upload_table(dfg_server_s* S, Group& G) {
   SCK(cudaMemcpyAsync(G.d_tab, G.h_tab, tab_bytes, cudaMemcpyHostToDevice, G.s_iter));
   SCK(cudaMemcpyAsync(G.d_sb, G.h_sb, sizeof(SweepBatch) * kClasses * 2, cudaMemcpyHostToDevice, G.s_iter));
   SCK(cudaMemcpyAsync(G.d_solo, G.h_solo, sizeof(SoloBatch) * kClasses * 2, cudaMemcpyHostToDevice, G.s_iter));
+  for (int k = 0; k < kStripClasses * 2; ++k)  // the used prefix of each strip batch
+    SCK(cudaMemcpyAsync(G.d_strip + k, G.h_strip + k,
+                        offsetof(StripBatch, slot) + sizeof(StripSlot) * (size_t)G.h_strip[k].nslots,
+                        cudaMemcpyHostToDevice, G.s_iter));
   return mask;
 }
 
@@ -954,6 +1097,17 @@ SoloArgs solo_args(dfg_server_s* S, Group& G, int k, int dir) {
   a.NS = S->solo_ns[k][dir];
   a.R = S->solo_R[k];
   a.max_nent = class_maxe(k);
+  return a;
+}
+
+StripArgs strip_args(dfg_server_s* S, Group& G, int k, int dir) {
+  StripArgs a{};
+  a.batch = G.d_strip + k * 2 + dir;
+  a.ticket = G.d_tickets + kClasses * 4 + k * 2 + dir;
+  a.err = reinterpret_cast<int*>(G.d_stat + sizeof(SrvStatus) * kSrvMaxSlots);
+  a.ne = kStripNe[k % 4];
+  a.W = kServeStripWarps;
+  a.NS = S->strip_ns[k][dir];
   return a;
 }
 
@@ -991,7 +1145,9 @@ cudaGraphExec_t capture_graph(dfg_server_s* S, Group& G, int mask, bool prof) {
     SCK(cudaEventRecord(G.ev_fork, G.s_iter));
     for (int k = 0; k < kClasses; ++k) {
       const bool ranged = mask >> k & 1, solo = mask >> (kClasses + k) & 1;
-      if (!ranged && !solo) continue;
+      bool strips = false;
+      for (int q = 0; q < kStripClasses; ++q) strips |= strip_host_class(q) == k && (mask >> (kStripBit + q) & 1);
+      if (!ranged && !solo && !strips) continue;
       SCK(cudaStreamWaitEvent(G.s_side[k], G.ev_fork, 0));
       for (int dir = 0; dir < 2; ++dir) {
         mk(6 + 2 * k + dir, 0, G.s_side[k]);
@@ -1001,14 +1157,18 @@ cudaGraphExec_t capture_graph(dfg_server_s* S, Group& G, int mask, bool prof) {
         if (solo)
           SCK(launch_solo(dir == 0, S->fp32, class_b(k), solo_args(S, G, k, dir), S->solo_grid[k],
                           S->solo_smem[k][dir], G.s_side[k]));
+        for (int q = 0; q < kStripClasses; ++q)
+          if (strip_host_class(q) == k && (mask >> (kStripBit + q) & 1))
+            SCK(launch_strip(dir == 0, S->fp32, class_b(k), strip_args(S, G, q, dir), S->strip_grid[q],
+                             S->strip_smem[q][dir], G.s_side[k], false));
         mk(6 + 2 * k + dir, 1, G.s_side[k]);
       }
       SCK(cudaEventRecord(G.ev_join[k], G.s_side[k]));
       SCK(cudaStreamWaitEvent(G.s_iter, G.ev_join[k], 0));
     }
     mk(0, 0, G.s_iter);
-    if (S->mixed) SCK(srvm_rz_beta(G.d_tab, G.d_partials, G.d_tickets, kClasses * 4, grid, G.s_iter));
-    else SCK(srv_rz_beta(G.d_tab, G.d_partials, G.d_tickets, kClasses * 4, S->fp32, grid, G.s_iter));
+    if (S->mixed) SCK(srvm_rz_beta(G.d_tab, G.d_partials, G.d_tickets, kTickets, grid, G.s_iter));
+    else SCK(srv_rz_beta(G.d_tab, G.d_partials, G.d_tickets, kTickets, S->fp32, grid, G.s_iter));
     mk(0, 1, G.s_iter);
     mk(1, 0, G.s_iter);
     if (S->mixed) SCK(srvm_update_p(G.d_tab, grid, G.s_iter));
@@ -1072,8 +1232,13 @@ void account_profile(dfg_server_s* S, Group& G) {
   }
   std::lock_guard<std::mutex> lk(S->mu);
   for (int k = 0; k < DFG_SERVER_NKERNELS; ++k) {
-    if (k >= 6 && !((G.graph_mask >> ((k - 6) / 2)) & 1) && !((G.graph_mask >> (kClasses + (k - 6) / 2)) & 1))
-      continue;
+    if (k >= 6) {
+      const int c = (k - 6) / 2;
+      bool present = (G.graph_mask >> c & 1) || (G.graph_mask >> (kClasses + c) & 1);
+      for (int q = 0; q < kStripClasses; ++q)
+        present |= strip_host_class(q) == c && (G.graph_mask >> (kStripBit + q) & 1);
+      if (!present) continue;
+    }
     float ms = 0.f;
     if (cudaEventElapsedTime(&ms, G.ev_prof[2 * k], G.ev_prof[2 * k + 1]) != cudaSuccess) {
       cudaGetLastError();
@@ -1087,7 +1252,7 @@ void account_profile(dfg_server_s* S, Group& G) {
 
 int kernels_per_replay(dfg_server_s* S, const Group& G) {
   int nc = 0;
-  for (int k = 0; k < 2 * kClasses; ++k) nc += (G.graph_mask >> k) & 1;
+  for (int k = 0; k < kStripBit + kStripClasses; ++k) nc += (G.graph_mask >> k) & 1;
   // per iteration: the sweeps, four batched kernels, and (outside the mixed
   // form) the three finishing launches of their per-slot reductions
   return S->chunk * (2 * nc + 4 + (S->mixed ? 0 : 3)) + 3;
@@ -1128,7 +1293,7 @@ void harvest(dfg_server_s* S, Group& G, std::vector<Req*>& retiring) {
   G.act.swap(keep);
   if (err != 0) {
     SCK(cudaMemsetAsync(G.d_stat + sizeof(SrvStatus) * kSrvMaxSlots, 0, 16, G.s_iter));
-    SCK(cudaMemsetAsync(G.d_tickets, 0, sizeof(int) * kClasses * 4, G.s_iter));
+    SCK(cudaMemsetAsync(G.d_tickets, 0, sizeof(int) * kTickets, G.s_iter));
     SCK(cudaStreamSynchronize(G.s_iter));
   }
 }
@@ -1268,6 +1433,21 @@ void class_shapes(dfg_server_s* S) {
     const int per_sm = std::max(1, std::min(16, (int)(per_sm_bytes / (worst + 1024))));
     S->cls_grid[k] = S->nsm * per_sm;
   }
+  // strip sweeps: one strip per CTA, two chunk stages or more, about four CTAs
+  // per SM
+  for (int k = 0; k < kStripClasses; ++k) {
+    const int b = k / 4 + 1;
+    size_t worst = 0;
+    for (int dir = 0; dir < 2; ++dir) {
+      const StripDims d = strip_dims(b, elem, dir == 0, kStripNe[k % 4]);
+      int ns = 8;
+      while (ns > 2 && strip_smem_bytes(d, kServeStripWarps, ns) > (size_t)per_sm_bytes / 4 - 1024) --ns;
+      S->strip_smem[k][dir] = strip_smem_bytes(d, kServeStripWarps, ns);
+      S->strip_ns[k][dir] = S->strip_smem[k][dir] <= S->ctx->smem_optin ? ns : 0;
+      worst = std::max(worst, S->strip_smem[k][dir]);
+    }
+    S->strip_grid[k] = S->nsm * std::max(1, std::min(8, (int)(per_sm_bytes / (worst + 1024))));
+  }
   // solo sweeps: one CTA per SM (solo_shape)
   for (int k = 0; k < kClasses; ++k) {
     const int b = class_b(k), maxe = class_maxe(k);
@@ -1354,22 +1534,26 @@ extern "C" int dfg_server_create(dfg_ctx ctx, const dfg_server_config* cfg, dfg_
       SCK(cudaMalloc(&G.d_tab, sizeof(SrvTable)));
       SCK(cudaMalloc(&G.d_sb, sizeof(SweepBatch) * kClasses * 2));
       SCK(cudaMalloc(&G.d_solo, sizeof(SoloBatch) * kClasses * 2));
-      SCK(cudaMalloc(&G.d_tickets, sizeof(int) * kClasses * 4));
+      SCK(cudaMalloc(&G.d_strip, sizeof(StripBatch) * kStripClasses * 2));
+      SCK(cudaMalloc(&G.d_tickets, sizeof(int) * kTickets));
       SCK(cudaMalloc(&G.d_partials, sizeof(double) * kMaxChunks));
       SCK(cudaMalloc(&G.d_chunk_slot, kMaxChunks));
       SCK(cudaHostAlloc(&G.h_chunk_slot, kMaxChunks, cudaHostAllocDefault));
       SCK(cudaMalloc(&G.d_stat, sizeof(SrvStatus) * kSrvMaxSlots + 64));
-      SCK(cudaMemset(G.d_tickets, 0, sizeof(int) * kClasses * 4));
+      SCK(cudaMemset(G.d_tickets, 0, sizeof(int) * kTickets));
+      SCK(cudaMemset(G.d_strip, 0, sizeof(StripBatch) * kStripClasses * 2));
       SCK(cudaMemset(G.d_solo, 0, sizeof(SoloBatch) * kClasses * 2));
       SCK(cudaMemset(G.d_stat, 0, sizeof(SrvStatus) * kSrvMaxSlots + 64));
       SCK(cudaMemset(G.d_sb, 0, sizeof(SweepBatch) * kClasses * 2));
       SCK(cudaHostAlloc(&G.h_tab, sizeof(SrvTable), cudaHostAllocDefault));
       SCK(cudaHostAlloc(&G.h_sb, sizeof(SweepBatch) * kClasses * 2, cudaHostAllocDefault));
       SCK(cudaHostAlloc(&G.h_solo, sizeof(SoloBatch) * kClasses * 2, cudaHostAllocDefault));
+      SCK(cudaHostAlloc(&G.h_strip, sizeof(StripBatch) * kStripClasses * 2, cudaHostAllocDefault));
       SCK(cudaHostAlloc(&G.h_stat, sizeof(SrvStatus) * kSrvMaxSlots + 64, cudaHostAllocDefault));
       std::memset(G.h_tab, 0, sizeof(SrvTable));
       std::memset(G.h_sb, 0, sizeof(SweepBatch) * kClasses * 2);
       std::memset(G.h_solo, 0, sizeof(SoloBatch) * kClasses * 2);
+      std::memset(G.h_strip, 0, sizeof(StripBatch) * kStripClasses * 2);
       std::memset(G.h_stat, 0, sizeof(SrvStatus) * kSrvMaxSlots + 64);
       SCK(cudaStreamCreateWithPriority(&G.s_iter, cudaStreamNonBlocking, hi));
       for (int k = 0; k < kClasses; ++k) {
@@ -1383,6 +1567,7 @@ extern "C" int dfg_server_create(dfg_ctx ctx, const dfg_server_config* cfg, dfg_
     }
     SCK(sweep_set_smem_limits(ctx->smem_optin));
     SCK(solo_set_smem_limits(ctx->smem_optin));
+    SCK(strip_set_smem_limits(ctx->smem_optin));
     class_shapes(S.get());
   } catch (const CudaFail& f) {
     cudaGetLastError();
@@ -1563,10 +1748,10 @@ extern "C" int dfg_server_destroy(dfg_server s) {
     for (cudaEvent_t e : {G.ev_fork, G.ev_done})
       if (e) cudaEventDestroy(e);
     if (G.s_iter) cudaStreamDestroy(G.s_iter);
-    for (void* p : {(void*)G.d_tab, (void*)G.d_sb, (void*)G.d_solo, (void*)G.d_tickets, (void*)G.d_partials,
+    for (void* p : {(void*)G.d_tab, (void*)G.d_sb, (void*)G.d_solo, (void*)G.d_strip, (void*)G.d_tickets, (void*)G.d_partials,
                     (void*)G.d_stat, (void*)G.d_chunk_slot})
       if (p) cudaFree(p);
-    for (void* p : {(void*)G.h_tab, (void*)G.h_sb, (void*)G.h_solo, (void*)G.h_stat, (void*)G.h_chunk_slot})
+    for (void* p : {(void*)G.h_tab, (void*)G.h_sb, (void*)G.h_solo, (void*)G.h_strip, (void*)G.h_stat, (void*)G.h_chunk_slot})
       if (p) cudaFreeHost(p);
   }
   for (auto& a : s->adm) {

@@ -233,13 +233,14 @@ int dfg_precond_set_fill_level(dfg_precond prec, int lev);
 int dfg_precond_set_linear_system(dfg_precond prec, dfg_system sys);
 /* How the triangular sweeps are scheduled (no counterpart in the reference,
  * whose substitutions are sequential loops): 0 (default) times the kinds
- * on the device at the symbolic set-up and keeps the fastest per direction;
- * 1 = ranged (contiguous row ranges pipelined across CTAs, good for the long
- * thin wavefronts of large 2D meshes); 2 = level-scheduled (one launch per
- * dependency level, good for the wide levels of 3D meshes); 3 = one CTA
- * (the whole sweep on one SM, level after level, its input first permuted
- * into the schedule's order: good for small 2D meshes, whose sweeps are
- * bound by the latency of each level).  Takes effect at the next
+ * on the device at the symbolic set-up and keeps the faster; 1 = ranged (rows
+ * pipelined across CTAs: in strips of grid lines, a warp each, where the rows
+ * fit them, else in contiguous row ranges); 2 = level-scheduled (one launch per
+ * dependency level, good for matrices with few wide levels, such as those of
+ * unordered meshes); 3 = one CTA (the whole sweep on one SM, level after
+ * level, its input first permuted into the schedule's order).  Where the rows
+ * fit strips, 0 chooses between 1 and 2 for both directions together; else
+ * among all three kinds per direction.  Takes effect at the next
  * dfg_precond_set_linear_system; results agree to rounding. */
 int dfg_precond_set_sweep_mode(dfg_precond prec, int mode);
 /* The kind chosen per direction after the symbolic set-up (1, 2 or 3). */
@@ -374,9 +375,10 @@ typedef struct {
   int profile_every;      /* every n-th replay times its first iteration per kernel; 0 = never */
   int size_groups;        /* solves grouped by size, each group iterating at its own pace on its own
                              streams: 1 = one table for all, 2-3 groups; 0 = 3 */
-  int sweeps;             /* triangular-sweep kernel: 0 = per solve (FP32 sweeps one CTA per solve
-                             except 3x3-block solves above 100,000 nodes; FP64 sweeps ranged over
-                             several CTAs), 1 = ranged, 2 = one CTA per solve; the same bits either way */
+  int sweeps;             /* triangular-sweep kernel: 0 = strips (a warp per strip of grid lines) where a
+                             solve's rows fit them, else one CTA per solve in FP32 (except 3x3-block
+                             solves above 100,000 nodes) and ranged over several CTAs otherwise,
+                             1 = ranged, 2 = one CTA per solve; the same bits either way */
 } dfg_server_config;
 
 /* kind: 1 Poisson 2D (P1 triangles), 2 Poisson 3D (P1 tetrahedra),

@@ -61,3 +61,20 @@ def test_strip_sweeps(gpu_ctx, oracle_lib, name, fill):
             s.close()
     for a, c in zip(got[1], got[3]):
         assert np.array_equal(a, c)
+
+
+@pytest.mark.parametrize("mode", ["fp64", "fp32f", "mixed"])
+def test_served_strips(gpu_ctx, mode):
+    """The server's strip sweeps (several solves and strips per launch) against
+    its one-CTA sweeps: the same bits and iteration counts."""
+    from delfem_gb300.serve import Server
+    probs = [_problem(n) for n in ("poisson2d:31x31", "poisson2d:20x150", "solid2d:33x12", "solid2d:40x70",
+                                   "poisson3d:12x9x8", "solid3d:7x11x6")]
+    got = []
+    for sweeps in (0, 2):
+        with Server(gpu_ctx, mode=mode, budget_bytes=512 << 20, sweeps=sweeps) as S:
+            ids = [S.submit(p) for p in probs]
+            got.append([S.wait(i) for i in ids])
+    for a, c in zip(*got):
+        assert a["status"] == 0 and a["rel_true"] <= 1e-8 and a["iterations"] == c["iterations"]
+        assert np.array_equal(a["x"], c["x"])
