@@ -32,6 +32,7 @@ SOURCES = {
     "k_solo.cu": [],
     "k_solve.cu": [],
     "k_bicg.cu": [],
+    "k_iter.cu": [],
     "k_level.cu": [],
     "k_pattern.cu": [],
     "k_assemble.cu": ["-fmad=false"],

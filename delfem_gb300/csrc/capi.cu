@@ -126,6 +126,11 @@ Red red_of(dfg_ctx c, int channel = 0) {
   return Red{s.partials, s.counters + channel, s.results + channel};
 }
 
+IterRed iter_red_of(dfg_ctx c) {
+  return IterRed{c->iter_red.as<double>(),
+                 reinterpret_cast<unsigned*>(c->iter_red.as<char>() + 3 * kRedGrid * 8), c->err_word.as<int>()};
+}
+
 double* vec_ptr(dfg_ctx ctx_, dfg_system s, int iv) {
   if (iv == -1) return s->res.as<double>();
   if (iv == -2) return s->upd.as<double>();
@@ -253,6 +258,8 @@ extern "C" int dfg_ctx_create(int device, dfg_ctx* out) {
     dalloc(c, c->scratch, kRedGrid * 8 + 16 * 4 + 16 * 8 + 16 * 4 + 256);
     CK(cudaMemsetAsync(c->err_word.p, 0, 64, c->stream));
     CK(cudaMemsetAsync(c->scratch.p, 0, c->scratch.bytes, c->stream));
+    dalloc(c, c->iter_red, 3 * kRedGrid * 8 + 64);
+    CK(cudaMemsetAsync(c->iter_red.p, 0, c->iter_red.bytes, c->stream));
     CK(sweep_set_smem_limits(c->smem_optin));
     CK(cudaStreamSynchronize(c->stream));
     return DFG_OK;
@@ -273,6 +280,7 @@ extern "C" int dfg_ctx_destroy(dfg_ctx ctx) {
   cudaStreamSynchronize(ctx->stream);
   ctx->err_word.release();
   ctx->scratch.release();
+  ctx->iter_red.release();
   cudaStreamDestroy(ctx->stream);
   delete ctx;
   return DFG_OK;
@@ -1819,6 +1827,7 @@ int timeout_status(dfg_ctx ctx_) {
   int w[4] = {0, 0, 0, 0};
   CK(cudaMemcpyAsync(w, ctx_->err_word.p, sizeof(w), cudaMemcpyDeviceToHost, ctx_->stream));
   CK(cudaMemsetAsync(ctx_->err_word.p, 0, sizeof(w), ctx_->stream));
+  CK(cudaMemsetAsync(ctx_->iter_red.p, 0, ctx_->iter_red.bytes, ctx_->stream));  // a grid barrier left half-way
   CK(cudaStreamSynchronize(ctx_->stream));
   set_err(ctx_, "a triangular-sweep wait timed out (site " + std::to_string(w[1]) + ", slot " +
                     std::to_string(w[2]) + ", range/row " + std::to_string(w[3]) + ")");
@@ -1889,27 +1898,26 @@ static int solve_pcg_f64vec(dfg_system sys, dfg_precond prec, bool fp32z, bool t
     run_sweep(ctx, F);
     run_sweep(ctx, B);
     CK(pcg_after_precond0(v, st, red, fp32z, ctx->stream));
-    launched(ctx, 2);
-    PcgState h{};
-    read_state(ctx, st, h);
-    // iterations: a graph of `chunk` iterations, replayed until done
-    const long long per_it = 4 + launches_of(F) + launches_of(B);
-    // level-scheduled sweeps put one graph node per level: fewer iterations per graph
-    const int chunk = std::max(2, std::min(m < 200000 ? 8 : 32, (int)(4096 / per_it)));
     ensure_sell(ctx, sys, false);
     const MatView A = view64(sys);
+    const IterRed ired = iter_red_of(ctx);
+    CK(pcg_iter(A, v, st, ired, sc.tickets, fp32z, true, ctx->nsm, ctx->stream));
+    launched(ctx, 3);
+    PcgState h{};
+    read_state(ctx, st, h);
+    // iterations from the preconditioner on: a graph of `chunk` of them,
+    // replayed until done
+    const long long per_it = 1 + launches_of(F) + launches_of(B);
+    // level-scheduled sweeps put one graph node per level: fewer iterations per graph
+    const int chunk = std::max(2, std::min(m < 200000 ? 8 : 32, (int)(4096 / per_it)));
     Chunk g;
     CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     for (int c = 0; c < chunk; ++c) {
-      // each kernel after the chunk's first starts as a programmatic
-      // dependent of the one before: its launch overlaps that kernel, and it
-      // waits for it at entry
-      pcg_spmv_pap(A, v, st, red, ctx->stream, c > 0);
-      pcg_update_rx(v, st, red, sc.tickets, fp32z, ctx->stream, true);
-      enqueue_sweep(F, ctx->stream, true);
+      // the sweeps start as programmatic dependents of the kernel before them:
+      // their launch overlaps it, and they wait for it at entry
+      enqueue_sweep(F, ctx->stream, c > 0);
       enqueue_sweep(B, ctx->stream, true);
-      pcg_rz_beta(v, st, red, fp32z, ctx->stream, true);
-      pcg_update_p(v, st, fp32z, ctx->stream, true);
+      pcg_iter(A, v, st, ired, sc.tickets, fp32z, false, ctx->nsm, ctx->stream);
     }
     CK(cudaStreamEndCapture(ctx->stream, &g.graph));
     CK(cudaGraphInstantiate(&g.exec, g.graph, 0));
@@ -1942,13 +1950,9 @@ static int solve_pcg_f64vec(dfg_system sys, dfg_precond prec, bool fp32z, bool t
         if (rel > tol) h.done = 2;
         break;
       }
-      // continue from the true residual: finish this iteration and resume
+      // continue from the true residual
       CK(pcg_replace(v, st, sc.tickets, fp32z, ctx->stream));
-      run_sweep(ctx, F);
-      run_sweep(ctx, B);
-      CK(pcg_rz_beta(v, st, red, fp32z, ctx->stream));
-      CK(pcg_update_p(v, st, fp32z, ctx->stream));
-      launched(ctx, 3);
+      launched(ctx, 1);
       read_state(ctx, st, h);
     }
     *conv_ratio = h.conv;
@@ -2038,18 +2042,17 @@ extern "C" int dfg_solve_pcg_mixed(dfg_system sys, dfg_precond prec, double* con
     run_sweep(ctx, F);
     run_sweep(ctx, B);
     CK(mix_after_precond0(v, st, red, ctx->stream));
-    launched(ctx, 4);
-    const long long per_it = 4 + launches_of(F) + launches_of(B);
+    const IterRed ired = iter_red_of(ctx);
+    CK(mix_iter(A32, v, st, ired, sc.tickets, true, ctx->nsm, ctx->stream));
+    launched(ctx, 5);
+    const long long per_it = 1 + launches_of(F) + launches_of(B);
     const int chunk = std::max(2, std::min(m < 200000 ? 8 : 32, (int)(4096 / per_it)));
     Chunk g;
     CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     for (int c = 0; c < chunk; ++c) {
-      mix_spmv_pap(A32, v, st, red, ctx->stream);
-      mix_update_rx(v, st, red, sc.tickets, ctx->stream);
-      enqueue_sweep(F, ctx->stream);
-      enqueue_sweep(B, ctx->stream);
-      mix_rz_beta(v, st, red, ctx->stream);
-      mix_update_p(v, st, ctx->stream);
+      enqueue_sweep(F, ctx->stream, c > 0);
+      enqueue_sweep(B, ctx->stream, true);
+      mix_iter(A32, v, st, ired, sc.tickets, false, ctx->nsm, ctx->stream);
     }
     CK(cudaStreamEndCapture(ctx->stream, &g.graph));
     CK(cudaGraphInstantiate(&g.exec, g.graph, 0));
@@ -2079,14 +2082,9 @@ extern "C" int dfg_solve_pcg_mixed(dfg_system sys, dfg_precond prec, double* con
       if (!(rel == rel)) { status = DFG_NAN_DETECTED; set_err(ctx, "NaN in the residual"); break; }
       if (rel <= tol) { status = DFG_OK; break; }
       if (h.done == 2) { set_err(ctx, "mixed PCG did not converge within the iteration limit"); break; }
-      // continue the recursion from the true residual: finish this iteration
-      // (preconditioner, beta, direction) and resume the graph
+      // continue the recursion from the true residual
       CK(mix_replace(v, st, sc.tickets, ctx->stream));
-      run_sweep(ctx, F);
-      run_sweep(ctx, B);
-      CK(mix_rz_beta(v, st, red, ctx->stream));
-      CK(mix_update_p(v, st, ctx->stream));
-      launched(ctx, 3);
+      launched(ctx, 1);
     }
     *conv_ratio = rel;
     *iteration = (unsigned)h.iter_out;

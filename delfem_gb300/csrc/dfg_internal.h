@@ -238,6 +238,7 @@ struct dfg_ctx_s {
   long long launches = 0;
   dfg::DBuf err_word;     // int, device error word (dfg::kErr*)
   dfg::DBuf scratch;      // reduction partials + scalars
+  dfg::DBuf iter_red;     // k_iter.cu: partials, grid barrier
   int* h_pinned = nullptr;  // small pinned host area for status reads
   int last_timeout_site = 0;  // wait site of the last reported timeout
 };

@@ -181,7 +181,7 @@ static size_t ilu_group_bytes(int b, int maxrow, int maxlow, int maxu) {
 constexpr int kIluWarps = 4;  // per CTA, one per scheduler
 
 template <int B>
-__global__ void __launch_bounds__(kIluWarps * 32) k_ilu(IluArgs a, size_t group_bytes) {
+__global__ void __launch_bounds__(kIluWarps * 32, 2) k_ilu(IluArgs a, size_t group_bytes) {
   constexpr int BS = B * B, G = IluLanes<B>::G, J = IluLanes<B>::J;
   extern __shared__ __align__(16) unsigned char smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

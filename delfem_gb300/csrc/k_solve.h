@@ -77,13 +77,12 @@ struct PcgVecs {
 // fp32z: the preconditioned vectors y, z are float (FP32 factor and sweeps)
 cudaError_t pcg_init(const PcgVecs& v, PcgState* st, Red red, double tol, int maxit, int* tickets, bool fp32z, cudaStream_t s);
 cudaError_t pcg_after_precond0(const PcgVecs& v, PcgState* st, Red red, bool fp32z, cudaStream_t s);
-// dep (the four iteration kernels): launch as a programmatic dependent of the
-// previous kernel in the stream, which must be a kernel (a graph's chain)
-cudaError_t pcg_spmv_pap(const MatView& A, const PcgVecs& v, PcgState* st, Red red, cudaStream_t s, bool dep = false);
-cudaError_t pcg_update_rx(const PcgVecs& v, PcgState* st, Red red, int* tickets, bool fp32z, cudaStream_t s,
-                          bool dep = false);
-cudaError_t pcg_rz_beta(const PcgVecs& v, PcgState* st, Red red, bool fp32z, cudaStream_t s, bool dep = false);
-cudaError_t pcg_update_p(const PcgVecs& v, PcgState* st, bool fp32z, cudaStream_t s, bool dep = false);
+// the four parts of an iteration that pcg_iter does in one launch (k_iter.cu),
+// as launches of their own: dfg_profile_kernels times them
+cudaError_t pcg_spmv_pap(const MatView& A, const PcgVecs& v, PcgState* st, Red red, cudaStream_t s);
+cudaError_t pcg_update_rx(const PcgVecs& v, PcgState* st, Red red, int* tickets, bool fp32z, cudaStream_t s);
+cudaError_t pcg_rz_beta(const PcgVecs& v, PcgState* st, Red red, bool fp32z, cudaStream_t s);
+cudaError_t pcg_update_p(const PcgVecs& v, PcgState* st, bool fp32z, cudaStream_t s);
 // rd = b - A x, rr = rd.rd (into st->rr; state otherwise untouched)
 cudaError_t pcg_true_residual(const MatView& A, const PcgVecs& v, PcgState* st, Red red, cudaStream_t s);
 // r = rd (and the sweeps' feed), tickets reset, done = 0: continue from the true residual
@@ -109,6 +108,7 @@ cudaError_t mix_replace(const MixVecs& v, PcgState* st, int* tickets, cudaStream
 // first call: state reset for a solve (tolerance, limits)
 cudaError_t mix_start(PcgState* st, double tol, double bb, double delta, int maxit, cudaStream_t s);
 cudaError_t mix_after_precond0(const MixVecs& v, PcgState* st, Red red, cudaStream_t s);
+// the parts of mix_iter, as above
 cudaError_t mix_spmv_pap(const MatView& A32, const MixVecs& v, PcgState* st, Red red, cudaStream_t s);
 cudaError_t mix_update_rx(const MixVecs& v, PcgState* st, Red red, int* tickets, cudaStream_t s);
 cudaError_t mix_rz_beta(const MixVecs& v, PcgState* st, Red red, cudaStream_t s);
@@ -117,6 +117,19 @@ cudaError_t mix_update_p(const MixVecs& v, PcgState* st, cudaStream_t s);
 cudaError_t mix_accumulate(const MixVecs& v, cudaStream_t s);
 cudaError_t mix_clear_done(PcgState* st, cudaStream_t s);
 cudaError_t to_fp32(long long m, const double* a, float* b, cudaStream_t s);
+
+// ---- one iteration between two preconditioner applications (k_iter.cu) ----
+// r.z, beta, the direction (unless `first`), A p, alpha, the r/x update with
+// the stop test and the sweeps' feed
+struct IterRed {
+  double* part;   // 3 x kRedGrid
+  unsigned* bar;  // zero between launches
+  int* err;       // device error word
+};
+cudaError_t pcg_iter(const MatView& A, const PcgVecs& v, PcgState* st, IterRed red, int* tickets, bool fp32z,
+                     bool first, int nsm, cudaStream_t s);
+cudaError_t mix_iter(const MatView& A32, const MixVecs& v, PcgState* st, IterRed red, int* tickets, bool first,
+                     int nsm, cudaStream_t s);
 
 // ---- preconditioned BiCGSTAB (k_bicg.cu) ----------------------------------
 struct BicgState {

@@ -22,12 +22,12 @@
 //     arrive.  `delivered` counts the arrived prefix; a step says how many
 //     items it needs, one compare when they are there.
 // Measured on GB300, FP32, per sweep (forward / backward): the 1000x500
-// cantilever 0.15 / 0.14 ms (ranged kernel 1.09 / 1.10), Poisson on 301x257
-// cells 49 / 46 us (one CTA per sweep 200 / 196), elasticity on 56^3 cells 107 /
-// 100 us (a launch per level 345 / 306).  FP64: the cantilever 0.65 / 0.50 ms
-// (2.36 / 2.08), Poisson on 128x128 cells 69 / 59 us (133 / 123).  Inside one
-// strip a level costs 115 (1x1 blocks) to 400 (3x3, 7 entries) cycles in FP32
-// and 420 to 2,100 in FP64, where each warp-wide FMA takes its scheduler 64; a
+// cantilever 0.14 / 0.13 ms (ranged kernel 1.09 / 1.10), Poisson on 301x257
+// cells 47 / 46 us (one CTA per sweep 200 / 196), elasticity on 56^3 cells 102 /
+// 96 us (a launch per level 345 / 306).  FP64: the cantilever 0.64 / 0.48 ms
+// (2.36 / 2.08), Poisson on 128x128 cells 67 / 56 us (133 / 123).  Inside one
+// strip a level costs 110 (1x1 blocks) to 330 (3x3, 7 entries) cycles in FP32
+// and 400 to 2,000 in FP64, where each warp-wide FMA takes its scheduler 64; a
 // hand-off between strips costs 1,500 to 3,000, of which the L2 takes 600-900.
 //
 // Strips are claimed in order, W per CTA, through a ticket, so a strip only
@@ -198,8 +198,10 @@ __device__ __forceinline__ void receive(const StripSlot& S, int r, unsigned char
   }
 }
 
+// (one CTA per SM in the bounds: without it ptxas aims at several and keeps
+// steps to 64 registers and fewer, 2 to 10 % slower)
 template <typename T, int B, bool FWD, int NE>
-__global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32) k_strip(StripArgs a) {
+__global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(StripArgs a) {
   constexpr int SZ = (int)sizeof(T);
   constexpr StripDims D = strip_dims(B, SZ, FWD, NE);
   constexpr int LPR = D.LPR, RW = D.RW, MC = D.MC, VC = D.VC, CH = D.CH, VS = D.VS;

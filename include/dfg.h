@@ -328,7 +328,8 @@ int dfg_solve_pcg_mixed(dfg_system sys, dfg_precond prec, double* conv_ratio,
  * context's stream, averaged over `reps` launches) with the system's current
  * matrix, factor and solver vectors; call after a solve of the same mode.
  * mode: DFG_PREC_FP64 or DFG_PREC_MIXED.  ms[0..5] = SpMV + p.Ap, forward
- * sweep, backward sweep, r/x update + r.r, r.z + beta, p update (ms per launch);
+ * sweep, backward sweep, r/x update + r.r, r.z + beta, p update (ms per launch;
+ * a solve does all but the sweeps in one launch, here each part is its own);
  * bytes[0..2] = algorithmic bytes of one SpMV, forward and backward sweep. */
 int dfg_profile_kernels(dfg_system sys, dfg_precond prec, int mode, int reps, double* ms, double* bytes);
 
