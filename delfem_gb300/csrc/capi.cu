@@ -1250,9 +1250,16 @@ bool setup_strip(dfg_ctx ctx_, dfg_precond pr, const FactorPattern& F, bool forw
   // one strip per CTA while the strips fit the SMs
   D.W = std::min(kStripMaxWarps, std::max(1, (P.nstrips + ctx_->nsm - 1) / ctx_->nsm));
   const size_t budget = ctx_->smem_optin;
+  // As many chunk stages as fit.  FP32 steps are short: they give a strip up
+  // rather than run with two stages, which do not cover a copy (elasticity on
+  // 96^3 cells 183 us per sweep with two strips and four stages, 242 with three and
+  // two; FP64 565 with four and two, 632 with three and three).
   D.NS = 8;
-  while (D.NS > 2 && strip_smem_bytes(D.d, D.W, D.NS) > budget) --D.NS;
-  while (D.W > 1 && strip_smem_bytes(D.d, D.W, D.NS) > budget) --D.W;
+  const int min_ns = fp32 ? 3 : 2;
+  auto too_big = [&] { return strip_smem_bytes(D.d, D.W, D.NS) > budget; };
+  while (D.NS > min_ns && too_big()) --D.NS;
+  while (D.W > 1 && too_big()) --D.W;
+  while (D.NS > 2 && too_big()) --D.NS;
   D.smem = strip_smem_bytes(D.d, D.W, D.NS);
   if (D.smem > budget) return false;
   D.grid = std::min((P.nstrips + D.W - 1) / D.W, ctx_->nsm);

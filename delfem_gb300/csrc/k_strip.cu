@@ -23,10 +23,10 @@
 //     items it needs, one compare when they are there.
 // Measured on GB300, FP32, per sweep (forward / backward): the 1000x500
 // cantilever 0.14 / 0.13 ms (ranged kernel 1.09 / 1.10), Poisson on 301x257
-// cells 47 / 46 us (one CTA per sweep 200 / 196), elasticity on 56^3 cells 102 /
-// 96 us (a launch per level 345 / 306).  FP64: the cantilever 0.64 / 0.48 ms
+// cells 47 / 46 us (one CTA per sweep 200 / 196), elasticity on 56^3 cells 81 /
+// 77 us (a launch per level 345 / 306).  FP64: the cantilever 0.60 / 0.48 ms
 // (2.36 / 2.08), Poisson on 128x128 cells 67 / 56 us (133 / 123).  Inside one
-// strip a level costs 110 (1x1 blocks) to 330 (3x3, 7 entries) cycles in FP32
+// strip a level costs 110 (1x1 blocks) to 640 (3x3, 7 entries) cycles in FP32
 // and 400 to 2,000 in FP64, where each warp-wide FMA takes its scheduler 64; a
 // hand-off between strips costs 1,500 to 3,000, of which the L2 takes 600-900.
 //
@@ -106,6 +106,16 @@ __device__ __forceinline__ void xstore(int on, double* p, const Vec<double, 1>& 
 __device__ __forceinline__ void xstore(int on, float* p, const Vec<float, 2>& y) {
   asm volatile("{\n .reg .pred q;\n setp.ge.s32 q, %0, 0;\n @q st.relaxed.gpu.global.v2.f32 [%1], {%2, %3};\n}" ::"r"(on),
                "l"(p), "f"(y.v[0]), "f"(y.v[1]));
+}
+__device__ __forceinline__ void xstore(int on, float* p, const Vec<float, 4>& y) {
+  asm volatile("{\n .reg .pred q;\n setp.ge.s32 q, %0, 0;\n @q st.relaxed.gpu.global.v4.f32 [%1], {%2, %3, %4, %5};\n}" ::"r"(on),
+               "l"(p), "f"(y.v[0]), "f"(y.v[1]), "f"(y.v[2]), "f"(y.v[3]));
+}
+__device__ __forceinline__ void ostore(int on, float* p, const Vec<float, 4>& y) {  // three elements
+  asm volatile(
+      "{\n .reg .pred q;\n setp.ge.s32 q, %0, 0;\n @q st.global.f32 [%1], %2;\n @q st.global.f32 [%1+4], %3;\n"
+      " @q st.global.f32 [%1+8], %4;\n}" ::"r"(on),
+      "l"(p), "f"(y.v[0]), "f"(y.v[1]), "f"(y.v[2]));
 }
 __device__ __forceinline__ void ostore(int on, float* p, const Vec<float, 1>& y) {
   asm volatile("{\n .reg .pred q;\n setp.ge.s32 q, %0, 0;\n @q st.global.f32 [%1], %2;\n}" ::"r"(on), "l"(p), "f"(y.v[0]));
@@ -211,11 +221,12 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
   constexpr int RHS_CHUNK = CH * D.rhs_bytes;
   // steps per test of the mailbox: short steps share one (a test is a branch,
   // about 10 cycles, and waiting for the last of four steps' items costs a
-  // hand-off three steps)
+  // hand-off three steps: 2x2 FP64, 200x100 cells, 133 us per sweep with four,
+  // 125 with one; 1x1 FP64, 128x128, 67 and 69)
   // values are loaded a step ahead where two sets of them fit the registers
   constexpr int VB = VC <= 8 ? 2 : 1;
   constexpr int HB = B == 3 ? 1 : 2;
-  constexpr int G = NE <= 4 && CH >= 4 ? 4 : 1;
+  constexpr int G = (SZ == 4 || B == 1) && NE <= 4 && CH >= 4 ? 4 : 1;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ int s_group, s_slot, s_stop;
   const int W = a.W, NS = a.NS;
@@ -431,6 +442,7 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
 #pragma unroll
                   for (int q = 0; q < B; ++q) acc[d] -= A(e * EV + d * B + q) * x[e].v[q];
               Vec<T, BP> y;
+              y.v[BP - 1] = 0;
 #pragma unroll
               for (int d = 0; d < B; ++d) {
                 if constexpr (FWD) {
@@ -511,8 +523,8 @@ __global__ void k_strip_meta(int CH, int MC, int step_bytes, int chunk_bytes, co
 // one block per step: value k of lane l in piece k / (16 / sizeof(T))
 template <typename T, int B, bool FWD>
 __global__ void k_strip_pack(StripPackArgs a) {
-  constexpr int SZ = (int)sizeof(T), PER16 = 16 / SZ, LPR = strip_lpr(B, SZ), BS = B * B;
-  constexpr int EV = B * (LPR == 1 ? B : 1);
+  constexpr int SZ = (int)sizeof(T), PER16 = 16 / SZ, BS = B * B;
+  const int LPR = a.d.LPR, EV = B * (LPR == 1 ? B : 1);
   const long long s = blockIdx.x;
   const int RW = a.d.RW, ne = a.ne;
   T* v = reinterpret_cast<T*>(a.rec + (size_t)(s / a.d.CH) * a.d.chunk_bytes + kStripHdr +

@@ -31,15 +31,19 @@ constexpr int kStripZero = 32;   // zero bytes at the start of a warp's value re
 constexpr int kStripMaxWarps = 4;
 
 // Lanes per row.  An FP64 step costs 64 cycles of its scheduler per
-// warp-wide FMA whatever the number of active lanes, and a 3x3 row 63 FMAs in
-// one lane: there each component of a row takes its own lane, which divides
-// the step's chain by b.  FP32 2x2 rows stay in one lane (16 FMAs): two lanes
-// per row would halve the rows of a strip and double the hand-offs between
-// strips.
-__host__ __device__ constexpr int strip_lpr(int b, int elem) { return b == 3 ? 3 : (b == 2 && elem == 8) ? 2 : 1; }
+// warp-wide FMA whatever the number of active lanes: there each component of a
+// row takes its own lane, which divides the step's chain by b.  FP32 rows stay in
+// one lane: more lanes per row would make steps shorter (3x3, 7 entries: 330
+// cycles a level against 620) but strips smaller and hand-offs between them more, and
+// those weigh more (elasticity on 56^3 cells 102 us per sweep with three lanes
+// per row, 81 with one; on 24^3 37 and 34).  3x3 rows of more than 7 entries do
+// not fit one lane's registers.
+__host__ __device__ constexpr int strip_lpr(int b, int elem, int ne) {
+  return elem == 8 || (b == 3 && ne > 7) ? b : 1;
+}
 __host__ __device__ constexpr StripDims strip_dims(int b, int elem, bool forward, int ne) {
   StripDims d{};
-  d.LPR = strip_lpr(b, elem);
+  d.LPR = strip_lpr(b, elem, ne);
   d.RW = 32 / d.LPR;
   d.MC = ((ne + 1) / 2 + 2 + 3) / 4;
   const int per_lane = (ne + (forward ? 1 : 0)) * b * (d.LPR == 1 ? b : 1);
