@@ -22,12 +22,12 @@
 //     arrive.  `delivered` counts the arrived prefix; a step says how many
 //     items it needs, one compare when they are there.
 // Measured on GB300, FP32, per sweep (forward / backward): the 1000x500
-// cantilever 0.14 / 0.13 ms (ranged kernel 1.09 / 1.10), Poisson on 301x257
+// cantilever 0.13 / 0.12 ms (ranged kernel 1.09 / 1.10), Poisson on 301x257
 // cells 47 / 46 us (one CTA per sweep 200 / 196), elasticity on 56^3 cells 81 /
-// 77 us (a launch per level 345 / 306).  FP64: the cantilever 0.60 / 0.48 ms
-// (2.36 / 2.08), Poisson on 128x128 cells 67 / 56 us (133 / 123).  Inside one
-// strip a level costs 110 (1x1 blocks) to 640 (3x3, 7 entries) cycles in FP32
-// and 400 to 2,000 in FP64, where each warp-wide FMA takes its scheduler 64; a
+// 77 us (a launch per level 345 / 306).  FP64: the cantilever 0.59 / 0.48 ms
+// (2.36 / 2.08), Poisson on 128x128 cells 65 / 55 us (133 / 123).  Inside one
+// strip a level costs 103 (1x1 blocks) to 490 (3x3, 7 entries) cycles in FP32
+// and 380 to 2,000 in FP64, where each warp-wide FMA takes its scheduler 64; a
 // hand-off between strips costs 1,500 to 3,000, of which the L2 takes 600-900.
 //
 // Strips are claimed in order, W per CTA, through a ticket, so a strip only
@@ -226,6 +226,13 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
   // values are loaded a step ahead where two sets of them fit the registers
   constexpr int VB = VC <= 8 ? 2 : 1;
   constexpr int HB = B == 3 ? 1 : 2;
+  // A step's stores to global memory are issued in the next step, while that
+  // step's dependency loads are under way, instead of between its result and
+  // them (one strip of 2000 lines, cycles per level: 1x1 FP32 113 -> 103, FP64 403
+  // -> 379; 2x2 FP32 147 -> 135, FP64 709 -> 699).  3x3 steps are long: there the
+  // exchange store goes at once, since waiting costs the next strip more (FP64
+  // 24^3 cells 100.4 us per sweep held back, 98.0 at once).
+  constexpr bool XNOW = B == 3;
   constexpr int G = (SZ == 4 || B == 1) && NE <= 4 && CH >= 4 ? 4 : 1;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ int s_group, s_slot, s_stop;
@@ -357,6 +364,12 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
         };
         T* const ring0 = reinterpret_cast<T*>(region + kStripZero) + lr * BP;
         bool abort = false;
+        Vec<T, LPR == 1 ? BP : 1> yl;  // the last step's result
+#pragma unroll
+        for (int d = 0; d < (LPR == 1 ? BP : 1); ++d) yl.v[d] = 0;
+        o[1] = xs[1] = -1;
+        op[1] = out;
+        xp[1] = xch;
         // waits until the progress word reaches `want`; its last value
         auto wait_for = [&](const int* word, int want, int site) -> int {
           int v;
@@ -416,6 +429,9 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
             for (int e = 0; e < NE; ++e) {
               x[e] = *reinterpret_cast<const Vec<T, BP>*>(reinterpret_cast<const float*>(smem) + cd[k][e]);
             }
+            // the last step's result leaves
+            if (!XNOW) xstore(xs[k ^ 1], xp[k ^ 1], yl);
+            ostore(o[k ^ 1], op[k ^ 1], yl);
             // the next step's data
             const bool more = j + 1 < CH || c + 1 < nch;
             if (j + 1 < CH) {
@@ -455,9 +471,9 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
                 }
               }
               *reinterpret_cast<Vec<T, BP>*>(rg + j * RW * BP) = y;
+              yl = y;
+              if (XNOW) xstore(xs[k], xp[k], yl);
               if (SZ == 4 && more) decode((j + 1) % K2);
-              xstore(xs[k], xp[k], y);
-              ostore(o[k], op[k], y);
             } else {
               T acc = t[k][0];
 #pragma unroll
@@ -475,10 +491,9 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
                 acc = y;
               }
               if (lr < RW) rg[j * RW * BP + p] = acc;
-              const Vec<T, 1> y1{{acc}};
+              yl.v[0] = acc;
+              if (XNOW) xstore(xs[k], xp[k], yl);
               if (SZ == 4 && more) decode((j + 1) % K2);
-              xstore(xs[k], xp[k], y1);
-              ostore(o[k], op[k], y1);
             }
             __syncwarp();
           }
@@ -488,7 +503,12 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
           vp = vp1;
           rg = (c + 1) * CH % kStripRing == 0 ? ring0 : rg + CH * RW * BP;
         }
-        if (abort && lane == 0) record_fail(a.err, kErrTimeout, kSiteRange, -1, r);
+        if (abort) {
+          if (lane == 0) record_fail(a.err, kErrTimeout, kSiteRange, -1, r);
+        } else {
+          if (!XNOW) xstore(xs[1], xp[1], yl);
+          ostore(o[1], op[1], yl);
+        }
       }
     }
     __syncthreads();

@@ -34,7 +34,7 @@ constexpr int kStripMaxWarps = 4;
 // warp-wide FMA whatever the number of active lanes: there each component of a
 // row takes its own lane, which divides the step's chain by b.  FP32 rows stay in
 // one lane: more lanes per row would make steps shorter (3x3, 7 entries: 330
-// cycles a level against 620) but strips smaller and hand-offs between them more, and
+// cycles a level against 490) but strips smaller and hand-offs between them more, and
 // those weigh more (elasticity on 56^3 cells 102 us per sweep with three lanes
 // per row, 81 with one; on 24^3 37 and 34).  3x3 rows of more than 7 entries do
 // not fit one lane's registers.
