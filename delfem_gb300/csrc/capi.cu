@@ -1176,7 +1176,8 @@ PrecondLaunch precond_launch(dfg_ctx ctx_, dfg_precond pr, bool fp32, const void
     StripDev &f = pr->strip[0][fp32 ? 1 : 0], &b = pr->strip[1][fp32 ? 1 : 0];
     L.F = strip_launch(ctx_, pr, 0, fp32, b.in.p, tickets, done);
     L.B = strip_launch(ctx_, pr, 1, fp32, z, tickets + 1, done);
-    L.feed = SweepFeed{f.in.p, f.pos.as<int>(), {f.xch.p, b.xch.p}, {f.nxch, b.nxch}};
+    L.B.ta.other_ticket = tickets;
+    L.feed = SweepFeed{f.in.p, f.pos.as<int>(), {f.xch.p, b.xch.p}, {f.nxch, b.nxch}, true};
     return L;
   }
   void* y = fp32 ? pr->ybuf32.p : pr->ybuf64.p;
@@ -1210,8 +1211,8 @@ long long launches_of(const SweepLaunch& L) {
   return L.solo ? 2 : L.levels ? (long long)L.lev->ptr.size() - 1 : 1;
 }
 
-void run_sweep(dfg_ctx ctx_, const SweepLaunch& L) {
-  CK(enqueue_sweep(L, ctx_->stream));
+void run_sweep(dfg_ctx ctx_, const SweepLaunch& L, bool dep = false) {
+  CK(enqueue_sweep(L, ctx_->stream, dep));
   launched(ctx_, launches_of(L));
 }
 
@@ -1777,7 +1778,7 @@ extern "C" int dfg_precond_solve(dfg_precond prec, dfg_system sys, int iv) {
       run_sweep(ctx, L.F);
       CK(fill_sentinel(m, v, false, ctx->stream));
     }
-    run_sweep(ctx, L.B);
+    run_sweep(ctx, L.B, prec->strips);
     launched(ctx, 2);  // the two sentinel fills
     if (read_err(ctx) != 0) {
       CK(cudaMemsetAsync(ctx->err_word.p, 0, sizeof(int), ctx->stream));
@@ -1903,7 +1904,7 @@ static int solve_pcg_f64vec(dfg_system sys, dfg_precond prec, bool fp32z, bool t
     // prologue (solver_ls_iter.cpp:106-128)
     CK(pcg_init(v, st, red, tol, maxit, sc.tickets, fp32z, ctx->stream));
     run_sweep(ctx, F);
-    run_sweep(ctx, B);
+    run_sweep(ctx, B, true);
     CK(pcg_after_precond0(v, st, red, fp32z, ctx->stream));
     ensure_sell(ctx, sys, false);
     const MatView A = view64(sys);
@@ -2047,7 +2048,7 @@ extern "C" int dfg_solve_pcg_mixed(dfg_system sys, dfg_precond prec, double* con
     CK(mix_true_residual(A64, v, st, red, ctx->stream));
     CK(mix_replace(v, st, sc.tickets, ctx->stream));
     run_sweep(ctx, F);
-    run_sweep(ctx, B);
+    run_sweep(ctx, B, true);
     CK(mix_after_precond0(v, st, red, ctx->stream));
     const IterRed ired = iter_red_of(ctx);
     CK(mix_iter(A32, v, st, ired, sc.tickets, true, ctx->nsm, ctx->stream));
@@ -2152,12 +2153,12 @@ extern "C" int dfg_solve_pbicgstab(dfg_system sys, dfg_precond prec, int mode, d
       for (int c = 0; c < chunk; ++c) {
         if (feed_launches) enqueue_strip_feed(P1, v.p, m, ctx->stream);
         enqueue_sweep(F1, ctx->stream);
-        enqueue_sweep(B1, ctx->stream);
+        enqueue_sweep(B1, ctx->stream, true);
         bicg_amp(A, v, st, red, ctx->stream);
         bicg_s(v, st, sc.tickets, ctx->stream);
         if (feed_launches) enqueue_strip_feed(P2, v.s, m, ctx->stream);
         enqueue_sweep(F2, ctx->stream);
-        enqueue_sweep(B2, ctx->stream);
+        enqueue_sweep(B2, ctx->stream, true);
         bicg_ams(A, v, st, red2, ctx->stream);
         bicg_update(v, st, red2, ctx->stream);
         bicg_p(v, st, sc.tickets, ctx->stream);

@@ -252,6 +252,10 @@ __global__ void __launch_bounds__(TPB, 1) k_pcg_iter(MatView A, PcgVecs v, PcgSt
                                                   int first) {
   __shared__ double ws[32];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (!v.feed.early) tickets[0] = 0;
+    tickets[1] = 0;
+  }
   if (st->done) return;
   GridWalk g{red.bar, red.err};
   double *part_rz = red.part, *part_pq = red.part + kRedGrid, *part_rr = red.part + 2 * kRedGrid;
@@ -313,8 +317,6 @@ __global__ void __launch_bounds__(TPB, 1) k_pcg_iter(MatView A, PcgVecs v, PcgSt
       st->conv = ratio;
       st->iter_out = st->it;
     }
-    tickets[0] = 0;
-    tickets[1] = 0;
   }
 }
 
@@ -324,6 +326,10 @@ __global__ void __launch_bounds__(TPB, 1) k_mix_iter(MatView A, MixVecs v, PcgSt
                                                   int first) {
   __shared__ double ws[32];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (!v.feed.early) tickets[0] = 0;
+    tickets[1] = 0;
+  }
   if (st->done) return;
   GridWalk g{red.bar, red.err};
   double *part_rz = red.part, *part_pq = red.part + kRedGrid, *part_rr = red.part + 2 * kRedGrid;
@@ -378,8 +384,6 @@ __global__ void __launch_bounds__(TPB, 1) k_mix_iter(MatView A, MixVecs v, PcgSt
       st->done = 2;
     }
     st->iter_out = st->it + 1;
-    tickets[0] = 0;
-    tickets[1] = 0;
   }
 }
 

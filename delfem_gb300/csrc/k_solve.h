@@ -60,6 +60,9 @@ struct SweepFeed {
   const int* pos;
   void* fill[2];
   long long nfill[2];
+  // the forward sweep may claim work while the kernel before it still runs:
+  // its ticket is the backward sweep's to reset, not that kernel's
+  bool early = false;
 };
 
 // ---- FP64 PCG (plain path) -------------------------------------------------

@@ -219,10 +219,6 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
   constexpr int PER16 = 16 / SZ;
   constexpr int EV = B * (LPR == 1 ? B : 1);  // values per entry and lane
   constexpr int RHS_CHUNK = CH * D.rhs_bytes;
-  // steps per test of the mailbox: short steps share one (a test is a branch,
-  // about 10 cycles, and waiting for the last of four steps' items costs a
-  // hand-off three steps: 2x2 FP64, 200x100 cells, 133 us per sweep with four,
-  // 125 with one; 1x1 FP64, 128x128, 67 and 69)
   // values are loaded a step ahead where two sets of them fit the registers
   constexpr int VB = VC <= 8 ? 2 : 1;
   constexpr int HB = B == 3 ? 1 : 2;
@@ -233,7 +229,7 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
   // exchange store goes at once, since waiting costs the next strip more (FP64
   // 24^3 cells 100.4 us per sweep held back, 98.0 at once).
   constexpr bool XNOW = B == 3;
-  constexpr int G = (SZ == 4 || B == 1) && NE <= 4 && CH >= 4 ? 4 : 1;
+  constexpr int G = D.G;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ int s_group, s_slot, s_stop;
   const int W = a.W, NS = a.NS;
@@ -251,8 +247,13 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
     for (int s = 0; s < W * NS; ++s) mbar_init(reinterpret_cast<uint64_t*>(smem) + s, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  pdl_enter();
-  if (a.one.done && *a.one.done) return;
+  // One solve's sweep claims its first strips and asks for their first records
+  // before it waits for the kernel ahead of it: the factor does not change
+  // within a solve, and the ticket is reset by another kernel than that one
+  // (a PCG iteration, Poisson on 24x24 cells 50 -> 47 us, on 128x128 134 -> 131, on
+  // 301x257, FP32 everything, 111 -> 109).
+  bool fresh = a.batch == nullptr;
+  if (!fresh) pdl_enter();
   int st = 0, ph = 0;  // stage and phase of the strip's next chunk (compute warps and loader alike)
   for (;;) {
     int issued = 0;  // loader: chunks of the strip issued
@@ -284,6 +285,26 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
     __syncthreads();
     const int group = s_group;
     const StripSlot S = a.batch ? a.batch->slot[s_slot] : a.one;
+    if (fresh) {
+      fresh = false;
+      const int r0 = group * W + w;
+      const bool mine = load_warp && lane < W && group >= 0 && r0 < S.nstrips;
+      const int c0 = mine ? S.strip_chunk[r0] : 0, first = mine ? min(S.strip_chunk[r0 + 1] - c0, NS) : 0;
+      for (; issued < first; ++issued) {
+        mbar_expect_tx(&full[issued], D.chunk_bytes + RHS_CHUNK);
+        tma_load_1d(rstage + (size_t)issued * D.chunk_bytes, S.rec + (size_t)(c0 + issued) * D.chunk_bytes,
+                    D.chunk_bytes, &full[issued]);
+      }
+      pdl_enter();
+      for (int k = 0; k < first; ++k)
+        tma_load_1d(vstage + (size_t)k * RHS_CHUNK,
+                    reinterpret_cast<const unsigned char*>(S.in) + (size_t)(c0 + k) * RHS_CHUNK, RHS_CHUNK, &full[k]);
+      if (a.other_ticket && blockIdx.x == 0 && threadIdx.x == 0) *a.other_ticket = 0;
+      if (S.done && *S.done) {
+        for (int k = 0; k < first; ++k) mbar_drain(&full[k], 0);
+        return;
+      }
+    }
     if (group == -1) break;
     if (group == -2) {  // a finished solve
       __syncthreads();
@@ -296,8 +317,8 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
       // right-hand sides, NS chunks ahead of the chunks the warp has finished
       const bool on = lane < W && r < S.nstrips;
       const int c0 = on ? S.strip_chunk[r] : 0, nch = on ? S.strip_chunk[r + 1] - c0 : 0;
-      const unsigned char* rec = S.rec + (size_t)c0 * D.chunk_bytes;
-      const unsigned char* in = reinterpret_cast<const unsigned char*>(S.in) + (size_t)c0 * RHS_CHUNK;
+      const unsigned char* rec = S.rec + (size_t)(c0 + issued) * D.chunk_bytes;
+      const unsigned char* in = reinterpret_cast<const unsigned char*>(S.in) + (size_t)(c0 + issued) * RHS_CHUNK;
       bool failing = false;
       for (unsigned n = 1; __any_sync(0xffffffffu, issued < nch && !failing); ++n) {
         if (issued < nch && !failing) {
@@ -412,6 +433,9 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
 #pragma unroll
           for (int j = 0; j < CH; ++j) {
             if (j % G == 0 && need[j + G - 1] > have) {
+              // only padding is left of the strip (the last step's stores are in set 1)
+              static_assert(!D.ends || G % 2 == 0, "the end is seen in an even step");
+              if (D.ends && need[j + G - 1] == kStripEnd) break;
               have = wait_for(delivered, need[j + G - 1], kSitePoll);
               if (abort) break;
             }

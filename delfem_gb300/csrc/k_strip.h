@@ -22,6 +22,8 @@ struct StripDims {
   int MC;      // 16-byte pieces of metadata per lane and step
   int VC;      // 16-byte pieces of factor values per lane and step
   int CH;      // steps per chunk (the unit copied into shared memory)
+  int G;       // steps per test of the mailbox
+  bool ends;   // the test also sees the strip's end (else the padding of its last chunk is swept)
   int VS;      // bytes of one row's value in the ring, the mailbox and the exchange buffer
   int step_bytes, rhs_bytes, chunk_bytes;
 };
@@ -29,6 +31,7 @@ constexpr int kStripHdr = 32;    // bytes before a chunk's steps: CH counts of m
 constexpr int kStripRing = 32;   // ring depth in steps
 constexpr int kStripZero = 32;   // zero bytes at the start of a warp's value region (padding entries)
 constexpr int kStripMaxWarps = 4;
+constexpr int kStripEnd = 0x7fffffff;  // item count of steps after a strip's last: the strip is done
 
 // Lanes per row.  An FP64 step costs 64 cycles of its scheduler per
 // warp-wide FMA whatever the number of active lanes: there each component of a
@@ -52,6 +55,14 @@ __host__ __device__ constexpr StripDims strip_dims(int b, int elem, bool forward
   d.step_bytes = 512 * (d.MC + d.VC);
   d.rhs_bytes = d.RW * b * elem;
   d.CH = d.step_bytes <= 2560 ? 8 : d.step_bytes <= 6144 ? 4 : 2;
+  // short steps share a test (it is a branch, about 10 cycles, and waiting for
+  // the last of four steps' items costs a hand-off three steps: 2x2 FP64, 200x100
+  // cells, 133 us per sweep with four, 125 with one; 1x1 FP64, 128x128, 67 and 69)
+  d.G = (elem == 4 || b == 1) && ne <= 4 && d.CH >= 4 ? 4 : 1;
+  // the padding is up to 7 steps of 380 cycles in 1x1 FP64 (Poisson on 128x128 cells
+  // 134 us per PCG iteration with it, 131 without); the other kinds' steps are
+  // shorter, or fewer to a chunk, and the test costs them 1 to 3 % in every step
+  d.ends = elem == 8 && d.G > 1;
   d.chunk_bytes = kStripHdr + d.CH * d.step_bytes;
   return d;
 }
@@ -72,7 +83,7 @@ struct StripPlan {
   std::vector<int> item_ptr;     // nstrips + 1
   std::vector<int> items;        // per item {exchange slot, step at which its mailbox slot is free}
   std::vector<int> pos;          // n
-  std::vector<int> need;         // nchunks * CH: mailbox items a step needs delivered
+  std::vector<int> need;         // nchunks * CH: mailbox items a step needs delivered, or kStripEnd
   std::vector<int> step_rows;    // nchunks * CH * RW, -1 = empty
   std::vector<int> ent_slot;     // nchunks * CH * RW * ne: CRS slot of the block, -1 = padding
   std::vector<int> codes;        // same shape: byte offset into the warp's value region
@@ -132,7 +143,12 @@ struct StripBatch {
 struct StripArgs {
   StripSlot one;
   const StripBatch* batch;  // non-null: batched launch (`one` unused)
-  int* ticket;   // 0 at launch
+  // 0 when the launch can begin.  A launch that may begin before the kernel
+  // ahead of it has ended (programmatic dependence) has it reset by an earlier
+  // kernel: the backward sweep resets the forward one's (other_ticket), the
+  // kernel after the backward sweep the backward one's.
+  int* ticket;
+  int* other_ticket;  // optional: set to 0
   int* err;      // device error word
   int ne;        // entry class
   int W;         // strips (compute warps) per CTA

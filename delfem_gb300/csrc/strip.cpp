@@ -225,6 +225,9 @@ bool strip_plan(int n, int b, int elem, const int* rowptr, const int* colind, co
       }
     }
     P.item_ptr.push_back((int)(P.items.size() / 2));
+    // (steps of a test's group that has rows keep their counts)
+    for (int q = s0 + (P.strip_steps[r] + P.d.G - 1) / P.d.G * P.d.G; P.d.ends && q < P.strip_chunk[r + 1] * CH; ++q)
+      P.need[q] = kStripEnd;
   }
   for (int row = 0; row < n; ++row)
     if (xslot[row] >= 0) P.exports[P.pos[row]] = xslot[row];

@@ -68,6 +68,8 @@ extern "C" int emul_strip(int n, int b, int elem, const int* rowptr, const int* 
       for (int l = 0; l < d.RW; ++l) region[(kStripZero + ((s % kStripRing) * d.RW + l) * d.VS) / 4] = done_rows[l];
       if ((s + 1) % d.CH == 0) consumed = s + 1;
     }
+    for (int q = s0; q < P.strip_chunk[r + 1] * d.CH; ++q)  // the end mark: after the last group of steps with rows
+      if ((P.need[q] == kStripEnd) != (d.ends && (q - s0) / d.G * d.G >= P.strip_steps[r])) return 9;
   }
   for (int i = 0; i < n; ++i)
     if (seen[i] != 1) return 8;
