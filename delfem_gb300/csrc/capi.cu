@@ -204,17 +204,42 @@ void check_pattern(dfg_ctx ctx_, int n, const int* rowptr, const int* colind) {
   }
 }
 
+// The context's pinned host area: what the host reads from the device goes
+// through it (a copy to pageable memory goes through a staging buffer of the
+// driver's, about 6 us more per read).
+struct HostArea {
+  PcgState replay[2];  // states after the graph replays in flight
+  PcgState state;
+  BicgState bicg;
+  int words[16];
+  double sum;          // written by a reduction kernel
+};
+static_assert(sizeof(HostArea) <= kPinnedBytes, "HostArea fits the pinned area");
+HostArea& host_area(dfg_ctx c) { return *static_cast<HostArea*>(c->h_pinned); }
+
 int read_state(dfg_ctx ctx_, PcgState* d_state, PcgState& h) {
-  CK(cudaMemcpyAsync(&h, d_state, sizeof(PcgState), cudaMemcpyDeviceToHost, ctx_->stream));
+  HostArea& H = host_area(ctx_);
+  CK(cudaMemcpyAsync(&H.state, d_state, sizeof(PcgState), cudaMemcpyDeviceToHost, ctx_->stream));
   CK(cudaStreamSynchronize(ctx_->stream));
+  h = H.state;
   return 0;
 }
 
 int read_err(dfg_ctx ctx_) {
-  int e = 0;
-  CK(cudaMemcpyAsync(&e, ctx_->err_word.p, sizeof(int), cudaMemcpyDeviceToHost, ctx_->stream));
+  HostArea& H = host_area(ctx_);
+  CK(cudaMemcpyAsync(H.words, ctx_->err_word.p, sizeof(int), cudaMemcpyDeviceToHost, ctx_->stream));
   CK(cudaStreamSynchronize(ctx_->stream));
-  return e;
+  return H.words[0];
+}
+
+// x.y on the host (the reduction kernel writes it there)
+double read_dot(dfg_ctx ctx_, long long m, const double* x, const double* y) {
+  Red r = red_of(ctx_, 0);
+  r.result = &host_area(ctx_).sum;
+  CK(api_dot(m, x, y, r, ctx_->stream));
+  launched(ctx_);
+  CK(cudaStreamSynchronize(ctx_->stream));
+  return host_area(ctx_).sum;
 }
 
 }  // namespace
@@ -261,11 +286,16 @@ extern "C" int dfg_ctx_create(int device, dfg_ctx* out) {
     dalloc(c, c->iter_red, 3 * kRedGrid * 8 + 64);
     CK(cudaMemsetAsync(c->iter_red.p, 0, c->iter_red.bytes, c->stream));
     CK(sweep_set_smem_limits(c->smem_optin));
+    CK(cudaHostAlloc(&c->h_pinned, kPinnedBytes, cudaHostAllocDefault));
+    for (cudaEvent_t& e : c->replay_done) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     CK(cudaStreamSynchronize(c->stream));
     return DFG_OK;
   });
   if (rc != DFG_OK) {
     g_create_error = c->last_error;
+    for (cudaEvent_t e : c->replay_done)
+      if (e) cudaEventDestroy(e);
+    if (c->h_pinned) cudaFreeHost(c->h_pinned);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
     return rc;
@@ -281,6 +311,8 @@ extern "C" int dfg_ctx_destroy(dfg_ctx ctx) {
   ctx->err_word.release();
   ctx->scratch.release();
   ctx->iter_red.release();
+  for (cudaEvent_t e : ctx->replay_done) cudaEventDestroy(e);
+  cudaFreeHost(ctx->h_pinned);
   cudaStreamDestroy(ctx->stream);
   delete ctx;
   return DFG_OK;
@@ -748,12 +780,7 @@ extern "C" int dfg_finalize_marge(dfg_system sys, double* norm_res) {
     sys->rhs0_valid = true;
     sys->mat32_valid = false;
     ++sys->mat_version;
-    Red r = red_of(ctx, 0);
-    CK(api_dot((long long)m, sys->res.as<double>(), sys->res.as<double>(), r, ctx->stream));
-    launched(ctx);
-    double s = 0.0;
-    CK(cudaMemcpyAsync(&s, r.result, 8, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
+    const double s = read_dot(ctx, (long long)m, sys->res.as<double>(), sys->res.as<double>());
     if (norm_res) *norm_res = std::sqrt(s);
     return DFG_OK;
   });
@@ -841,11 +868,7 @@ extern "C" int dfg_dot(dfg_system sys, int iv1, int iv2, double* out) {
     dfg_ctx ctx_ = ctx;
     const double* a = vec_ptr(ctx, sys, iv1);
     const double* b = vec_ptr(ctx, sys, iv2);
-    Red r = red_of(ctx, 0);
-    CK(api_dot((long long)sys->n * sys->b, a, b, r, ctx->stream));
-    launched(ctx);
-    CK(cudaMemcpyAsync(out, r.result, 8, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
+    *out = read_dot(ctx, (long long)sys->n * sys->b, a, b);
     return DFG_OK;
   });
 }
@@ -1712,8 +1735,9 @@ extern "C" int dfg_precond_set_value(dfg_precond prec, dfg_system sys) {
                             ctx->stream, l > 0));
       launched(ctx, nl);
     }
-    int h_sync[kIluSync] = {};
-    CK(cudaMemcpyAsync(h_sync, sync, sizeof(h_sync), cudaMemcpyDeviceToHost, ctx->stream));
+    const int* h_sync = host_area(ctx).words;
+    static_assert(kIluSync <= 16, "kIluSync words of HostArea");
+    CK(cudaMemcpyAsync(host_area(ctx).words, sync, kIluSync * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     if (prec->strips) {
       pack_strips(ctx, prec, false);
     } else {
@@ -1829,6 +1853,50 @@ struct Chunk {
   }
 };
 
+// Replays of a solve's graph of `chunk` iterations.  The host looks at the
+// state after each; while the residual's last drop says that the replay under
+// way will not end the solve, the one after it is sent before that look, so that
+// the device does not wait for the host in between (some 20 us a replay:
+// Poisson on 24x24 cells, 4 replays of 318 us).  A replay sent too many does
+// nothing: every kernel sees the stop flag.
+struct Replays {
+  dfg_ctx ctx_;
+  cudaGraphExec_t exec;
+  PcgState* st;
+  long long launches;  // per replay
+  unsigned sent = 0, seen = 0;
+  bool ahead = false;
+  bool spare = false;  // a replay too many was sent
+  double last = -1.0;  // residual at the look before
+
+  void send() {
+    CK(cudaGraphLaunch(exec, ctx_->stream));
+    launched(ctx_, launches);
+    CK(cudaMemcpyAsync(&host_area(ctx_).replay[sent & 1], st, sizeof(PcgState), cudaMemcpyDeviceToHost, ctx_->stream));
+    CK(cudaEventRecord(ctx_->replay_done[sent & 1], ctx_->stream));
+    ++sent;
+  }
+  // The state after the next replay.  Residuals below stop(h) end the replays.
+  template <typename F>
+  void next(PcgState& h, F&& stop) {
+    while (sent - seen < (ahead ? 2u : 1u)) send();
+    CK(cudaEventSynchronize(ctx_->replay_done[seen & 1]));
+    h = host_area(ctx_).replay[seen & 1];
+    ++seen;
+    if (h.done != 0 && seen != sent) {  // its state is not looked at
+      spare = true;
+      seen = sent;
+    }
+    const double drop = last > 0.0 ? h.rr / last : 0.0;
+    // half as much again as the last drop stays above the stop
+    ahead = h.done == 0 && drop > 0.0 && h.rr * std::min(drop, 1.0) * std::sqrt(std::min(drop, 1.0)) > stop(h);
+    last = h.rr;
+  }
+  ~Replays() {  // the graph goes away
+    if (spare || sent != seen) cudaEventSynchronize(ctx_->replay_done[(sent - 1) & 1]);
+  }
+};
+
 // Reads and clears the error word (code, wait site, slot, range or row) and
 // reports the timeout; the context stays usable.
 int timeout_status(dfg_ctx ctx_) {
@@ -1911,8 +1979,6 @@ static int solve_pcg_f64vec(dfg_system sys, dfg_precond prec, bool fp32z, bool t
     const IterRed ired = iter_red_of(ctx);
     CK(pcg_iter(A, v, st, ired, sc.tickets, fp32z, true, ctx->nsm, ctx->stream));
     launched(ctx, 3);
-    PcgState h{};
-    read_state(ctx, st, h);
     // iterations from the preconditioner on: a graph of `chunk` of them,
     // replayed until done
     const long long per_it = 1 + launches_of(F) + launches_of(B);
@@ -1929,24 +1995,20 @@ static int solve_pcg_f64vec(dfg_system sys, dfg_precond prec, bool fp32z, bool t
     }
     CK(cudaStreamEndCapture(ctx->stream, &g.graph));
     CK(cudaGraphInstantiate(&g.exec, g.graph, 0));
+    Replays replays{ctx, g.exec, st, per_it * chunk};
+    PcgState h{};
     unsigned refin = 0;
     long long guard = 0;
     double bb = 0.0;
     for (;;) {
       while (!h.done) {
-        CK(cudaGraphLaunch(g.exec, ctx->stream));
-        launched(ctx, per_it * chunk);
-        read_state(ctx, st, h);
-        if (read_err(ctx) != 0) return timeout_status(ctx);
+        replays.next(h, [](const PcgState& s) { return s.tol2 / s.inv_rr0; });
         if (++guard > (long long)maxit / chunk + 64) break;
       }
+      if (h.done == kDoneError || (h.done == 0 && read_err(ctx) != 0)) return timeout_status(ctx);
       if (h.done != 1 || !target_true) break;
       // recursive residual converged: check the true one
-      if (bb == 0.0) {
-        CK(api_dot(m, v.b, v.b, red_of(ctx, 0), ctx->stream));
-        launched(ctx);
-        CK(cudaMemcpyAsync(&bb, red_of(ctx, 0).result, 8, cudaMemcpyDeviceToHost, ctx->stream));
-      }
+      if (bb == 0.0) bb = read_dot(ctx, m, v.b, v.b);
       CK(pcg_true_residual(A, v, st, red, ctx->stream));
       launched(ctx);
       ++refin;
@@ -2030,11 +2092,7 @@ extern "C" int dfg_solve_pcg_mixed(dfg_system sys, dfg_precond prec, double* con
     v.feed = PL.feed;
     CK(cudaMemsetAsync(v.x, 0, (size_t)m * 8, ctx->stream));
     CK(cudaMemsetAsync(v.d, 0, (size_t)m * 8, ctx->stream));
-    CK(api_dot(m, v.b, v.b, red, ctx->stream));
-    launched(ctx);
-    double bb = 0.0;
-    CK(cudaMemcpyAsync(&bb, red.result, 8, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
+    const double bb = read_dot(ctx, m, v.b, v.b);
     const double tol = *conv_ratio;
     const int maxit = (int)std::min<unsigned>(*iteration, 0x7fffffffu);
     if (bb < 1.0e-30) {
@@ -2069,11 +2127,10 @@ extern "C" int dfg_solve_pcg_mixed(dfg_system sys, dfg_precond prec, double* con
     double rel = 1.0;
     int status = DFG_NOT_CONVERGED;
     long long guard = 0;
+    Replays replays{ctx, g.exec, st, per_it * chunk};
     for (;;) {
-      CK(cudaGraphLaunch(g.exec, ctx->stream));
-      launched(ctx, per_it * chunk);
-      read_state(ctx, st, h);
-      if (read_err(ctx) != 0) return timeout_status(ctx);
+      replays.next(h, [](const PcgState& s) { return std::max(s.tolb2, s.delta2 * s.rr_ref); });
+      if (h.done == kDoneError) return timeout_status(ctx);
       if (h.done == 0) {
         if (++guard > (long long)maxit / chunk + 64) break;
         continue;
@@ -2140,8 +2197,10 @@ extern "C" int dfg_solve_pbicgstab(dfg_system sys, dfg_precond prec, int mode, d
     CK(bicg_init(v, st, red, tol, maxit, sc.tickets, ctx->stream));
     launched(ctx, 2);
     BicgState h{};
-    CK(cudaMemcpyAsync(&h, st, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
+    HostArea& H = host_area(ctx);
+    CK(cudaMemcpyAsync(&H.bicg, st, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
+    h = H.bicg;
     if (h.done == 0) {
       ensure_sell(ctx, sys, false);
       const MatView A = view64(sys);
@@ -2169,9 +2228,9 @@ extern "C" int dfg_solve_pbicgstab(dfg_system sys, dfg_precond prec, int mode, d
       while (!h.done) {
         CK(cudaGraphLaunch(g.exec, ctx->stream));
         launched(ctx, per_it * chunk);
-        CK(cudaMemcpyAsync(&h, st, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaStreamSynchronize(ctx->stream));
+        CK(cudaMemcpyAsync(&H.bicg, st, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
         if (read_err(ctx) != 0) return timeout_status(ctx);
+        h = H.bicg;
         if (++guard > (long long)maxit / chunk + 64) break;
       }
     }
@@ -2224,15 +2283,8 @@ extern "C" int dfg_true_residual(dfg_system sys, const double* b, double* rel) {
     dalloc(ctx, rr, (size_t)m * 8 + 64);
     CK(cudaMemcpyAsync(rr.p, bp, (size_t)m * 8, cudaMemcpyDeviceToDevice, ctx->stream));
     CK(api_matvec(view64(sys), -1.0, sys->upd.as<double>(), 1.0, rr.as<double>(), ctx->stream));
-    Red red = red_of(ctx, 0);
-    CK(api_dot(m, rr.as<double>(), rr.as<double>(), red, ctx->stream));
-    double r2 = 0.0, b2 = 0.0;
-    CK(cudaMemcpyAsync(&r2, red.result, 8, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    CK(api_dot(m, bp, bp, red, ctx->stream));
-    CK(cudaMemcpyAsync(&b2, red.result, 8, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    launched(ctx, 3);
+    const double r2 = read_dot(ctx, m, rr.as<double>(), rr.as<double>()), b2 = read_dot(ctx, m, bp, bp);
+    launched(ctx);
     *rel = b2 > 0 ? std::sqrt(r2 / b2) : std::sqrt(r2);
     return DFG_OK;
   });

@@ -229,6 +229,8 @@ struct StripDev {
 
 }  // namespace dfg
 
+constexpr size_t kPinnedBytes = 1024;
+
 struct dfg_ctx_s {
   int device = 0;
   int nsm = 0;
@@ -239,7 +241,8 @@ struct dfg_ctx_s {
   dfg::DBuf err_word;     // int, device error word (dfg::kErr*)
   dfg::DBuf scratch;      // reduction partials + scalars
   dfg::DBuf iter_red;     // k_iter.cu: partials, grid barrier
-  int* h_pinned = nullptr;  // small pinned host area for status reads
+  void* h_pinned = nullptr;           // kPinnedBytes of pinned host memory for status reads and sums
+  cudaEvent_t replay_done[2] = {};    // graph replays in flight (Replays in capi.cu)
   int last_timeout_site = 0;  // wait site of the last reported timeout
 };
 

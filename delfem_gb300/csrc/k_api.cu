@@ -125,7 +125,9 @@ cudaError_t api_scal(long long m, double alpha, double* x, cudaStream_t s) {
   return cudaGetLastError();
 }
 cudaError_t api_dot(long long m, const double* x, const double* y, Red red, cudaStream_t s) {
-  k_api_dot<<<kRedGrid, kRedTpb, 0, s>>>(m, x, y, red);
+  // (a block without elements would add a zero)
+  const long long need = (m + kRedTpb - 1) / kRedTpb;
+  k_api_dot<<<(int)(need < 1 ? 1 : need < kRedGrid ? need : kRedGrid), kRedTpb, 0, s>>>(m, x, y, red);
   return cudaGetLastError();
 }
 

@@ -256,7 +256,12 @@ __global__ void __launch_bounds__(TPB, 1) k_pcg_iter(MatView A, PcgVecs v, PcgSt
     if (!v.feed.early) tickets[0] = 0;
     tickets[1] = 0;
   }
+  const int failed = ld_relaxed_int(red.err);
   if (st->done) return;
+  if (failed) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) st->done = kDoneError;
+    return;
+  }
   GridWalk g{red.bar, red.err};
   double *part_rz = red.part, *part_pq = red.part + kRedGrid, *part_rr = red.part + 2 * kRedGrid;
   const int nvb = virtual_blocks(v.m, kRedTpb), nvr = virtual_blocks(A.n, kSpmvTpb);
@@ -330,7 +335,12 @@ __global__ void __launch_bounds__(TPB, 1) k_mix_iter(MatView A, MixVecs v, PcgSt
     if (!v.feed.early) tickets[0] = 0;
     tickets[1] = 0;
   }
+  const int failed = ld_relaxed_int(red.err);
   if (st->done) return;
+  if (failed) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) st->done = kDoneError;
+    return;
+  }
   GridWalk g{red.bar, red.err};
   double *part_rz = red.part, *part_pq = red.part + kRedGrid, *part_rr = red.part + 2 * kRedGrid;
   const int nvb = virtual_blocks(v.m, kRedTpb), nvr = virtual_blocks(A.n, kSpmvTpb);

@@ -19,7 +19,9 @@ struct PcgState {
   int pad;
 };
 // done codes: 0 running, 1 converged, 2 iteration limit, 3 NaN,
-//             4 reliable update due (mixed), 5 recursive residual below tol (mixed)
+//             4 reliable update due (mixed), 5 recursive residual below tol (mixed),
+//             kDoneError a wait of a kernel of the solve has given up
+constexpr int kDoneError = 6;
 
 // deterministic reductions: fixed grid, per-block partials, the last block
 // to finish sums the partials in index order
