@@ -1239,14 +1239,6 @@ void run_sweep(dfg_ctx ctx_, const SweepLaunch& L, bool dep = false) {
   launched(ctx_, launches_of(L));
 }
 
-// Strips whose input no kernel feeds: r (row order, FP64) into step order and
-// the exchange buffers to the sentinel.
-cudaError_t enqueue_strip_feed(const PrecondLaunch& L, const double* r, long long m, cudaStream_t st) {
-  cudaError_t e = launch_solo_permute(false, m, 1, L.feed.pos, r, L.feed.in, st);
-  for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = fill_sentinel(L.feed.nfill[i], L.feed.fill[i], false, st);
-  return e;
-}
-
 struct GraphHolder {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -1791,19 +1783,19 @@ extern "C" int dfg_precond_solve(dfg_precond prec, dfg_system sys, int iv) {
     double* v = vec_ptr(ctx, sys, iv);
     const long long m = (long long)sys->n * sys->b;
     Scratch sc = scratch_of(ctx);
-    CK(cudaMemsetAsync(sc.tickets, 0, 2 * sizeof(int), ctx->stream));
     PrecondLaunch L = precond_launch(ctx, prec, false, v, nullptr, v, sc.tickets, nullptr);
     if (prec->strips) {
-      CK(enqueue_strip_feed(L, v, m, ctx->stream));
+      CK(sweep_feed(L.feed, m, v, sc.tickets, ctx->stream));
       launched(ctx, 1);
       run_sweep(ctx, L.F);
     } else {
+      CK(cudaMemsetAsync(sc.tickets, 0, 2 * sizeof(int), ctx->stream));
+      launched(ctx, 2);  // the two sentinel fills
       CK(fill_sentinel(m, prec->ybuf64.p, false, ctx->stream));
       run_sweep(ctx, L.F);
       CK(fill_sentinel(m, v, false, ctx->stream));
     }
     run_sweep(ctx, L.B, prec->strips);
-    launched(ctx, 2);  // the two sentinel fills
     if (read_err(ctx) != 0) {
       CK(cudaMemsetAsync(ctx->err_word.p, 0, sizeof(int), ctx->stream));
       set_err(ctx, "a triangular-sweep wait timed out");
@@ -2180,7 +2172,7 @@ extern "C" int dfg_solve_pbicgstab(dfg_system sys, dfg_precond prec, int mode, d
     double* vec[7];
     for (int k = 0; k < 7; ++k) vec[k] = reinterpret_cast<double*>(w + k * v8);
     BicgVecs v{sys->res.as<double>(), sys->upd.as<double>(), vec[0], vec[1], vec[2], vec[3], vec[4], vec[5], vec[6],
-               prec->ybuf64.as<double>(), m};
+               {}, {}, m};
     BicgState* st = reinterpret_cast<BicgState*>(w + off_st);
     Red red2{reinterpret_cast<double*>(w + off_red), reinterpret_cast<unsigned*>(w + off_red + 2 * kRedGrid * 8),
              nullptr};
@@ -2191,7 +2183,8 @@ extern "C" int dfg_solve_pbicgstab(dfg_system sys, dfg_precond prec, int mode, d
     const PrecondLaunch P1 = precond_launch(ctx, prec, false, v.p, nullptr, v.mp, sc.tickets, done);
     const PrecondLaunch P2 = precond_launch(ctx, prec, false, v.s, nullptr, v.ms, sc.tickets, done);
     const SweepLaunch &F1 = P1.F, &B1 = P1.B, &F2 = P2.F, &B2 = P2.B;
-    const int feed_launches = prec->strips ? 3 : 0;  // strips: the sweeps' input and exchange buffers
+    v.feed_p = P1.feed;
+    v.feed_s = P2.feed;
     const int maxit = (int)std::min<unsigned>(*iteration, 0x7fffffffu);
     const double tol = *conv_ratio;
     CK(bicg_init(v, st, red, tol, maxit, sc.tickets, ctx->stream));
@@ -2204,18 +2197,15 @@ extern "C" int dfg_solve_pbicgstab(dfg_system sys, dfg_precond prec, int mode, d
     if (h.done == 0) {
       ensure_sell(ctx, sys, false);
       const MatView A = view64(sys);
-      const long long per_it =
-          5 + launches_of(F1) + launches_of(B1) + launches_of(F2) + launches_of(B2) + 2 * feed_launches;
+      const long long per_it = 5 + launches_of(F1) + launches_of(B1) + launches_of(F2) + launches_of(B2);
       const int chunk = std::max(2, std::min(m < 200000 ? 4 : 16, (int)(4096 / per_it)));
       Chunk g;
       CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
       for (int c = 0; c < chunk; ++c) {
-        if (feed_launches) enqueue_strip_feed(P1, v.p, m, ctx->stream);
         enqueue_sweep(F1, ctx->stream);
         enqueue_sweep(B1, ctx->stream, true);
         bicg_amp(A, v, st, red, ctx->stream);
         bicg_s(v, st, sc.tickets, ctx->stream);
-        if (feed_launches) enqueue_strip_feed(P2, v.s, m, ctx->stream);
         enqueue_sweep(F2, ctx->stream);
         enqueue_sweep(B2, ctx->stream, true);
         bicg_ams(A, v, st, red2, ctx->stream);

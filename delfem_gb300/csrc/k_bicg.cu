@@ -22,6 +22,7 @@
 #include <cmath>
 
 #include "dfg_common.cuh"
+#include "k_feed.cuh"
 #include "k_reduce.cuh"
 #include "k_rowmv.cuh"
 #include "k_solve.h"
@@ -60,7 +61,7 @@ __global__ void k_bicg_init0(BicgVecs v, BicgState* st, Red red, double tol, int
   }
 }
 
-// x := 0 x; r2 = r; p = r; sweep outputs to the sentinel; tickets reset
+// x := 0 x; r2 = r; p = r; the sweeps' feed; tickets reset
 __global__ void k_bicg_init1(BicgVecs v, BicgState* st, int* tickets) {
   if (st->done == 4) return;
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < v.m; k += (long long)gridDim.x * blockDim.x) {
@@ -68,9 +69,9 @@ __global__ void k_bicg_init1(BicgVecs v, BicgState* st, int* tickets) {
     const double r = v.r[k];
     v.r2[k] = r;
     v.p[k] = r;
-    v.y[k] = sentinel_value<double>();
-    v.mp[k] = sentinel_value<double>();
+    feed_put<double>(v.feed_p, k, r);
   }
+  feed_fill<double>(v.feed_p);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     tickets[0] = 0;
     tickets[1] = 0;
@@ -96,7 +97,7 @@ __global__ void __launch_bounds__(kSpmvTpb, 2) k_bicg_amp(MatView Am, BicgVecs v
   if (grid_sum(part, red, &tot) && threadIdx.x == 0) st->alpha = st->rho / tot;
 }
 
-// s = r; s += -alpha AMp; sweep outputs to the sentinel; tickets reset
+// s = r; s += -alpha AMp; the sweeps' feed; tickets reset
 __global__ void k_bicg_s(BicgVecs v, BicgState* st, int* tickets) {
   if (st->done) return;
   const double na = -st->alpha;
@@ -104,9 +105,9 @@ __global__ void k_bicg_s(BicgVecs v, BicgState* st, int* tickets) {
     double s = v.r[k];
     if (na != 0.0) s = axpy1(s, na, v.amp[k]);
     v.s[k] = s;
-    v.y[k] = sentinel_value<double>();
-    v.ms[k] = sentinel_value<double>();
+    feed_put<double>(v.feed_s, k, s);
   }
+  feed_fill<double>(v.feed_s);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     tickets[0] = 0;
     tickets[1] = 0;
@@ -181,9 +182,9 @@ __global__ void k_bicg_p(BicgVecs v, BicgState* st, int* tickets) {
     p = __dadd_rn(p, v.r[k]);
     if (c != 0.0) p = axpy1(p, c, v.amp[k]);
     v.p[k] = p;
-    v.y[k] = sentinel_value<double>();
-    v.mp[k] = sentinel_value<double>();
+    feed_put<double>(v.feed_p, k, p);
   }
+  feed_fill<double>(v.feed_p);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     tickets[0] = 0;
     tickets[1] = 0;

@@ -31,6 +31,7 @@
 #include <cmath>
 
 #include "dfg_common.cuh"
+#include "k_feed.cuh"
 #include "k_mbar.cuh"
 #include "k_rowmv.cuh"
 #include "k_solve.h"
@@ -152,18 +153,6 @@ struct GridWalk {
     return s_last != 0;
   }
 };
-
-template <typename Z, typename R>
-__device__ __forceinline__ void feed_put(const SweepFeed& f, long long k, R r) {
-  if (f.in) reinterpret_cast<Z*>(f.in)[f.pos ? f.pos[k] : k] = (Z)r;
-}
-template <typename Z>
-__device__ __forceinline__ void feed_fill(const SweepFeed& f) {
-  const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-    for (long long k = first; k < f.nfill[i]; k += step) reinterpret_cast<Z*>(f.fill[i])[k] = sentinel_value<Z>();
-}
 
 // Elements of the vectors: virtual block vb holds the elements vb*kRedTpb + t +
 // j*kRedGrid*kRedTpb.  Calls f(k) for the thread's elements, which returns what

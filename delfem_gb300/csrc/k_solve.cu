@@ -10,6 +10,7 @@
 #include <cmath>
 
 #include "dfg_common.cuh"
+#include "k_feed.cuh"
 #include "k_reduce.cuh"
 #include "k_rowmv.cuh"
 #include "k_solve.h"
@@ -79,20 +80,6 @@ cudaError_t sell_pack(int nslices, int b, const long long* ptr, const int* src, 
 template <typename Z>
 __device__ __forceinline__ double zval(const void* z, long long k) {
   return (double)reinterpret_cast<const Z*>(z)[k];
-}
-
-// element k of a residual into the forward sweep's input (Z: the sweeps' type)
-template <typename Z, typename R>
-__device__ __forceinline__ void feed_put(const SweepFeed& f, long long k, R r) {
-  if (f.in) reinterpret_cast<Z*>(f.in)[f.pos ? f.pos[k] : k] = (Z)r;
-}
-template <typename Z>
-__device__ __forceinline__ void feed_fill(const SweepFeed& f) {
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < f.nfill[i];
-         k += (long long)gridDim.x * blockDim.x)
-      reinterpret_cast<Z*>(f.fill[i])[k] = sentinel_value<Z>();
 }
 
 // x := 0 * x (SCAL(0,x)); rr0 = r.r; early exit below 1e-30; sentinels
@@ -371,6 +358,14 @@ __global__ void k_to_fp32(long long m, const double* a, float* b) {
     b[k] = (float)a[k];
 }
 
+// The sweeps' input where no solver kernel writes it (strips): r into step order,
+// exchange buffers, tickets.
+__global__ void k_sweep_feed(SweepFeed f, long long m, const double* r, int* tickets) {
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < m; k += (long long)gridDim.x * blockDim.x)
+    feed_put<double>(f, k, r[k]);
+  feed_fill<double>(f);
+  if (blockIdx.x == 0 && threadIdx.x < 2) tickets[threadIdx.x] = 0;
+}
 __global__ void k_fill_sentinel64(long long m, double* p) {
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < m; k += (long long)gridDim.x * blockDim.x)
     p[k] = sentinel_value<double>();
@@ -486,6 +481,11 @@ cudaError_t mix_accumulate(const MixVecs& v, cudaStream_t s) {
 }
 cudaError_t to_fp32(long long m, const double* a, float* b, cudaStream_t s) {
   if (m > 0) k_to_fp32 RED_LAUNCH(m, a, b);
+  return cudaGetLastError();
+}
+cudaError_t sweep_feed(const SweepFeed& f, long long m, const double* r, int* tickets, cudaStream_t s) {
+  const long long need = (m + kRedTpb - 1) / kRedTpb;
+  k_sweep_feed<<<(int)(need < 1 ? 1 : need < kRedGrid ? need : kRedGrid), kRedTpb, 0, s>>>(f, m, r, tickets);
   return cudaGetLastError();
 }
 cudaError_t fill_sentinel(long long m, void* p, bool fp32, cudaStream_t s) {

@@ -156,7 +156,7 @@ struct BicgVecs {
   double* ams; // A M^-1 s
   double* mp;  // M^-1 p
   double* ms;  // M^-1 s
-  double* y;   // forward-sweep output
+  SweepFeed feed_p, feed_s;  // for M^-1 p and M^-1 s
   long long m;
 };
 // red2: partials for 2 x kRedGrid values and its own counter
@@ -172,6 +172,7 @@ cudaError_t api_matvec(const MatView& A, double alpha, const double* x, double b
 cudaError_t api_axpy(long long m, double alpha, const double* x, double* y, cudaStream_t s);
 cudaError_t api_scal(long long m, double alpha, double* x, cudaStream_t s);
 cudaError_t api_dot(long long m, const double* x, const double* y, Red red, cudaStream_t s);
+cudaError_t sweep_feed(const SweepFeed& f, long long m, const double* r, int* tickets, cudaStream_t s);
 cudaError_t fill_sentinel(long long m, void* p, bool fp32, cudaStream_t s);
 
 }  // namespace dfg
