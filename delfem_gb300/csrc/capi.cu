@@ -127,8 +127,9 @@ Red red_of(dfg_ctx c, int channel = 0) {
 }
 
 IterRed iter_red_of(dfg_ctx c) {
-  return IterRed{c->iter_red.as<double>(),
-                 reinterpret_cast<unsigned*>(c->iter_red.as<char>() + 3 * kRedGrid * 8), c->err_word.as<int>()};
+  double* part = c->iter_red.as<double>();
+  double* slices = part + 3 * kRedGrid;
+  return IterRed{part, slices, reinterpret_cast<unsigned*>(slices + kIterSlices), c->err_word.as<int>()};
 }
 
 double* vec_ptr(dfg_ctx ctx_, dfg_system s, int iv) {
@@ -283,7 +284,7 @@ extern "C" int dfg_ctx_create(int device, dfg_ctx* out) {
     dalloc(c, c->scratch, kRedGrid * 8 + 16 * 4 + 16 * 8 + 16 * 4 + 256);
     CK(cudaMemsetAsync(c->err_word.p, 0, 64, c->stream));
     CK(cudaMemsetAsync(c->scratch.p, 0, c->scratch.bytes, c->stream));
-    dalloc(c, c->iter_red, 3 * kRedGrid * 8 + 64);
+    dalloc(c, c->iter_red, (3 * kRedGrid + kIterSlices) * 8 + 64);
     CK(cudaMemsetAsync(c->iter_red.p, 0, c->iter_red.bytes, c->stream));
     CK(sweep_set_smem_limits(c->smem_optin));
     CK(cudaHostAlloc(&c->h_pinned, kPinnedBytes, cudaHostAllocDefault));

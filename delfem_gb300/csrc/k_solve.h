@@ -126,8 +126,10 @@ cudaError_t to_fp32(long long m, const double* a, float* b, cudaStream_t s);
 // ---- one iteration between two preconditioner applications (k_iter.cu) ----
 // r.z, beta, the direction (unless `first`), A p, alpha, the r/x update with
 // the stop test and the sweeps' feed
+constexpr int kIterSlices = 1216;  // 32-row slices of the largest system whose blocks have 256 threads (152 SMs x 8)
 struct IterRed {
   double* part;   // 3 x kRedGrid
+  double* slices; // kIterSlices
   unsigned* bar;  // zero between launches
   int* err;       // device error word
 };

@@ -1,5 +1,6 @@
 """The fused PCG iteration (k_iter.cu) at the sizes where its grid changes:
-fewer rows than a warp, the last slice partly filled, one row slice more than
+fewer rows than a warp, the last slice partly filled, the largest system of one
+cluster and the smallest of the grid, one row slice more than
 eight per SM (blocks of 1024 threads), in all three forms and block sizes,
 against the oracle: FP64 iterations within +-2 and the solution to 1e-6, the
 FP32 forms to a true residual of 1e-8; the same bits when run again."""
@@ -12,11 +13,12 @@ pytestmark = pytest.mark.gpu
 def _problem(name):
     from delfem_gb300 import meshgen as mg
     return {"p3": lambda: mg.poisson2d_square(3, seed=1), "p31": lambda: mg.poisson2d_square(31, seed=2),
+            "p77": lambda: mg.poisson2d_square(77, seed=7), "p78": lambda: mg.poisson2d_square(78, seed=8),
             "s20x7": lambda: mg.solid2d_cantilever(20, 7, seed=3), "c5": lambda: mg.solid3d_cube(5, seed=4),
             "p196": lambda: mg.poisson2d_square(196, seed=5), "p198": lambda: mg.poisson2d_square(198, seed=6)}[name]()
 
 
-@pytest.mark.parametrize("name", ["p3", "p31", "s20x7", "c5", "p196", "p198"])
+@pytest.mark.parametrize("name", ["p3", "p31", "s20x7", "c5", "p77", "p78", "p196", "p198"])
 def test_fused_iteration(gpu_ctx, oracle_lib, name):
     from delfem_gb300.solver import FESolve
     p = _problem(name)
