@@ -1180,6 +1180,7 @@ SweepLaunch strip_launch(dfg_ctx ctx_, dfg_precond pr, int dir, bool fp32, void*
   L.ta.ticket = ticket;
   L.ta.err = ctx_->err_word.as<int>();
   L.ta.ne = D.ne;
+  L.ta.split = D.d.split;
   L.ta.W = D.W;
   L.ta.NS = D.NS;
   return L;
@@ -1258,7 +1259,7 @@ bool setup_strip(dfg_ctx ctx_, dfg_precond pr, const FactorPattern& F, bool forw
   D = StripDev{};
   const int n = pr->n, b = pr->b, elem = fp32 ? 4 : 8;
   StripPlan P;
-  if (!strip_plan(n, b, elem, F.rowptr, F.colind, F.diaind, forward, P)) return false;
+  if (!strip_plan(n, b, elem, F.rowptr, F.colind, F.diaind, forward, strip_can_split(b, elem), P)) return false;
   D.d = P.d;
   D.ne = P.ne;
   D.nstrips = P.nstrips;

@@ -37,7 +37,7 @@
 //
 // A row is evaluated by the operations of the other sweep kernels in their
 // order (entries ascending, FMA chain, then D^-1), so the ranged and one-CTA
-// kernels give the same bits.
+// kernels give the same bits; with split, column by column.
 //
 // Chunk layout: [need: CH ints, kStripHdr bytes][steps: step_bytes each]; a
 // step is pieces of 16 bytes per lane, piece j of lane l at (j*32 + l)*16:
@@ -210,14 +210,14 @@ __device__ __forceinline__ void receive(const StripSlot& S, int r, unsigned char
 
 // (one CTA per SM in the bounds: without it ptxas aims at several and keeps
 // steps to 64 registers and fewer, 2 to 10 % slower)
-template <typename T, int B, bool FWD, int NE>
+template <typename T, int B, bool FWD, int NE, bool SPLIT>
 __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(StripArgs a) {
   constexpr int SZ = (int)sizeof(T);
-  constexpr StripDims D = strip_dims(B, SZ, FWD, NE);
+  constexpr StripDims D = strip_dims(B, SZ, FWD, NE, SPLIT);
   constexpr int LPR = D.LPR, RW = D.RW, MC = D.MC, VC = D.VC, CH = D.CH, VS = D.VS;
   constexpr int BP = B == 3 ? 4 : B;          // elements of a row's value, padded
   constexpr int PER16 = 16 / SZ;
-  constexpr int EV = B * (LPR == 1 ? B : 1);  // values per entry and lane
+  constexpr int EV = B * B / LPR;             // values per entry and lane
   constexpr int RHS_CHUNK = CH * D.rhs_bytes;
   // values are loaded a step ahead where two sets of them fit the registers
   constexpr int VB = VC <= 8 ? 2 : 1;
@@ -341,7 +341,8 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
       } else {
         // ------------------------------------------------------------- compute
         const int c0 = S.strip_chunk[r], nch = S.strip_chunk[r + 1] - c0;
-        const int lr = lane / LPR, p = lane - lr * LPR;  // row of the step, component (LPR > 1)
+        const int lr = lane / LPR, el = lane - lr * LPR;  // row of the step, part of it (LPR > 1)
+        const int p = SPLIT ? el / B : el, col = SPLIT ? el % B : 0;  // component, column of the block
         T* out = reinterpret_cast<T*>(S.out) + p;
         T* xch = reinterpret_cast<T*>(S.xch) + p;
         // one step's data, loaded a step ahead of its use; the addresses taken
@@ -364,6 +365,8 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
           if constexpr (LPR == 1) {
 #pragma unroll
             for (int d = 0; d < B; ++d) t[k][d] = rh[lane * B + d];
+          } else if constexpr (SPLIT) {
+            t[k][0] = col == 0 ? rh[lr * B + p] : T(0);
           } else {
             t[k][0] = rh[lane];
           }
@@ -379,6 +382,7 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
           }
           o[k] = mint((NE + 1) / 2);
           xs[k] = mint((NE + 1) / 2 + 1);
+          if (SPLIT && col != 0) o[k] = xs[k] = -1;
           op[k] = out + (long long)o[k] * B;
           xp[k] = xch + (long long)xs[k] * BP;
           asm volatile("" : "+l"(op[k]), "+l"(xp[k]));
@@ -448,10 +452,11 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
             }
             auto A = [&](int i) -> T { return val[k % VB][i / PER16].v[i % PER16]; };
             // dependency values
-            Vec<T, BP> x[NE];
+            Vec<T, SPLIT ? 1 : BP> x[NE];
 #pragma unroll
             for (int e = 0; e < NE; ++e) {
-              x[e] = *reinterpret_cast<const Vec<T, BP>*>(reinterpret_cast<const float*>(smem) + cd[k][e]);
+              const float* at = reinterpret_cast<const float*>(smem) + cd[k][e];
+              x[e] = reinterpret_cast<const Vec<T, SPLIT ? 1 : BP>*>(at)[col];
             }
             // the last step's result leaves
             if (!XNOW) xstore(xs[k ^ 1], xp[k ^ 1], yl);
@@ -498,6 +503,18 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
               yl = y;
               if (XNOW) xstore(xs[k], xp[k], yl);
               if (SZ == 4 && more) decode((j + 1) % K2);
+            } else if constexpr (SPLIT) {
+              T acc = t[k][0];
+#pragma unroll
+              for (int e = 0; e < NE; ++e) acc -= A(e) * x[e].v[0];
+              acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+              if constexpr (FWD) {
+                acc = A(NE) * __shfl_sync(0xffffffffu, acc, lane - el + col * B);
+                acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+              }
+              rg[j * RW * BP + p] = acc;
+              yl.v[0] = acc;
+              if (XNOW) xstore(xs[k], xp[k], yl);
             } else {
               T acc = t[k][0];
 #pragma unroll
@@ -568,7 +585,7 @@ __global__ void k_strip_meta(int CH, int MC, int step_bytes, int chunk_bytes, co
 template <typename T, int B, bool FWD>
 __global__ void k_strip_pack(StripPackArgs a) {
   constexpr int SZ = (int)sizeof(T), PER16 = 16 / SZ, BS = B * B;
-  const int LPR = a.d.LPR, EV = B * (LPR == 1 ? B : 1);
+  const int LPR = a.d.LPR, EV = BS / LPR;
   const long long s = blockIdx.x;
   const int RW = a.d.RW, ne = a.ne;
   T* v = reinterpret_cast<T*>(a.rec + (size_t)(s / a.d.CH) * a.d.chunk_bytes + kStripHdr +
@@ -578,7 +595,7 @@ __global__ void k_strip_pack(StripPackArgs a) {
     const int l = lane / LPR, p = lane - l * LPR, e = k / EV, q = k - e * EV;
     double x = 0.0;
     if (l < RW) {
-      const int m = LPR == 1 ? q : p * B + q;
+      const int m = p * EV + q;
       if (e < ne) {
         const int c = a.ent_slot[((size_t)s * RW + l) * ne + e];
         if (c >= 0) x = a.foffd[(size_t)c * BS + m];
@@ -617,19 +634,30 @@ cudaError_t launch_strip_pack(bool forward, bool fp32, const StripPackArgs& a, c
   return forward ? pack_t<double, true>(a, st) : pack_t<double, false>(a, st);
 }
 
-// calls f(kernel) for the instance of (fp32, b, forward, ne)
-template <typename F>
-static cudaError_t with_kernel(bool fp32, int b, bool forward, int ne, F&& f) {
-#define DFG_STRIP_NE(T, B, FWD)                   switch (ne) {                                     case 3: return f(k_strip<T, B, FWD, 3>);        case 4: return f(k_strip<T, B, FWD, 4>);        case 7: return f(k_strip<T, B, FWD, 7>);        case 16: return f(k_strip<T, B, FWD, 16>);      default: return cudaErrorInvalidValue;        }
-#define DFG_STRIP_B(B)                                                                    if (fp32) {                                                                               if (forward) { DFG_STRIP_NE(float, B, true) } else { DFG_STRIP_NE(float, B, false) }   } else {                                                                                  if (forward) { DFG_STRIP_NE(double, B, true) } else { DFG_STRIP_NE(double, B, false) }   }
-  switch (b) {
-    case 1: DFG_STRIP_B(1)
-    case 2: DFG_STRIP_B(2)
-    case 3: DFG_STRIP_B(3)
+// calls f(kernel) for the instance of (fp32, b, forward, ne, split)
+template <typename T, int B, bool FWD, bool SPLIT, typename F>
+static cudaError_t with_class(int ne, F&& f) {
+  switch (ne) {
+    case 3: return f(k_strip<T, B, FWD, 3, SPLIT>);
+    case 4: return f(k_strip<T, B, FWD, 4, SPLIT>);
+    case 7: return f(k_strip<T, B, FWD, 7, SPLIT>);
+    case 16: return f(k_strip<T, B, FWD, 16, SPLIT>);
     default: return cudaErrorInvalidValue;
   }
-#undef DFG_STRIP_B
-#undef DFG_STRIP_NE
+}
+template <typename T, typename F>
+static cudaError_t with_block(int b, bool forward, int ne, F&& f) {
+  switch (b) {
+    case 1: return forward ? with_class<T, 1, true, false>(ne, f) : with_class<T, 1, false, false>(ne, f);
+    case 2: return forward ? with_class<T, 2, true, false>(ne, f) : with_class<T, 2, false, false>(ne, f);
+    case 3: return forward ? with_class<T, 3, true, false>(ne, f) : with_class<T, 3, false, false>(ne, f);
+    default: return cudaErrorInvalidValue;
+  }
+}
+template <typename F>
+static cudaError_t with_kernel(bool fp32, int b, bool forward, int ne, bool split, F&& f) {
+  if (split) return forward ? with_class<double, 2, true, true>(ne, f) : with_class<double, 2, false, true>(ne, f);
+  return fp32 ? with_block<float>(b, forward, ne, f) : with_block<double>(b, forward, ne, f);
 }
 
 cudaError_t launch_strip(bool forward, bool fp32, int b, const StripArgs& a, int grid, size_t smem, cudaStream_t st,
@@ -644,19 +672,19 @@ cudaError_t launch_strip(bool forward, bool fp32, int b, const StripArgs& a, int
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = dep ? 1 : 0;
-  return with_kernel(fp32, b, forward, a.ne, [&](auto k) { return cudaLaunchKernelEx(&cfg, k, a); });
+  return with_kernel(fp32, b, forward, a.ne, a.split, [&](auto k) { return cudaLaunchKernelEx(&cfg, k, a); });
 }
 
 cudaError_t strip_set_smem_limits(size_t max_smem) {
-  for (int fp32 = 0; fp32 < 2; ++fp32)
-    for (int b = 1; b <= 3; ++b)
-      for (int fwd = 0; fwd < 2; ++fwd)
-        for (int ne : {3, 4, 7, 16}) {
-          const cudaError_t e = with_kernel(fp32, b, fwd, ne, [&](auto k) {
-            return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem);
-          });
-          if (e != cudaSuccess) return e;
-        }
+  auto set = [&](auto k) { return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem); };
+  for (int fwd = 0; fwd < 2; ++fwd)
+    for (int ne : {3, 4, 7, 16})
+      for (int b = 1; b <= 3; ++b)
+        for (int fp32 = 0; fp32 < 2; ++fp32)
+          for (int split = 0; split <= (strip_can_split(b, fp32 ? 4 : 8) ? 1 : 0); ++split) {
+            const cudaError_t e = with_kernel(fp32, b, fwd, ne, split, set);
+            if (e != cudaSuccess) return e;
+          }
   return cudaSuccess;
 }
 

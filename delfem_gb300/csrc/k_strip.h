@@ -17,7 +17,8 @@ namespace dfg {
 // Shapes that follow from the block size, the element size, the direction and
 // the entry class (entries per row: 3, 4, 7 or 16).
 struct StripDims {
-  int LPR;     // lanes per row: 1, or b (lane = one component of a row)
+  bool split;  // a lane per element of a row's blocks
+  int LPR;     // lanes per row: 1, b (lane = one component of a row) or b*b
   int RW;      // rows per step
   int MC;      // 16-byte pieces of metadata per lane and step
   int VC;      // 16-byte pieces of factor values per lane and step
@@ -41,15 +42,26 @@ constexpr int kStripEnd = 0x7fffffff;  // item count of steps after a strip's la
 // those weigh more (elasticity on 56^3 cells 102 us per sweep with three lanes
 // per row, 81 with one; on 24^3 37 and 34).  3x3 rows of more than 7 entries do
 // not fit one lane's registers.
-__host__ __device__ constexpr int strip_lpr(int b, int elem, int ne) {
-  return elem == 8 || (b == 3 && ne > 7) ? b : 1;
+//
+// split (2x2 FP64): each element of the blocks takes a lane, a row's sum being
+// those of its two columns: 6 dependent operations a level instead of 8 (forward,
+// 3 entries), 4 instead of 6 (backward), for strips of 8 lines instead of 16.  2D
+// elasticity on 200x100 cells 129 / 100 -> 116 / 83 us per sweep (forward /
+// backward), 1000x500 594 / 479 -> 567 / 404, ILU(1) on 161x83 162 / 130 -> 135 /
+// 100.  The sums round differently from those of the other sweep kernels (their
+// error against a wider type is no larger); the server, whose kernels give the
+// same bits, does not split.
+__host__ __device__ constexpr int strip_lpr(int b, int elem, int ne, bool split) {
+  return split ? b * b : elem == 8 || (b == 3 && ne > 7) ? b : 1;
 }
-__host__ __device__ constexpr StripDims strip_dims(int b, int elem, bool forward, int ne) {
+constexpr bool strip_can_split(int b, int elem) { return b == 2 && elem == 8; }
+__host__ __device__ constexpr StripDims strip_dims(int b, int elem, bool forward, int ne, bool split) {
   StripDims d{};
-  d.LPR = strip_lpr(b, elem, ne);
+  d.split = split;
+  d.LPR = strip_lpr(b, elem, ne, split);
   d.RW = 32 / d.LPR;
   d.MC = ((ne + 1) / 2 + 2 + 3) / 4;
-  const int per_lane = (ne + (forward ? 1 : 0)) * b * (d.LPR == 1 ? b : 1);
+  const int per_lane = (ne + (forward ? 1 : 0)) * (b * b / d.LPR);
   d.VC = (per_lane * elem + 15) / 16;
   d.VS = (b == 3 ? 4 : b) * elem;
   d.step_bytes = 512 * (d.MC + d.VC);
@@ -109,8 +121,9 @@ __host__ __device__ constexpr size_t strip_region_offset(const StripDims& d, int
 inline size_t strip_smem_bytes(const StripDims& d, int W, int NS) { return strip_stage_offset(d, W, NS, W); }
 // False when the rows do not fit the sweep: more than 16 entries in a row, or
 // more dependencies on other strips within a chunk than the mailbox holds.
+// split: only where strip_can_split.
 bool strip_plan(int n, int b, int elem, const int* rowptr, const int* colind, const int* diaind, bool forward,
-                StripPlan& P);
+                bool split, StripPlan& P);
 // Metadata of every step and lane as the records hold it ([step][piece][lane]
 // of 4 ints): ne 16-bit codes (offset / 4 from the start of the CTA's dynamic
 // shared memory, for W warps of NS stages each), then the output position (-1:
@@ -151,6 +164,7 @@ struct StripArgs {
   int* other_ticket;  // optional: set to 0
   int* err;      // device error word
   int ne;        // entry class
+  bool split;    // StripDims
   int W;         // strips (compute warps) per CTA
   int NS;        // chunk stages per warp
 };

@@ -363,7 +363,7 @@ constexpr int kServeStripWarps = 1;  // strips per CTA
 bool use_strips(const dfg_server_s* S, Req* r, int elem) {
   if (S->sweeps != 0) return false;
   for (int dir = 0; dir < 2; ++dir)
-    if (!strip_plan(r->n, r->b, elem, r->rowptr.data(), r->colind.data(), r->diaind.data(), dir == 0, r->strip[dir]) ||
+    if (!strip_plan(r->n, r->b, elem, r->rowptr.data(), r->colind.data(), r->diaind.data(), dir == 0, false, r->strip[dir]) ||
         S->strip_ns[strip_class_index(r->b, r->strip[dir].ne)][dir] == 0)
       return false;
   return true;
@@ -1439,7 +1439,7 @@ void class_shapes(dfg_server_s* S) {
     const int b = k / 4 + 1;
     size_t worst = 0;
     for (int dir = 0; dir < 2; ++dir) {
-      const StripDims d = strip_dims(b, elem, dir == 0, kStripNe[k % 4]);
+      const StripDims d = strip_dims(b, elem, dir == 0, kStripNe[k % 4], false);
       int ns = 8;
       while (ns > 2 && strip_smem_bytes(d, kServeStripWarps, ns) > (size_t)per_sm_bytes / 4 - 1024) --ns;
       S->strip_smem[k][dir] = strip_smem_bytes(d, kServeStripWarps, ns);

@@ -135,7 +135,7 @@ bool tile_strips(const Rows& R, int RW, std::vector<int>& strip, std::vector<int
 
 }  // namespace
 
-bool strip_plan(int n, int b, int elem, const int* rowptr, const int* colind, const int* diaind, bool forward,
+bool strip_plan(int n, int b, int elem, const int* rowptr, const int* colind, const int* diaind, bool forward, bool split,
                 StripPlan& P) {
   P = StripPlan{};
   P.forward = forward;
@@ -149,7 +149,7 @@ bool strip_plan(int n, int b, int elem, const int* rowptr, const int* colind, co
   for (int i = 0; i < n; ++i) maxe = std::max(maxe, end(i) - first(i));
   P.ne = strip_class(maxe);
   if (n == 0 || P.ne == 0) return false;
-  P.d = strip_dims(b, elem, forward, P.ne);
+  P.d = strip_dims(b, elem, forward, P.ne, split);
   const int RW = P.d.RW, CH = P.d.CH, ne = P.ne;
 
   // level of every row in the whole sweep

@@ -11,7 +11,7 @@ using namespace dfg;
 // info: strips, steps, exchange slots, items; returns 0, or the number of the
 // check that failed (-1: the rows do not fit the sweep)
 extern "C" int emul_strip(int n, int b, int elem, const int* rowptr, const int* colind, int forward, int eager,
-                          long long* info) {
+                          int split, long long* info) {
   std::vector<int> diaind(n);
   for (int i = 0; i < n; ++i) {
     int d = rowptr[i];
@@ -19,7 +19,7 @@ extern "C" int emul_strip(int n, int b, int elem, const int* rowptr, const int* 
     diaind[i] = d;
   }
   StripPlan P;
-  if (!strip_plan(n, b, elem, rowptr, colind, diaind.data(), forward != 0, P)) return -1;
+  if (!strip_plan(n, b, elem, rowptr, colind, diaind.data(), forward != 0, split != 0, P)) return -1;
   const StripDims& d = P.d;
   const int W = 3, NS = 2;
   const int M = strip_mailbox(d.VS), ne = P.ne, iout = (ne + 1) / 2;

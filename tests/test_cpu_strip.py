@@ -24,15 +24,15 @@ def strip_lib():
                    check=True)
     L = ctypes.CDLL(so)
     P = ctypes.c_void_p
-    L.emul_strip.argtypes = [ctypes.c_int] * 3 + [P, P, ctypes.c_int, ctypes.c_int, P]
+    L.emul_strip.argtypes = [ctypes.c_int] * 3 + [P, P, ctypes.c_int, ctypes.c_int, ctypes.c_int, P]
     return L
 
 
-def _run(L, rowptr, colind, b, elem, forward, eager):
+def _run(L, rowptr, colind, b, elem, forward, eager, split=0):
     info = np.zeros(4, np.int64)
     ci = np.ascontiguousarray(colind if colind.size else np.zeros(1), np.int32)
     rp = np.ascontiguousarray(rowptr, np.int32)
-    rc = L.emul_strip(rp.size - 1, b, elem, rp.ctypes.data, ci.ctypes.data, forward, eager, info.ctypes.data)
+    rc = L.emul_strip(rp.size - 1, b, elem, rp.ctypes.data, ci.ctypes.data, forward, eager, split, info.ctypes.data)
     return rc, info
 
 
@@ -60,8 +60,9 @@ def test_strip_plan(strip_lib, oracle_lib, name, b, elem):
     rowptr, colind = _pattern(name)
     for forward in (1, 0):
         for eager in (0, 1):
-            rc, info = _run(strip_lib, rowptr, colind, b, elem, forward, eager)
-            assert rc == 0, (rc, info)
+            for split in (0, 1) if (b, elem) == (2, 8) else (0,):
+                rc, info = _run(strip_lib, rowptr, colind, b, elem, forward, eager, split)
+                assert rc == 0, (rc, info, split)
 
 
 def test_strip_plan_steps_are_levels_of_a_grid(strip_lib, oracle_lib):

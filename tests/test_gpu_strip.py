@@ -3,7 +3,11 @@ where their plan can go wrong: one line and one line more than a strip, more
 items than a mailbox has slots, more strips than the device has CTAs, and every
 entry class.  A row is evaluated in the one-CTA kernel's order, so both kinds
 give the same bits, in FP64 and (through a few FP32-factor iterations) in FP32;
-the FP64 preconditioner also meets the oracle's to 1e-12."""
+the FP64 preconditioner also meets the oracle's to 1e-12.  2x2 blocks in FP64 are
+summed by columns: there FP64 agrees to rounding (1e-12 through the oracle, a few
+iterations to 1e-10), and the error against sums in a wider type is the one-CTA kernel's,
+but for the one rounding more of a row's two halves (its 6 operations or more
+make that 1/6 at most, and 1.5 leaves room for chance)."""
 import numpy as np
 import pytest
 
@@ -59,8 +63,56 @@ def test_strip_sweeps(gpu_ctx, oracle_lib, name, fill):
             got[mode] = (z, x32, s.solution())
         finally:
             s.close()
+    if b == 2:
+        (z, x32, x64), (z3, y32, y64) = got[1], got[3]
+        assert np.array_equal(x32, y32)
+        assert np.linalg.norm(x64 - y64) <= 1e-10 * np.linalg.norm(y64)
+        np.testing.assert_allclose(z3, zref, rtol=1e-12, atol=1e-13 * np.abs(zref).max())
+        return
     for a, c in zip(got[1], got[3]):
         assert np.array_equal(a, c)
+
+
+def _substitute_wide(rp, ci, fd, fo, rhs):
+    n, z = fd.shape[0], rhs.reshape(-1, 2).astype(np.longdouble)
+    for i in range(n):  # L y = r, D^-1 applied
+        for c in range(rp[i], rp[i + 1]):
+            if ci[c] < i:
+                z[i] -= fo[c].astype(np.longdouble) @ z[ci[c]]
+        z[i] = fd[i].astype(np.longdouble) @ z[i]
+    for i in range(n - 1, -1, -1):
+        for c in range(rp[i], rp[i + 1]):
+            if ci[c] > i:
+                z[i] -= fo[c].astype(np.longdouble) @ z[ci[c]]
+    return z
+
+
+@pytest.mark.parametrize("name,fill", [("solid2d:45x38", 0), ("solid2d:30x21", 1)])
+def test_split_strips_are_as_exact(gpu_ctx, name, fill):
+    if np.finfo(np.longdouble).nmant <= 52:
+        pytest.skip("no wider type than FP64 here")
+    from delfem_gb300.solver import FESolve
+    p = _problem(name)
+    err = {}
+    for mode in (1, 3):
+        s = FESolve(gpu_ctx, p, fill_level=fill, sweep_mode=mode)
+        try:
+            s.assemble()
+            assert s.factor()
+            rp, ci = s.prec.GetPattern()
+            fd, fo = (np.asarray(v).reshape(-1, 2, 2) for v in s.prec.GetFactor())
+            s.ls.ReSizeTmpVecSolver(1)
+            err[mode] = 0.0
+            for seed in range(3):
+                rhs = np.random.default_rng(seed).standard_normal(p.nnode * 2)
+                s.ls.SetVector(0, rhs)
+                s.prec.SolvePrecond(s.ls, 0)
+                ref = _substitute_wide(rp, ci, fd, fo, rhs)
+                err[mode] += float(np.linalg.norm(s.ls.GetVector(0).reshape(-1, 2) - ref) / np.linalg.norm(ref))
+        finally:
+            s.close()
+    print("error against sums in a wider type: by columns %.3g, in order %.3g" % (err[1] / 3, err[3] / 3))
+    assert err[1] <= 1.5 * err[3]
 
 
 @pytest.mark.parametrize("mode", ["fp64", "fp32f", "mixed"])
