@@ -1258,15 +1258,23 @@ bool setup_strip(dfg_ctx ctx_, dfg_precond pr, const FactorPattern& F, bool forw
   StripDev& D = pr->strip[forward ? 0 : 1][fp32 ? 1 : 0];
   D = StripDev{};
   const int n = pr->n, b = pr->b, elem = fp32 ? 4 : 8;
+  // 3x3 rows are split over four warps unless the strips are more than two per
+  // SM: a level takes 12 FP64 operations of four schedulers per 12 rows instead of
+  // 24 of one per 10 rows, a longer time on a full chip (elasticity on 56^3 cells,
+  // 285 strips, 240 / 219 -> 220 / 182 us per sweep; 72^3, 460 strips, 320 / 293 ->
+  // 373 / 310).
   StripPlan P;
-  if (!strip_plan(n, b, elem, F.rowptr, F.colind, F.diaind, forward, strip_can_split(b, elem), P)) return false;
+  const bool split = strip_can_split(b, elem);
+  if (!strip_plan(n, b, elem, F.rowptr, F.colind, F.diaind, forward, split, P)) return false;
+  if (P.d.Q > 1 && P.nstrips > 2 * ctx_->nsm && !strip_plan(n, b, elem, F.rowptr, F.colind, F.diaind, forward, false, P))
+    return false;
   D.d = P.d;
   D.ne = P.ne;
   D.nstrips = P.nstrips;
   D.nsteps = P.steps();
   D.nxch = (long long)P.nexport * (P.d.VS / elem);
   // one strip per CTA while the strips fit the SMs
-  D.W = std::min(kStripMaxWarps, std::max(1, (P.nstrips + ctx_->nsm - 1) / ctx_->nsm));
+  D.W = P.d.Q > 1 ? 1 : std::min(kStripMaxWarps, std::max(1, (P.nstrips + ctx_->nsm - 1) / ctx_->nsm));
   const size_t budget = ctx_->smem_optin;
   // As many chunk stages as fit.  FP32 steps are short: they give a strip up
   // rather than run with two stages, which do not cover a copy (elasticity on

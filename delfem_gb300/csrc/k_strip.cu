@@ -214,7 +214,7 @@ template <typename T, int B, bool FWD, int NE, bool SPLIT>
 __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(StripArgs a) {
   constexpr int SZ = (int)sizeof(T);
   constexpr StripDims D = strip_dims(B, SZ, FWD, NE, SPLIT);
-  constexpr int LPR = D.LPR, RW = D.RW, MC = D.MC, VC = D.VC, CH = D.CH, VS = D.VS;
+  constexpr int LPR = D.LPR, Q = D.Q, RW = D.RW, MC = D.MC, VC = D.VC, CH = D.CH, VS = D.VS;
   constexpr int BP = B == 3 ? 4 : B;          // elements of a row's value, padded
   constexpr int PER16 = 16 / SZ;
   constexpr int EV = B * B / LPR;             // values per entry and lane
@@ -234,8 +234,8 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
   __shared__ int s_group, s_slot, s_stop;
   const int W = a.W, NS = a.NS;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool compute = warp < W, load_warp = warp == 2 * W;
-  const int w = compute ? warp : load_warp ? min(lane, W - 1) : warp - W;  // (the loader's lane w serves warp w)
+  const bool compute = warp < W * Q, load_warp = warp == W * Q + W;
+  const int w = compute ? warp / Q : load_warp ? min(lane, W - 1) : warp - W * Q;  // (the loader's lane w serves strip w)
   uint64_t* full = reinterpret_cast<uint64_t*>(smem) + w * NS;
   int* delivered = reinterpret_cast<int*>(smem + (size_t)W * NS * 8) + w * 4;
   int* consumed = delivered + 1;
@@ -341,7 +341,13 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
       } else {
         // ------------------------------------------------------------- compute
         const int c0 = S.strip_chunk[r], nch = S.strip_chunk[r + 1] - c0;
-        const int lr = lane / LPR, el = lane - lr * LPR;  // row of the step, part of it (LPR > 1)
+        const int tid = warp % Q * 32 + lane;                             // lane of the strip
+        const int lr = strip_row(D, tid), el = lane - lane / LPR * LPR;  // row of the step, part of it (LPR > 1)
+        // the strip's warps meet after every step
+        auto step_sync = [&] {
+          if constexpr (Q == 1) __syncwarp();
+          else asm volatile("bar.sync %0, %1;" ::"r"(1 + w), "n"(32 * Q) : "memory");
+        };
         const int p = SPLIT ? el / B : el, col = SPLIT ? el % B : 0;  // component, column of the block
         T* out = reinterpret_cast<T*>(S.out) + p;
         T* xch = reinterpret_cast<T*>(S.xch) + p;
@@ -357,16 +363,16 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
         T *op[2], *xp[2];
         auto load = [&](int k, const unsigned char* sp, const unsigned char* vp) {
 #pragma unroll
-          for (int j = 0; j < MC; ++j) meta[j] = *reinterpret_cast<const int4*>(sp + j * 512);
+          for (int j = 0; j < MC; ++j) meta[j] = *reinterpret_cast<const int4*>(sp + j * 512 * Q);
 #pragma unroll
           for (int j = 0; j < VC; ++j)
-            if (VB == 2) val[k % VB][j] = *reinterpret_cast<const Vec<T, PER16>*>(sp + (MC + j) * 512);
+            if (VB == 2) val[k % VB][j] = *reinterpret_cast<const Vec<T, PER16>*>(sp + (MC + j) * 512 * Q);
           const T* rh = reinterpret_cast<const T*>(vp);
           if constexpr (LPR == 1) {
 #pragma unroll
             for (int d = 0; d < B; ++d) t[k][d] = rh[lane * B + d];
           } else if constexpr (SPLIT) {
-            t[k][0] = col == 0 ? rh[lr * B + p] : T(0);
+            t[k][0] = col == 0 && lr < RW ? rh[lr * B + p] : T(0);
           } else {
             t[k][0] = rh[lane];
           }
@@ -388,6 +394,16 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
           asm volatile("" : "+l"(op[k]), "+l"(xp[k]));
         };
         T* const ring0 = reinterpret_cast<T*>(region + kStripZero) + lr * BP;
+        // the sum over the columns of a row's component (SPLIT)
+        auto columns = [&](T v) -> T {
+          if constexpr (B == 2) {
+            return v + __shfl_xor_sync(0xffffffffu, v, 1);
+          } else {
+            const int l0 = lane - el + p * B;
+            const T sum = __shfl_sync(0xffffffffu, v, l0) + __shfl_sync(0xffffffffu, v, l0 + 1);
+            return sum + __shfl_sync(0xffffffffu, v, l0 + 2);
+          }
+        };
         bool abort = false;
         Vec<T, LPR == 1 ? BP : 1> yl;  // the last step's result
 #pragma unroll
@@ -414,12 +430,12 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
         };
         abort = !__all_sync(0xffffffffu, mbar_wait(&full[st], (unsigned)ph, a.err, kSiteFull, -1, r));
         int have = 0;
-        const unsigned char *const sp0 = rstage + kStripHdr + lane * 16, *const vp0 = vstage;
+        const unsigned char *const sp0 = rstage + kStripHdr + tid * 16, *const vp0 = vstage;
         const unsigned char *sp = sp0 + (size_t)st * D.chunk_bytes, *vp = vp0 + (size_t)st * RHS_CHUNK;
         int need[CH];  // (one in G is used)
         auto load_need = [&](const unsigned char* s) {
 #pragma unroll
-          for (int j = G - 1; j < CH; j += G) need[j] = reinterpret_cast<const int*>(s - kStripHdr - lane * 16)[j];
+          for (int j = G - 1; j < CH; j += G) need[j] = reinterpret_cast<const int*>(s - kStripHdr - tid * 16)[j];
         };
         if (!abort) {
           load(0, sp, vp);
@@ -427,7 +443,8 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
           load_need(sp);
         }
         T* rg = ring0;
-        for (int c = 0; c < nch && !abort; ++c) {
+        // (a strip of several warps meets in every step, also after one has given up)
+        for (int c = 0; c < nch && (Q > 1 || !abort); ++c) {
           if (++st == NS) { st = 0; ph ^= 1; }
           // the test for the next chunk takes about 100 cycles: asked for here,
           // looked at in the last step
@@ -436,19 +453,27 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
           const unsigned char* vp1 = st == 0 ? vp0 : vp + RHS_CHUNK;
 #pragma unroll
           for (int j = 0; j < CH; ++j) {
+            if (Q > 1 && abort) {
+              step_sync();
+              continue;
+            }
             if (j % G == 0 && need[j + G - 1] > have) {
               // only padding is left of the strip (the last step's stores are in set 1)
               static_assert(!D.ends || G % 2 == 0, "the end is seen in an even step");
               if (D.ends && need[j + G - 1] == kStripEnd) break;
               have = wait_for(delivered, need[j + G - 1], kSitePoll);
-              if (abort) break;
+              if (abort) {
+                if (Q == 1) break;
+                step_sync();
+                continue;
+              }
             }
             constexpr int K2 = 2;
             const int k = j % K2;
             if (VB == 1) {
 #pragma unroll
               for (int v = 0; v < VC; ++v)
-                val[0][v] = *reinterpret_cast<const Vec<T, PER16>*>(sp + j * D.step_bytes + (MC + v) * 512);
+                val[0][v] = *reinterpret_cast<const Vec<T, PER16>*>(sp + j * D.step_bytes + (MC + v) * 512 * Q);
             }
             auto A = [&](int i) -> T { return val[k % VB][i / PER16].v[i % PER16]; };
             // dependency values
@@ -469,7 +494,9 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
               if (!__all_sync(0xffffffffu, landed) &&
                   !__all_sync(0xffffffffu, mbar_wait(&full[st], (unsigned)ph, a.err, kSiteFull, -1, r))) {
                 abort = true;
-                break;
+                if (Q == 1) break;
+                step_sync();
+                continue;
               }
               load(0, sp1, vp1);
               load_need(sp1);
@@ -507,12 +534,9 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
               T acc = t[k][0];
 #pragma unroll
               for (int e = 0; e < NE; ++e) acc -= A(e) * x[e].v[0];
-              acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-              if constexpr (FWD) {
-                acc = A(NE) * __shfl_sync(0xffffffffu, acc, lane - el + col * B);
-                acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-              }
-              rg[j * RW * BP + p] = acc;
+              acc = columns(acc);
+              if constexpr (FWD) acc = columns(A(NE) * __shfl_sync(0xffffffffu, acc, lane - el + col * B));
+              if (lr < RW) rg[j * RW * BP + p] = acc;
               yl.v[0] = acc;
               if (XNOW) xstore(xs[k], xp[k], yl);
             } else {
@@ -536,10 +560,10 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
               if (XNOW) xstore(xs[k], xp[k], yl);
               if (SZ == 4 && more) decode((j + 1) % K2);
             }
-            __syncwarp();
+            step_sync();
           }
-          if (abort) break;
-          if (lane == 0) st_release_s(consumed, (c + 1) * CH);  // the chunk's stage is free
+          if (Q == 1 && abort) break;
+          if (tid == 0) st_release_s(consumed, (c + 1) * CH);  // the chunk's stage is free
           sp = sp1;
           vp = vp1;
           rg = (c + 1) * CH % kStripRing == 0 ? ring0 : rg + CH * RW * BP;
@@ -570,12 +594,12 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
 
 // ------------------------------------------------------------------ records
 
-__global__ void k_strip_meta(int CH, int MC, int step_bytes, int chunk_bytes, const int* __restrict__ meta,
+__global__ void k_strip_meta(int CH, int lane_pieces, int step_bytes, int chunk_bytes, const int* __restrict__ meta,
                              const int* __restrict__ need, unsigned char* rec) {
   unsigned char* ck = rec + (size_t)blockIdx.x * chunk_bytes;
   if (threadIdx.x < kStripHdr / 4)
     reinterpret_cast<int*>(ck)[threadIdx.x] = (int)threadIdx.x < CH ? need[(size_t)blockIdx.x * CH + threadIdx.x] : 0;
-  const int per = MC * 32;  // pieces per step
+  const int per = lane_pieces;  // pieces per step
   const int4* m = reinterpret_cast<const int4*>(meta) + (size_t)blockIdx.x * CH * per;
   for (int i = threadIdx.x; i < CH * per; i += blockDim.x)
     reinterpret_cast<int4*>(ck + kStripHdr + (size_t)(i / per) * step_bytes)[i % per] = m[i];
@@ -585,14 +609,14 @@ __global__ void k_strip_meta(int CH, int MC, int step_bytes, int chunk_bytes, co
 template <typename T, int B, bool FWD>
 __global__ void k_strip_pack(StripPackArgs a) {
   constexpr int SZ = (int)sizeof(T), PER16 = 16 / SZ, BS = B * B;
-  const int LPR = a.d.LPR, EV = BS / LPR;
+  const int LPR = a.d.LPR, EV = BS / LPR, lanes = 32 * a.d.Q;
   const long long s = blockIdx.x;
   const int RW = a.d.RW, ne = a.ne;
   T* v = reinterpret_cast<T*>(a.rec + (size_t)(s / a.d.CH) * a.d.chunk_bytes + kStripHdr +
-                              (size_t)(s % a.d.CH) * a.d.step_bytes + (size_t)a.d.MC * 512);
-  for (int i = threadIdx.x; i < a.d.VC * 32 * PER16; i += blockDim.x) {
-    const int lane = (i / PER16) & 31, k = (i / PER16 / 32) * PER16 + i % PER16;
-    const int l = lane / LPR, p = lane - l * LPR, e = k / EV, q = k - e * EV;
+                              (size_t)(s % a.d.CH) * a.d.step_bytes + (size_t)a.d.MC * lanes * 16);
+  for (int i = threadIdx.x; i < a.d.VC * lanes * PER16; i += blockDim.x) {
+    const int lane = i / PER16 % lanes, k = (i / PER16 / lanes) * PER16 + i % PER16;
+    const int l = strip_row(a.d, lane), p = lane % 32 % LPR, e = k / EV, q = k - e * EV;
     double x = 0.0;
     if (l < RW) {
       const int m = p * EV + q;
@@ -613,7 +637,7 @@ __global__ void k_strip_pack(StripPackArgs a) {
 cudaError_t launch_strip_meta(const StripDims& d, int nchunks, const int* meta, const int* need, unsigned char* rec,
                               cudaStream_t st) {
   if (nchunks <= 0) return cudaSuccess;
-  k_strip_meta<<<nchunks, 128, 0, st>>>(d.CH, d.MC, d.step_bytes, d.chunk_bytes, meta, need, rec);
+  k_strip_meta<<<nchunks, 128, 0, st>>>(d.CH, d.MC * 32 * d.Q, d.step_bytes, d.chunk_bytes, meta, need, rec);
   return cudaGetLastError();
 }
 
@@ -656,7 +680,8 @@ static cudaError_t with_block(int b, bool forward, int ne, F&& f) {
 }
 template <typename F>
 static cudaError_t with_kernel(bool fp32, int b, bool forward, int ne, bool split, F&& f) {
-  if (split) return forward ? with_class<double, 2, true, true>(ne, f) : with_class<double, 2, false, true>(ne, f);
+  if (split && b == 2) return forward ? with_class<double, 2, true, true>(ne, f) : with_class<double, 2, false, true>(ne, f);
+  if (split && b == 3) return forward ? with_class<double, 3, true, true>(ne, f) : with_class<double, 3, false, true>(ne, f);
   return fp32 ? with_block<float>(b, forward, ne, f) : with_block<double>(b, forward, ne, f);
 }
 
@@ -664,7 +689,8 @@ cudaError_t launch_strip(bool forward, bool fp32, int b, const StripArgs& a, int
                          bool dep) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(32 * (2 * a.W + 1));
+  const int Q = a.split && b == 3 ? 4 : 1;  // warps per strip
+  cfg.blockDim = dim3(32 * (a.W * (Q + 1) + 1));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];

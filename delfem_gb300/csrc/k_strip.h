@@ -19,6 +19,7 @@ namespace dfg {
 struct StripDims {
   bool split;  // a lane per element of a row's blocks
   int LPR;     // lanes per row: 1, b (lane = one component of a row) or b*b
+  int Q;       // warps per strip
   int RW;      // rows per step
   int MC;      // 16-byte pieces of metadata per lane and step
   int VC;      // 16-byte pieces of factor values per lane and step
@@ -43,28 +44,36 @@ constexpr int kStripEnd = 0x7fffffff;  // item count of steps after a strip's la
 // per row, 81 with one; on 24^3 37 and 34).  3x3 rows of more than 7 entries do
 // not fit one lane's registers.
 //
-// split (2x2 FP64): each element of the blocks takes a lane, a row's sum being
-// those of its two columns: 6 dependent operations a level instead of 8 (forward,
-// 3 entries), 4 instead of 6 (backward), for strips of 8 lines instead of 16.  2D
+// split (2x2 and 3x3 FP64): each element of the blocks takes a lane, a row's sum being
+// that of its columns' sums.  2x2 with 3 entries: 6 dependent operations a level
+// instead of 8 (backward 4 instead of 6), for strips of 8 lines instead of 16: 2D
 // elasticity on 200x100 cells 129 / 100 -> 116 / 83 us per sweep (forward /
 // backward), 1000x500 594 / 479 -> 567 / 404, ILU(1) on 161x83 162 / 130 -> 135 /
-// 100.  The sums round differently from those of the other sweep kernels (their
+// 100.  3x3 FP64 with 7 entries: 12 operations instead of 24 (9 instead of 21), by
+// four warps, one per scheduler, that meet at a barrier after every step; 12 lines
+// per strip instead of 10 (24^3 cells 98 / 90 -> 73 / 62 us).  The sums round differently from those of the other sweep kernels (their
 // error against a wider type is no larger); the server, whose kernels give the
 // same bits, does not split.
 __host__ __device__ constexpr int strip_lpr(int b, int elem, int ne, bool split) {
   return split ? b * b : elem == 8 || (b == 3 && ne > 7) ? b : 1;
 }
-constexpr bool strip_can_split(int b, int elem) { return b == 2 && elem == 8; }
+constexpr bool strip_can_split(int b, int elem) { return b >= 2 && elem == 8; }
+// row of a step that lane t of the strip's 32 Q works on (RW: none)
+__host__ __device__ constexpr int strip_row(const StripDims& d, int t) {
+  const int per = 32 / d.LPR, l = t % 32 / d.LPR;
+  return l < per ? t / 32 * per + l : d.RW;
+}
 __host__ __device__ constexpr StripDims strip_dims(int b, int elem, bool forward, int ne, bool split) {
   StripDims d{};
   d.split = split;
   d.LPR = strip_lpr(b, elem, ne, split);
-  d.RW = 32 / d.LPR;
+  d.Q = split && b == 3 ? 4 : 1;
+  d.RW = 32 / d.LPR * d.Q;
   d.MC = ((ne + 1) / 2 + 2 + 3) / 4;
   const int per_lane = (ne + (forward ? 1 : 0)) * (b * b / d.LPR);
   d.VC = (per_lane * elem + 15) / 16;
   d.VS = (b == 3 ? 4 : b) * elem;
-  d.step_bytes = 512 * (d.MC + d.VC);
+  d.step_bytes = 512 * d.Q * (d.MC + d.VC);
   d.rhs_bytes = d.RW * b * elem;
   d.CH = d.step_bytes <= 2560 ? 8 : d.step_bytes <= 6144 ? 4 : 2;
   // short steps share a test (it is a branch, about 10 cycles, and waiting for

@@ -235,17 +235,17 @@ bool strip_plan(int n, int b, int elem, const int* rowptr, const int* colind, co
 }
 
 std::vector<int> strip_meta(const StripPlan& P, const int* out_pos, int W, int NS) {
-  const int RW = P.d.RW, LPR = P.d.LPR, MC = P.d.MC, ne = P.ne;
+  const int RW = P.d.RW, MC = P.d.MC, ne = P.ne, lanes = 32 * P.d.Q;
   const size_t nsteps = (size_t)P.steps();
-  std::vector<int> m(nsteps * MC * 128, 0);
+  std::vector<int> m(nsteps * MC * lanes * 4, 0);
   const int iout = (ne + 1) / 2;
   int strip = 0;
   for (size_t s = 0; s < nsteps; ++s) {
     while ((long long)P.strip_chunk[strip + 1] * P.d.CH <= (long long)s) ++strip;
     const unsigned region = (unsigned)strip_region_offset(P.d, W, NS, strip % W);
-    for (int lane = 0; lane < 32; ++lane) {
-      auto put = [&](int i) -> int& { return m[((s * MC + i / 4) * 32 + lane) * 4 + (i & 3)]; };
-      const int l = lane / LPR;
+    for (int lane = 0; lane < lanes; ++lane) {
+      auto put = [&](int i) -> int& { return m[((s * MC + i / 4) * lanes + lane) * 4 + (i & 3)]; };
+      const int l = strip_row(P.d, lane);
       const size_t at = s * RW + l;
       const int row = l < RW ? P.step_rows[at] : -1;
       put(iout) = row >= 0 ? out_pos[row] : -1;

@@ -21,7 +21,7 @@ extern "C" int emul_strip(int n, int b, int elem, const int* rowptr, const int* 
   StripPlan P;
   if (!strip_plan(n, b, elem, rowptr, colind, diaind.data(), forward != 0, split != 0, P)) return -1;
   const StripDims& d = P.d;
-  const int W = 3, NS = 2;
+  const int W = d.Q > 1 ? 1 : 3, NS = 2, lanes = 32 * d.Q;
   const int M = strip_mailbox(d.VS), ne = P.ne, iout = (ne + 1) / 2;
   if (d.CH * 4 > kStripHdr || strip_smem_bytes(d, W, NS) / 4 > 65536) return 1;
   if (d.chunk_bytes % 16 || d.CH * d.rhs_bytes % 16) return 2;
@@ -49,12 +49,12 @@ extern "C" int emul_strip(int n, int b, int elem, const int* rowptr, const int* 
       deliver(eager ? cnt : P.need[s0 + s]);
       if (P.need[s0 + s] > delivered) return 3;  // would wait for ever
       std::vector<int> done_rows(d.RW, -1);
-      for (int lane = 0; lane < 32; ++lane) {
-        auto get = [&](int i) { return meta[(((size_t)(s0 + s) * d.MC + i / 4) * 32 + lane) * 4 + (i & 3)]; };
-        const int row = get(iout), l = lane / d.LPR;
+      for (int lane = 0; lane < lanes; ++lane) {
+        auto get = [&](int i) { return meta[(((size_t)(s0 + s) * d.MC + i / 4) * lanes + lane) * 4 + (i & 3)]; };
+        const int row = get(iout), l = strip_row(d, lane);
         if (row < 0) continue;
         if (l >= d.RW || P.pos[row] != (s0 + s) * d.RW + l) return 4;
-        if (lane % d.LPR == 0 && seen[row]++) return 5;
+        if (lane % 32 % d.LPR == 0 && seen[row]++) return 5;
         const int c0 = forward ? rowptr[row] : diaind[row], c1 = forward ? diaind[row] : rowptr[row + 1];
         for (int e = 0; e < ne; ++e) {
           const int cd = (int)((unsigned)get(e / 2) >> (16 * (e & 1)) & 0xffffu);

@@ -3,7 +3,7 @@ where their plan can go wrong: one line and one line more than a strip, more
 items than a mailbox has slots, more strips than the device has CTAs, and every
 entry class.  A row is evaluated in the one-CTA kernel's order, so both kinds
 give the same bits, in FP64 and (through a few FP32-factor iterations) in FP32;
-the FP64 preconditioner also meets the oracle's to 1e-12.  2x2 blocks in FP64 are
+the FP64 preconditioner also meets the oracle's to 1e-12.  2x2 and 3x3 blocks in FP64 are
 summed by columns: there FP64 agrees to rounding (1e-12 through the oracle, a few
 iterations to 1e-10), and the error against sums in a wider type is the one-CTA kernel's,
 but for the one rounding more of a row's two halves (its 6 operations or more
@@ -63,7 +63,7 @@ def test_strip_sweeps(gpu_ctx, oracle_lib, name, fill):
             got[mode] = (z, x32, s.solution())
         finally:
             s.close()
-    if b == 2:
+    if b > 1:
         (z, x32, x64), (z3, y32, y64) = got[1], got[3]
         assert np.array_equal(x32, y32)
         assert np.linalg.norm(x64 - y64) <= 1e-10 * np.linalg.norm(y64)
@@ -74,7 +74,7 @@ def test_strip_sweeps(gpu_ctx, oracle_lib, name, fill):
 
 
 def _substitute_wide(rp, ci, fd, fo, rhs):
-    n, z = fd.shape[0], rhs.reshape(-1, 2).astype(np.longdouble)
+    n, z = fd.shape[0], rhs.reshape(fd.shape[0], -1).astype(np.longdouble)
     for i in range(n):  # L y = r, D^-1 applied
         for c in range(rp[i], rp[i + 1]):
             if ci[c] < i:
@@ -87,7 +87,8 @@ def _substitute_wide(rp, ci, fd, fo, rhs):
     return z
 
 
-@pytest.mark.parametrize("name,fill", [("solid2d:45x38", 0), ("solid2d:30x21", 1)])
+@pytest.mark.parametrize("name,fill", [("solid2d:45x38", 0), ("solid2d:30x21", 1), ("solid3d:13x10x8", 0),
+                                       ("solid3d:5x6x4", 1)])
 def test_split_strips_are_as_exact(gpu_ctx, name, fill):
     if np.finfo(np.longdouble).nmant <= 52:
         pytest.skip("no wider type than FP64 here")
@@ -100,15 +101,15 @@ def test_split_strips_are_as_exact(gpu_ctx, name, fill):
             s.assemble()
             assert s.factor()
             rp, ci = s.prec.GetPattern()
-            fd, fo = (np.asarray(v).reshape(-1, 2, 2) for v in s.prec.GetFactor())
+            fd, fo = (np.asarray(v).reshape(-1, p.b, p.b) for v in s.prec.GetFactor())
             s.ls.ReSizeTmpVecSolver(1)
             err[mode] = 0.0
             for seed in range(3):
-                rhs = np.random.default_rng(seed).standard_normal(p.nnode * 2)
+                rhs = np.random.default_rng(seed).standard_normal(p.nnode * p.b)
                 s.ls.SetVector(0, rhs)
                 s.prec.SolvePrecond(s.ls, 0)
                 ref = _substitute_wide(rp, ci, fd, fo, rhs)
-                err[mode] += float(np.linalg.norm(s.ls.GetVector(0).reshape(-1, 2) - ref) / np.linalg.norm(ref))
+                err[mode] += float(np.linalg.norm(s.ls.GetVector(0).reshape(ref.shape) - ref) / np.linalg.norm(ref))
         finally:
             s.close()
     print("error against sums in a wider type: by columns %.3g, in order %.3g" % (err[1] / 3, err[3] / 3))
