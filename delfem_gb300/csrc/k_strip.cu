@@ -1,7 +1,7 @@
 // k_strip.cu -- forward / backward substitution of the block ILU factor
 // (CMatDiaFrac_BlkCrs::ForwardSubstitution / BackwardSubstitution,
 // src/matvec/matdiafrac_blkcrs.cpp:332-669) in the reference's natural order,
-// one warp per strip of rows.
+// one warp per strip of rows (3x3 FP64: four).
 //
 // What bounds a sweep is its chain of dependency levels, so the kernel is
 // built around the time from one level to the next.  A strip (strip.cpp) holds
