@@ -59,21 +59,58 @@ __device__ double block_sum(double v) {
 // This block's chunks (blockIdx.x, + gridDim.x, ...) with their slot index,
 // the next chunk's index loaded one chunk ahead so that only the slot's
 // fields and state stand between a chunk and its data.
+//
+// CUT: where the chunks would leave most of the grid without work (cut_shift),
+// each is cut into 2^sh runs of rows, a block each (a loop of its own: cut and
+// uncut chunks in one loop spill at 40 registers).  With 2,048 rows a block, the
+// last few solves of a stream keep a few dozen SMs busy, each for eight rows
+// per thread one after the other: on 24 requests of 2k-40k nodes the product
+// took 59 us per launch, the r/x update 30; cut 26 and 20, the
+// whole stream 139 -> 115 ms.
+template <bool CUT = false>
 struct ChunkWalk {
   const unsigned char* map;
-  int nch, c, si_next;
-  __device__ explicit ChunkWalk(const SrvTable* T) : map(T->chunk_slot), nch(T->total_chunks), c(blockIdx.x) {
-    si_next = c < nch ? __ldg(map + c) : 0;
+  int units, u, si_next;
+  int sh_, sub_ = 0;
+  __device__ explicit ChunkWalk(const SrvTable* T, int shift = 0) : map(T->chunk_slot), u(blockIdx.x), sh_(shift) {
+    units = T->total_chunks << sh();
+    si_next = u < units ? __ldg(map + (u >> sh())) : 0;
   }
-  __device__ bool next(int& cc, int& si) {
-    if (c >= nch) return false;
-    cc = c;
+  __device__ int sh() const { return CUT ? sh_ : 0; }
+  __device__ int sub() const { return CUT ? sub_ : 0; }
+  __device__ bool next(int& c, int& si) {
+    if (u >= units) return false;
+    c = u >> sh();
+    if (CUT) sub_ = u & ((1 << sh()) - 1);
     si = si_next;
-    c += gridDim.x;
-    si_next = c < nch ? __ldg(map + c) : 0;
+    u += gridDim.x;
+    si_next = u < units ? __ldg(map + (u >> sh())) : 0;
     return true;
   }
 };
+__device__ __forceinline__ int cut_shift(const SrvTable* T) {
+  const int nch = T->total_chunks;
+  return nch > kSrvMaxCut ? 0 : nch * 8 <= (int)gridDim.x ? 3 : nch * 4 <= (int)gridDim.x ? 2 : 0;
+}
+
+// A chunk's runs done: true (block-uniform) in the last of its blocks, which
+// then takes the chunk's sum from memory, in the order of an uncut chunk.
+__device__ __noinline__ bool chunk_last(double* partials, int c, int sh) {
+  if (sh == 0) return true;
+  __shared__ bool last;
+  unsigned* cnt = reinterpret_cast<unsigned*>(partials + kSrvMaxChunks) + c;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(cnt, 1u) == (1u << sh) - 1;
+    if (last) {
+      *cnt = 0u;
+      __threadfence();
+    }
+  }
+  __syncthreads();
+  return last;
+}
 
 // Publishes this chunk's partial; true (block-uniform) in the slot's last
 // arriving block, which then holds the slot total in *tot.
@@ -136,11 +173,12 @@ __device__ __forceinline__ void put_sweep_input(const SrvSlot& S, long long k, d
   }
 }
 
-// The share of chunk c in the sentinel fill of the slot's exchange buffers.
-template <typename Z>
-__device__ __forceinline__ void fill_xch(const SrvSlot& S, int c) {
-  const long long k = c - S.chunk0, e1 = S.nx * (k + 1) / S.nchunks;
-  for (long long e = S.nx * k / S.nchunks + threadIdx.x; e < e1; e += kSrvTpb)
+// The share of chunk c's run in the sentinel fill of the slot's exchange buffers.
+template <typename Z, typename W>
+__device__ __forceinline__ void fill_xch(const SrvSlot& S, int c, const W& w) {
+  const long long k = ((long long)(c - S.chunk0) << w.sh()) + w.sub(), n = (long long)S.nchunks << w.sh();
+  const long long e1 = S.nx * (k + 1) / n;
+  for (long long e = S.nx * k / n + threadIdx.x; e < e1; e += kSrvTpb)
     reinterpret_cast<Z*>(S.xch)[e] = sentinel_value<Z>();
 }
 
@@ -150,6 +188,44 @@ __device__ __forceinline__ void chunk_elems(const SrvSlot& S, int c, long long& 
   const long long row1 = min(row0 + kSrvRows, (long long)S.n);
   e0 = row0 * S.b;
   e1 = row1 * S.b;
+}
+
+// rows and elements of the walk's run of chunk c
+template <typename W>
+__device__ __forceinline__ void run_rows(const SrvSlot& S, int c, const W& w, int& row0, int& row1) {
+  const int len = kSrvRows >> w.sh();
+  row0 = (c - S.chunk0) * kSrvRows + w.sub() * len;
+  row1 = min(row0 + len, S.n);
+}
+template <typename W>
+__device__ __forceinline__ void run_elems(const SrvSlot& S, int c, const W& w, long long& e0, long long& e1) {
+  int row0, row1;
+  run_rows(S, c, w, row0, row1);
+  e0 = (long long)row0 * S.b;
+  e1 = (long long)row1 * S.b;
+}
+
+// p.q over rows [row0, row1) as chunk_q_pap adds it up
+template <typename V>
+__device__ __noinline__ double chunk_pap(const SrvSlot& S, const V* p, const V* q, int c) {
+  const int b = S.b, row0 = (c - S.chunk0) * kSrvRows, row1 = min(row0 + kSrvRows, S.n);
+  double part = 0.0;
+  for (int i = row0 + threadIdx.x; i < row1; i += kSrvTpb)
+    for (int d = 0; d < b; ++d) part += (double)p[(size_t)i * b + d] * (double)__ldcg(q + (size_t)i * b + d);
+  return part;
+}
+// r.r over elements [e0, e1) as the r/x updates add it up
+template <typename V>
+__device__ __noinline__ double chunk_rr(const SrvSlot& S, const V* r, int c) {
+  long long e0, e1;
+  chunk_elems(S, c, e0, e1);
+  double part = 0.0;
+#pragma unroll 4
+  for (long long k = e0 + threadIdx.x; k < e1; k += kSrvTpb) {
+    const double v = (double)__ldcg(r + k);
+    part += v * v;
+  }
+  return part;
 }
 
 // q = A p over rows [row0, row1) of one chunk (thread per row, sliced ELL);
@@ -196,7 +272,7 @@ template <typename Z>
 __global__ void __launch_bounds__(kSrvTpb, kSrvVecBlocks) k_srv_rz_beta(const SrvTable* T, double* partials, int* tickets,
                                                          int ntickets) {
   if (blockIdx.x == 0 && threadIdx.x < ntickets) tickets[threadIdx.x] = 0;
-  ChunkWalk w(T);
+  ChunkWalk<> w(T);
   for (int c, si; w.next(c, si);) {
     const SrvSlot S = T->slot[si];
     if (ld_relaxed_int(&S.st->done) != 0) continue;
@@ -221,34 +297,48 @@ __global__ void __launch_bounds__(kSrvTpb) k_srv_fin_rz_beta(const SrvTable* T, 
 }
 
 // p := z in the first iteration, else p := beta p + z (SCAL + AXPY)
-template <typename Z>
-__global__ void __launch_bounds__(kSrvTpb, kSrvVecBlocks) k_srv_update_p(const SrvTable* T) {
-  ChunkWalk w(T);
+template <typename Z, bool CUT>
+__device__ __forceinline__ void srv_update_p_chunks(const SrvTable* T, int shift) {
+  ChunkWalk<CUT> w(T, shift);
   for (int c, si; w.next(c, si);) {
     const SrvSlot S = T->slot[si];
     if (ld_relaxed_int(&S.st->done) != 0) continue;
     long long e0, e1;
-    chunk_elems(S, c, e0, e1);
+    run_elems(S, c, w, e0, e1);
     const bool first = S.st->it == 0;
     const double beta = S.st->beta;
-    #pragma unroll 4
+#pragma unroll (CUT ? 1 : 4)
     for (long long k = e0 + threadIdx.x; k < e1; k += kSrvTpb)
       S.p[k] = first ? zval<Z>(S.z, k) : __dadd_rn(__dmul_rn(S.p[k], beta), zval<Z>(S.z, k));
   }
 }
+template <typename Z>
+__global__ void __launch_bounds__(kSrvTpb, kSrvVecBlocks) k_srv_update_p(const SrvTable* T) {
+  const int shift = cut_shift(T);
+  if (shift) srv_update_p_chunks<Z, true>(T, shift);
+  else srv_update_p_chunks<Z, false>(T, 0);
+}
 
 // q = A p; pAp; alpha = rz / pAp
-__global__ void __launch_bounds__(kSrvTpb, kSrvVecBlocks) k_srv_spmv_pap(const SrvTable* T, double* partials) {
-  ChunkWalk w(T);
+template <bool CUT>
+__device__ __forceinline__ void srv_spmv_pap_chunks(const SrvTable* T, double* partials, int shift) {
+  ChunkWalk<CUT> w(T, shift);
   for (int c, si; w.next(c, si);) {
     const SrvSlot S = T->slot[si];
     if (ld_relaxed_int(&S.st->done) != 0) continue;
     int row0, row1;
-    chunk_rows(S, c, row0, row1);
-    const double part = S.b == 1 ? chunk_q_pap<1>(S, row0, row1)
+    run_rows(S, c, w, row0, row1);
+    double part = S.b == 1 ? chunk_q_pap<1>(S, row0, row1)
                         : S.b == 2 ? chunk_q_pap<2>(S, row0, row1) : chunk_q_pap<3>(S, row0, row1);
+    if (!chunk_last(partials, c, w.sh())) continue;
+    if (CUT) part = chunk_pap(T->slot[si], T->slot[si].p, T->slot[si].q, c);
     publish(part, c, partials);
   }
+}
+__global__ void __launch_bounds__(kSrvTpb, kSrvVecBlocks) k_srv_spmv_pap(const SrvTable* T, double* partials) {
+  const int shift = cut_shift(T);
+  if (shift) srv_spmv_pap_chunks<true>(T, partials, shift);
+  else srv_spmv_pap_chunks<false>(T, partials, 0);
 }
 
 __global__ void __launch_bounds__(kSrvTpb) k_srv_fin_pap(const SrvTable* T, const double* partials) {
@@ -263,17 +353,17 @@ __global__ void __launch_bounds__(kSrvTpb) k_srv_fin_pap(const SrvTable* T, cons
 
 // r := r - alpha q; x := x + alpha p; rr = r.r; stop test; sweep outputs back
 // to the sentinel; FP32 copy of r for FP32 sweeps
-template <typename Z>
-__global__ void __launch_bounds__(kSrvTpb, kSrvVecBlocks) k_srv_update_rx(const SrvTable* T, double* partials) {
-  ChunkWalk w(T);
+template <typename Z, bool CUT>
+__device__ __forceinline__ void srv_update_rx_chunks(const SrvTable* T, double* partials, int shift) {
+  ChunkWalk<CUT> w(T, shift);
   for (int c, si; w.next(c, si);) {
     const SrvSlot S = T->slot[si];
     if (ld_relaxed_int(&S.st->done) != 0) continue;
     long long e0, e1;
-    chunk_elems(S, c, e0, e1);
+    run_elems(S, c, w, e0, e1);
     const double alpha = S.st->alpha;
     double part = 0.0;
-    #pragma unroll 4
+#pragma unroll (CUT ? 1 : 4)
     for (long long k = e0 + threadIdx.x; k < e1; k += kSrvTpb) {
       double r = S.r[k];
       if (alpha != 0.0) {
@@ -288,9 +378,17 @@ __global__ void __launch_bounds__(kSrvTpb, kSrvVecBlocks) k_srv_update_rx(const 
       }
       put_sweep_input<Z>(S, k, r);
     }
-    fill_xch<Z>(T->slot[si], c);
+    fill_xch<Z>(T->slot[si], c, w);
+    if (!chunk_last(partials, c, w.sh())) continue;
+    if (CUT) part = chunk_rr(T->slot[si], T->slot[si].r, c);
     publish(part, c, partials);
   }
+}
+template <typename Z>
+__global__ void __launch_bounds__(kSrvTpb, kSrvVecBlocks) k_srv_update_rx(const SrvTable* T, double* partials) {
+  const int shift = cut_shift(T);
+  if (shift) srv_update_rx_chunks<Z, true>(T, partials, shift);
+  else srv_update_rx_chunks<Z, false>(T, partials, 0);
 }
 
 __global__ void __launch_bounds__(kSrvTpb) k_srv_fin_rx(const SrvTable* T, const double* partials) {
@@ -324,7 +422,7 @@ constexpr int kMaxReplace = 8;
 // ||rd||^2 <= tol^2 ||b||^2, else marked for residual replacement (done = 6),
 // or given up (done = 7) after kMaxReplace replacements
 __global__ void __launch_bounds__(kSrvTpb) k_srv_check_true(const SrvTable* T, double* partials) {
-  ChunkWalk w(T);
+  ChunkWalk<> w(T);
   for (int c, si; w.next(c, si);) {
     const SrvSlot S = T->slot[si];
     if (ld_relaxed_int(&S.st->done) != 1 || ld_relaxed_int(&S.st->verified) != 0) continue;
@@ -345,7 +443,7 @@ __global__ void __launch_bounds__(kSrvTpb) k_srv_check_true(const SrvTable* T, d
 // done == 6: r := rd and the recursion continues (residual replacement)
 template <typename Z>
 __global__ void __launch_bounds__(kSrvTpb, kSrvVecBlocks) k_srv_replace(const SrvTable* T, double* partials) {
-  ChunkWalk w(T);
+  ChunkWalk<> w(T);
   for (int c, si; w.next(c, si);) {
     const SrvSlot S = T->slot[si];
     if (ld_relaxed_int(&S.st->done) != 6) continue;
@@ -413,7 +511,7 @@ __device__ __forceinline__ bool mixed_live(const PcgState* st) { return ld_relax
 __global__ void __launch_bounds__(kSrvTpb, kSrvVecBlocks) k_srvm_rz_beta(const SrvTable* T, double* partials, int* tickets,
                                                           int ntickets) {
   if (blockIdx.x == 0 && threadIdx.x < ntickets) tickets[threadIdx.x] = 0;
-  ChunkWalk w(T);
+  ChunkWalk<> w(T);
   for (int c, si; w.next(c, si);) {
     const SrvSlot S = T->slot[si];
     if (!mixed_live(S.st)) continue;
@@ -433,19 +531,25 @@ __global__ void __launch_bounds__(kSrvTpb, kSrvVecBlocks) k_srvm_rz_beta(const S
 }
 
 // p := z in the first iteration, else p := z + beta p (FP32)
-__global__ void __launch_bounds__(kSrvTpb, kSrvVecBlocks) k_srvm_update_p(const SrvTable* T) {
-  ChunkWalk w(T);
+template <bool CUT>
+__device__ __forceinline__ void srvm_update_p_chunks(const SrvTable* T, int shift) {
+  ChunkWalk<CUT> w(T, shift);
   for (int c, si; w.next(c, si);) {
     const SrvSlot S = T->slot[si];
     if (!mixed_live(S.st)) continue;
     long long e0, e1;
-    chunk_elems(S, c, e0, e1);
+    run_elems(S, c, w, e0, e1);
     const bool first = S.st->it == 0;
     const float beta = (float)S.st->beta;
     const float* z = reinterpret_cast<const float*>(S.z);
-    #pragma unroll 4
+#pragma unroll (CUT ? 1 : 4)
     for (long long k = e0 + threadIdx.x; k < e1; k += kSrvTpb) S.p32[k] = first ? z[k] : z[k] + beta * S.p32[k];
   }
+}
+__global__ void __launch_bounds__(kSrvTpb, kSrvVecBlocks) k_srvm_update_p(const SrvTable* T) {
+  const int shift = cut_shift(T);
+  if (shift) srvm_update_p_chunks<true>(T, shift);
+  else srvm_update_p_chunks<false>(T, 0);
 }
 
 // q = A p on the FP32 values with FP32 accumulation; pAp in FP64; alpha
@@ -464,15 +568,18 @@ __device__ __forceinline__ double chunk_q_pap32(const SrvSlot& S, int row0, int 
   return part;
 }
 
-__global__ void __launch_bounds__(kSrvTpb) k_srvm_spmv_pap(const SrvTable* T, double* partials) {
-  ChunkWalk w(T);
+template <bool CUT>
+__device__ __forceinline__ void srvm_spmv_pap_chunks(const SrvTable* T, double* partials, int shift) {
+  ChunkWalk<CUT> w(T, shift);
   for (int c, si; w.next(c, si);) {
     const SrvSlot S = T->slot[si];
     if (!mixed_live(S.st)) continue;
     int row0, row1;
-    chunk_rows(S, c, row0, row1);
-    const double part = S.b == 1 ? chunk_q_pap32<1>(S, row0, row1)
+    run_rows(S, c, w, row0, row1);
+    double part = S.b == 1 ? chunk_q_pap32<1>(S, row0, row1)
                         : S.b == 2 ? chunk_q_pap32<2>(S, row0, row1) : chunk_q_pap32<3>(S, row0, row1);
+    if (!chunk_last(partials, c, w.sh())) continue;
+    if (CUT) part = chunk_pap(T->slot[si], T->slot[si].p32, T->slot[si].q32, c);
     double tot;
     if (slot_sum(part, c, S, partials, &tot) && threadIdx.x == 0) {
       S.st->pap = tot;
@@ -480,24 +587,30 @@ __global__ void __launch_bounds__(kSrvTpb) k_srvm_spmv_pap(const SrvTable* T, do
     }
   }
 }
+__global__ void __launch_bounds__(kSrvTpb) k_srvm_spmv_pap(const SrvTable* T, double* partials) {
+  const int shift = cut_shift(T);
+  if (shift) srvm_spmv_pap_chunks<true>(T, partials, shift);
+  else srvm_spmv_pap_chunks<false>(T, partials, 0);
+}
 
 // r := r - alpha q (FP32); d := d + alpha p (FP64); rr = r.r (FP64); the
 // recursive stop (done 5: the true residual decides at the end of the replay),
 // the reliable-update trigger, the iteration limit; sweep outputs back to the
 // sentinel
-__global__ void __launch_bounds__(kSrvTpb, kSrvVecBlocks) k_srvm_update_rx(const SrvTable* T, double* partials) {
-  ChunkWalk w(T);
+template <bool CUT>
+__device__ __forceinline__ void srvm_update_rx_chunks(const SrvTable* T, double* partials, int shift) {
+  ChunkWalk<CUT> w(T, shift);
   for (int c, si; w.next(c, si);) {
     const SrvSlot S = T->slot[si];
     if (!mixed_live(S.st)) continue;
     long long e0, e1;
-    chunk_elems(S, c, e0, e1);
+    run_elems(S, c, w, e0, e1);
     const double alpha = S.st->alpha;
     const float alpha32 = (float)alpha;
     float* y = reinterpret_cast<float*>(S.y);
     float* z = reinterpret_cast<float*>(S.z);
     double part = 0.0;
-    #pragma unroll 4
+#pragma unroll (CUT ? 1 : 4)
     for (long long k = e0 + threadIdx.x; k < e1; k += kSrvTpb) {
       float r = S.r32[k];
       if (alpha != 0.0) {
@@ -512,7 +625,9 @@ __global__ void __launch_bounds__(kSrvTpb, kSrvVecBlocks) k_srvm_update_rx(const
         z[k] = sentinel_value<float>();
       }
     }
-    fill_xch<float>(S, c);
+    fill_xch<float>(T->slot[si], c, w);
+    if (!chunk_last(partials, c, w.sh())) continue;
+    if (CUT) part = chunk_rr(T->slot[si], T->slot[si].r32, c);
     double tot;
     if (slot_sum(part, c, S, partials, &tot) && threadIdx.x == 0) {
       PcgState* st = S.st;
@@ -534,6 +649,11 @@ __global__ void __launch_bounds__(kSrvTpb, kSrvVecBlocks) k_srvm_update_rx(const
     }
   }
 }
+__global__ void __launch_bounds__(kSrvTpb, kSrvVecBlocks) k_srvm_update_rx(const SrvTable* T, double* partials) {
+  const int shift = cut_shift(T);
+  if (shift) srvm_update_rx_chunks<true>(T, partials, shift);
+  else srvm_update_rx_chunks<false>(T, partials, 0);
+}
 
 __device__ __forceinline__ bool mixed_due(const PcgState* st) {
   const int dn = ld_relaxed_int(&st->done);
@@ -543,7 +663,7 @@ __device__ __forceinline__ bool mixed_due(const PcgState* st) {
 // x := x + d, d := 0 for slots due for a reliable update, stopped, or at
 // the end (limit, NaN)
 __global__ void __launch_bounds__(kSrvTpb, kSrvVecBlocks) k_srvm_fold(const SrvTable* T) {
-  ChunkWalk w(T);
+  ChunkWalk<> w(T);
   for (int c, si; w.next(c, si);) {
     const SrvSlot S = T->slot[si];
     const int dn = ld_relaxed_int(&S.st->done);
@@ -578,7 +698,7 @@ __device__ __forceinline__ double chunk_refine(const SrvSlot& S, int row0, int r
 }
 
 __global__ void __launch_bounds__(kSrvTpb) k_srvm_refine(const SrvTable* T, double* partials) {
-  ChunkWalk w(T);
+  ChunkWalk<> w(T);
   for (int c, si; w.next(c, si);) {
     const SrvSlot S = T->slot[si];
     if (!mixed_due(S.st)) continue;

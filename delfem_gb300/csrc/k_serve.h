@@ -10,6 +10,8 @@ namespace dfg {
 constexpr int kSrvRows = 2048;      // block rows per chunk
 constexpr int kSrvMaxSlots = 256;   // in-flight solves per server
 constexpr int kSrvTpb = 256;        // threads per block of the batched kernels
+constexpr int kSrvMaxChunks = 1 << 20;  // chunk space of one launch
+constexpr int kSrvMaxCut = 1024;        // chunks that a launch cuts into runs, at most (a quarter of its grid)
 
 // One in-flight solve.  Its rows are cut into chunks of kSrvRows; chunk k of
 // the slot is chunk chunk0 + k of the launch's chunk space.  Reductions sum a
@@ -71,6 +73,7 @@ struct SrvStatus {
 
 // fp32z: sweep outputs y, z are float (FP32 factor); tickets: the batched
 // sweep launches' counters, reset once the sweeps of an iteration are over.
+// partials: kSrvMaxChunks doubles, then kSrvMaxCut counters, zero between launches.
 // srv_rz_beta, srv_spmv_pap and srv_update_rx are two launches each: the
 // batched kernel, then one block per slot for the slot's reduction.
 cudaError_t srv_rz_beta(const SrvTable* T, double* partials, int* tickets, int ntickets, bool fp32z, int grid,

@@ -57,7 +57,7 @@ constexpr int kClasses = 9;         // block size 1..3 x dependency entries <= 4
 constexpr int kStripNe[] = {3, 4, 7, 16};
 constexpr int kStripClasses = 12;   // block size 1..3 x entry class of the strip sweeps
 constexpr int kStripBit = 2 * kClasses;  // their first bit in Group::graph_mask
-constexpr int kMaxChunks = 1 << 20; // chunk space of one launch (kSrvRows rows each)
+constexpr int kMaxChunks = kSrvMaxChunks;
 constexpr int kRingSteps = 32;
 constexpr int kServeStages = 3;   // sweep pipeline depth in batched launches
 // mixed form: a reliable update falls due once the recursive residual norm
@@ -228,7 +228,7 @@ struct Group {
   StripBatch* d_strip = nullptr;   // kStripClasses x 2: strip sweeps
   StripBatch* h_strip = nullptr;
   int* d_tickets = nullptr;        // kClasses x 2 ranged, kClasses x 2 solo, kStripClasses x 2 strips
-  double* d_partials = nullptr;    // kMaxChunks
+  double* d_partials = nullptr;    // kMaxChunks, then kSrvMaxCut counters
   unsigned char* d_chunk_slot = nullptr;  // kMaxChunks: each chunk's slot
   unsigned char* h_chunk_slot = nullptr;
   unsigned char* d_stat = nullptr; // SrvStatus[kSrvMaxSlots] then the error word
@@ -1536,7 +1536,8 @@ extern "C" int dfg_server_create(dfg_ctx ctx, const dfg_server_config* cfg, dfg_
       SCK(cudaMalloc(&G.d_solo, sizeof(SoloBatch) * kClasses * 2));
       SCK(cudaMalloc(&G.d_strip, sizeof(StripBatch) * kStripClasses * 2));
       SCK(cudaMalloc(&G.d_tickets, sizeof(int) * kTickets));
-      SCK(cudaMalloc(&G.d_partials, sizeof(double) * kMaxChunks));
+      SCK(cudaMalloc(&G.d_partials, sizeof(double) * kMaxChunks + sizeof(unsigned) * kSrvMaxCut));
+      SCK(cudaMemset(G.d_partials + kMaxChunks, 0, sizeof(unsigned) * kSrvMaxCut));
       SCK(cudaMalloc(&G.d_chunk_slot, kMaxChunks));
       SCK(cudaHostAlloc(&G.h_chunk_slot, kMaxChunks, cudaHostAllocDefault));
       SCK(cudaMalloc(&G.d_stat, sizeof(SrvStatus) * kSrvMaxSlots + 64));
