@@ -245,7 +245,7 @@ def run_gpu(args, rank, world, local):
     p = make_problem(args.config)
     ctx = L.Context(local)
     s = FESolve(ctx, p, fill_level=args.fill_level, sweep_mode=args.sweep_mode)
-    sched = {1: "ranged", 2: "level-scheduled", 3: "one CTA"}
+    sched = {1: "strips or ranged", 2: "level-scheduled", 3: "one CTA"}
     sweeps = dict(zip(("forward", "backward"), (sched[k] for k in s.prec.GetSweepMode())))
     stream = ctx.stream
 
@@ -740,9 +740,8 @@ def compose_serve_line(args, world, cfg, items, timed_items, timed_probs, result
         achieved = v["bytes"] / (v["ms"] * 1e-3) / 1e9
         roof = {"bound": "hbm", "achieved": round(achieved, 1), "peak": hbm_peak, "unit": "GB/s",
                 "frac": round(achieved / hbm_peak, 4),
-                # FP32 sweeps of the 2D classes run one CTA per solve, FP64 ones ranged
-                "traffic": ncu_traffic(dom + (":one_CTA" if results[head]["mode"] != "fp64" else ":ranged")
-                                       if dom.startswith("sweep") else dom, v["bytes"]),
+                # served sweeps run in strips where the rows fit them
+                "traffic": ncu_traffic(dom + ":strips" if dom.startswith("sweep") else dom, v["bytes"]),
                 "peak_source": peak_kind,
                 "kernel": dom, "ms_per_launch": round(v["ms"], 4), "algorithmic_bytes": int(v["bytes"]),
                 "launches_timed": int(v["n"])}
