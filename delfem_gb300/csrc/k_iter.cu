@@ -30,7 +30,8 @@
 // Measured on GB300, a whole PCG iteration (four launches -> one): Poisson
 // 24x24 54.7 -> 51.1 us, 128x128 148 -> 137, 301x257 FP32 everything 122 -> 114,
 // cantilever 200x100 262 -> 251, 401x199 FP32 factor 153 -> 142, elasticity 24^3
-// 234 -> 216, 56^3 FP32 factor 327 -> 300 (some 3 % of it the sweeps').
+// 234 -> 216, 56^3 FP32 factor 327 -> 300 (some 3 % of it the sweeps'); now, with
+// what is said here and shorter sweeps, 39, 127, 107, 212, 132, 154 and 275.
 //
 // Waits are bounded; one that gives up records kErrTimeout.
 #include <algorithm>

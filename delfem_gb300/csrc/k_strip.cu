@@ -23,11 +23,11 @@
 //     items it needs, one compare when they are there.
 // Measured on GB300, FP32, per sweep (forward / backward): the 1000x500
 // cantilever 0.13 / 0.12 ms (ranged kernel 1.09 / 1.10), Poisson on 301x257
-// cells 47 / 46 us (one CTA per sweep 200 / 196), elasticity on 56^3 cells 81 /
-// 77 us (a launch per level 345 / 306).  FP64: the cantilever 0.59 / 0.48 ms
-// (2.36 / 2.08), Poisson on 128x128 cells 65 / 55 us (133 / 123).  Inside one
+// cells 45 / 45 us (one CTA per sweep 200 / 196), elasticity on 56^3 cells 81 /
+// 77 us (a launch per level 345 / 306).  FP64: the cantilever 0.57 / 0.40 ms
+// (2.36 / 2.08), Poisson on 128x128 cells 64 / 54 us (133 / 123).  Inside one
 // strip a level costs 103 (1x1 blocks) to 490 (3x3, 7 entries) cycles in FP32
-// and 380 to 2,000 in FP64, where each warp-wide FMA takes its scheduler 64; a
+// and 380 to 1,280 in FP64, where each warp-wide FMA takes its scheduler 64; a
 // hand-off between strips costs 1,500 to 3,000, of which the L2 takes 600-900.
 //
 // Strips are claimed in order, W per CTA, through a ticket, so a strip only
