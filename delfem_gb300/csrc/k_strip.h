@@ -130,9 +130,16 @@ __host__ __device__ constexpr size_t strip_region_offset(const StripDims& d, int
 inline size_t strip_smem_bytes(const StripDims& d, int W, int NS) { return strip_stage_offset(d, W, NS, W); }
 // False when the rows do not fit the sweep: more than 16 entries in a row, or
 // more dependencies on other strips within a chunk than the mailbox holds.
-// split: only where strip_can_split.
+// split: only where strip_can_split.  min_ne: an entry class that is not gone
+// below (0, or one of strip_class's).
 bool strip_plan(int n, int b, int elem, const int* rowptr, const int* colind, const int* diaind, bool forward,
-                bool split, StripPlan& P);
+                bool split, StripPlan& P, int min_ne = 0);
+// Both directions ([0] forward) in one entry class, that of the widest row of
+// either.  By itself a direction takes the class of its own widest row, and in
+// meshes whose numbering is not a grid's the two differ (a triangle grid with its
+// boundary nodes numbered first: 7 lower entries, 3 upper ones).
+bool strip_plan_both(int n, int b, int elem, const int* rowptr, const int* colind, const int* diaind, bool split,
+                     StripPlan (&P)[2]);
 // Metadata of every step and lane as the records hold it ([step][piece][lane]
 // of 4 ints): ne 16-bit codes (offset / 4 from the start of the CTA's dynamic
 // shared memory, for W warps of NS stages each), then the output position (-1:

@@ -172,7 +172,7 @@ struct Req {
   std::vector<unsigned char> hf, hb;
   std::vector<long long> of, ob;
   long long maxrf = 0, maxrb = 0;
-  int cls = -1, maxe = 0, group = 0;
+  int cls = -1, scls = -1, maxe = 0, group = 0;  // class of its sweeps, strip class (both directions)
   bool solo = false;  // sweeps by one CTA per solve (k_solo.cu), else ranged (k_sweep.cu)
   // solo: chunk tables, first chunk per level, and the forward plan's
   // position of every row (where the forward input is stored)
@@ -362,11 +362,19 @@ bool use_solo(const dfg_server_s* S, const Req* r) {
 constexpr int kServeStripWarps = 1;  // strips per CTA
 bool use_strips(const dfg_server_s* S, Req* r, int elem) {
   if (S->sweeps != 0) return false;
-  for (int dir = 0; dir < 2; ++dir)
-    if (!strip_plan(r->n, r->b, elem, r->rowptr.data(), r->colind.data(), r->diaind.data(), dir == 0, false, r->strip[dir]) ||
-        S->strip_ns[strip_class_index(r->b, r->strip[dir].ne)][dir] == 0)
-      return false;
-  return true;
+  // one class for both directions: a class's forward launch stands before its
+  // backward launch on the class's stream, and nothing else orders a request's
+  // backward sweep after the forward sweep that writes its input
+  if (strip_plan_both(r->n, r->b, elem, r->rowptr.data(), r->colind.data(), r->diaind.data(), false, r->strip)) {
+    const int k = strip_class_index(r->b, r->strip[0].ne);
+    if (S->strip_ns[k][0] > 0 && S->strip_ns[k][1] > 0) {
+      r->scls = k;
+      r->cls = strip_host_class(k);
+      return true;
+    }
+  }
+  for (StripPlan& P : r->strip) P = StripPlan{};
+  return false;
 }
 
 // Fills the request's host-side set-up; returns false with r->error on failure.
@@ -408,8 +416,8 @@ bool symbolic(dfg_server_s* S, Req* r) {
     for (int i = 0; i < n; ++i) ident[i] = i;
     for (int dir = 0; dir < 2; ++dir) {
       StripPlan& P = r->strip[dir];
-      const int k = strip_class_index(r->b, P.ne);
-      r->smeta[dir] = strip_meta(P, dir == 0 ? r->strip[1].pos.data() : ident.data(), kServeStripWarps, S->strip_ns[k][dir]);
+      r->smeta[dir] = strip_meta(P, dir == 0 ? r->strip[1].pos.data() : ident.data(), kServeStripWarps,
+                                 S->strip_ns[r->scls][dir]);
       P.codes = {};
       P.exports = {};
     }
@@ -999,10 +1007,10 @@ int upload_table(dfg_server_s* S, Group& G) {
   for (int i : order) {
     Req* r = act[i];
     const SrvSlot& sl = T->slot[i];
+    const int k = r->scls;
+    mask |= 1 << (kStripBit + k);
     for (int dir = 0; dir < 2; ++dir) {
       const StripPlan& Q = r->strip[dir];
-      const int k = strip_class_index(r->b, Q.ne);
-      mask |= 1 << (kStripBit + k);
       StripBatch& B = G.h_strip[k * 2 + dir];
       const int j = B.nslots++;
       StripSlot& w = B.slot[j];

@@ -136,7 +136,7 @@ bool tile_strips(const Rows& R, int RW, std::vector<int>& strip, std::vector<int
 }  // namespace
 
 bool strip_plan(int n, int b, int elem, const int* rowptr, const int* colind, const int* diaind, bool forward, bool split,
-                StripPlan& P) {
+                StripPlan& P, int min_ne) {
   P = StripPlan{};
   P.forward = forward;
   P.n = n;
@@ -149,6 +149,7 @@ bool strip_plan(int n, int b, int elem, const int* rowptr, const int* colind, co
   for (int i = 0; i < n; ++i) maxe = std::max(maxe, end(i) - first(i));
   P.ne = strip_class(maxe);
   if (n == 0 || P.ne == 0) return false;
+  P.ne = std::max(P.ne, min_ne);
   P.d = strip_dims(b, elem, forward, P.ne, split);
   const int RW = P.d.RW, CH = P.d.CH, ne = P.ne;
 
@@ -231,6 +232,17 @@ bool strip_plan(int n, int b, int elem, const int* rowptr, const int* colind, co
   }
   for (int row = 0; row < n; ++row)
     if (xslot[row] >= 0) P.exports[P.pos[row]] = xslot[row];
+  return true;
+}
+
+bool strip_plan_both(int n, int b, int elem, const int* rowptr, const int* colind, const int* diaind, bool split,
+                     StripPlan (&P)[2]) {
+  int maxe = 0;
+  for (int i = 0; i < n; ++i) maxe = std::max({maxe, diaind[i] - rowptr[i], rowptr[i + 1] - diaind[i]});
+  const int ne = strip_class(maxe);
+  if (ne == 0) return false;
+  for (int dir = 0; dir < 2; ++dir)
+    if (!strip_plan(n, b, elem, rowptr, colind, diaind, dir == 0, split, P[dir], ne)) return false;
   return true;
 }
 
