@@ -147,6 +147,20 @@ bool strip_plan_both(int n, int b, int elem, const int* rowptr, const int* colin
 // result goes.
 std::vector<int> strip_meta(const StripPlan& P, const int* out_pos, int W, int NS);
 
+// A strip's chunk stages.  `consumed` counts the steps of the chunks that its
+// warps are through with; the loader keeps the NS chunks from there on issued.
+// Chunk c of the strip lies in stage c % NS, so a stage is issued again only
+// when its copies have landed and been read.  A strip that has given up
+// publishes nothing more: the chunks from `consumed` on that were issued are then
+// those whose copies may be in flight, and the launch waits for them.
+__host__ __device__ constexpr int strip_publish(bool gave_up, int chunk, int CH) {  // 0: nothing to publish
+  return gave_up ? 0 : (chunk + 1) * CH;
+}
+__host__ __device__ constexpr int strip_issue_end(int consumed, int CH, int NS, int nchunks) {
+  return consumed / CH + NS < nchunks ? consumed / CH + NS : nchunks;
+}
+__host__ __device__ constexpr int strip_drain_begin(int consumed, int CH) { return consumed / CH; }
+
 // One solve's sweep.
 struct StripSlot {
   const unsigned char* rec;  // chunks
