@@ -109,6 +109,8 @@ struct StripPlan {
   std::vector<int> ent_slot;     // nchunks * CH * RW * ne: CRS slot of the block, -1 = padding
   std::vector<int> codes;        // same shape: byte offset into the warp's value region
   std::vector<int> exports;      // nchunks * CH * RW: exchange slot of the row, -1 = none
+  int levels = 0;                // dependency levels of the sweep
+  long long chain = 0;           // its longest chain in steps, a hand-off between strips counted kStripHop
   long long steps() const { return (long long)nchunks * d.CH; }
 };
 __host__ __device__ constexpr size_t strip_up128(size_t v) { return (v + 127) / 128 * 128; }
@@ -128,18 +130,58 @@ __host__ __device__ constexpr size_t strip_region_offset(const StripDims& d, int
   return strip_stage_offset(d, W, NS, w) + strip_stage_bytes(d, NS);
 }
 inline size_t strip_smem_bytes(const StripDims& d, int W, int NS) { return strip_stage_offset(d, W, NS, W); }
-// False when the rows do not fit the sweep: more than 16 entries in a row, or
-// more dependencies on other strips within a chunk than the mailbox holds.
+// Places for rows in the steps, per row.
+inline double strip_fill(const StripPlan& P) { return (double)P.steps() * P.d.RW / P.n; }
+// Whether the strips are those of a grid's numbering: few, or long and full ones
+// (rows for two and a half steps or more in a strip, a row or more in every sixth
+// place) whose chain is at most 10 times the levels'.  Grids row by row have chains
+// of 1.0 to 2.7 times in 2D and up to 5.3 in 3D, with the boundary first or last up
+// to 9.3 in 3D.  Where rows that follow one another lie far apart (numbered by
+// distance from a point, by coordinate, at random, as an unstructured mesher does)
+// strips hold a row or two per step or end after a few steps, and every step
+// waits for other strips.
+constexpr int kStripHop = 15;  // a hand-off between strips in steps (FP32, 1x1)
+constexpr long long kStripChain = 10;
+inline bool strip_like_grid(const StripPlan& P) {
+  return P.nstrips <= 16 || (P.chain <= kStripChain * P.levels && 2LL * P.n >= 5LL * P.nstrips * P.d.RW &&
+                             strip_fill(P) <= 6.0);
+}
+// Whether a plan is worth building at all.  Beside a grid's: records of up to 8 MB,
+// or chains of up to 10 times the levels' with up to 16 places per row.  Beyond,
+// records are tens of times the factor's bytes (an x-sorted Delaunay mesh of 100,000
+// nodes: 76,000 strips, 1.3 GB of FP32 1x1 records for 1.2 MB of factor) and the
+// sweeps slower than the older kinds (3,172 us per iteration, 1,135 with one CTA per
+// sweep).
+inline bool strip_suits(const StripPlan& P) {
+  return strip_like_grid(P) || (size_t)P.nchunks * P.d.chunk_bytes <= (8u << 20) ||
+         (P.chain <= kStripChain * P.levels && strip_fill(P) <= 16.0);
+}
+// Whether a plan that suits also serves a solve among many.  A strip keeps its CTA
+// from its claim to its end, so a solve of many strips that wait for one another
+// keeps the other solves out, whatever its own time.  Measured on GB300, 12 equal
+// requests at once, FP32 factor, the older kinds -> strips: 20,000-node Delaunay
+// meshes of jittered grid points 2D 1x1 (382 strips, rows for 1.6 steps each, fill
+// 27) 87 -> 182 ms, 3D 1x1 (818, 0.8, 20) 154 -> 161; 2D sorted by coordinate
+// (13,000, 0.05, 167) 127 -> 1,965; by reverse Cuthill-McKee (2,808, 0.2, 37) 109 ->
+// 649; but 3D grids with the boundary first (48, 12.8, 2.9) 41 -> 33, and by reverse
+// Cuthill-McKee at 4,000 nodes (143, 0.9, 16) 67 -> 13.
+inline bool strip_serves(const StripPlan& P) {
+  return strip_like_grid(P) || (P.chain <= kStripChain * P.levels &&
+                                (P.nstrips <= 64 || (P.nstrips <= 160 && strip_fill(P) <= 16.0)));
+}
+// False when the rows do not fit the sweep: more than 16 entries in a row, more
+// dependencies on other strips within a chunk than the mailbox holds, or (suited)
+// a plan that does not suit.
 // split: only where strip_can_split.  min_ne: an entry class that is not gone
 // below (0, or one of strip_class's).
 bool strip_plan(int n, int b, int elem, const int* rowptr, const int* colind, const int* diaind, bool forward,
-                bool split, StripPlan& P, int min_ne = 0);
+                bool split, StripPlan& P, int min_ne = 0, bool suited = false);
 // Both directions ([0] forward) in one entry class, that of the widest row of
 // either.  By itself a direction takes the class of its own widest row, and in
 // meshes whose numbering is not a grid's the two differ (a triangle grid with its
 // boundary nodes numbered first: 7 lower entries, 3 upper ones).
 bool strip_plan_both(int n, int b, int elem, const int* rowptr, const int* colind, const int* diaind, bool split,
-                     StripPlan (&P)[2]);
+                     StripPlan (&P)[2], bool suited = false);
 // Metadata of every step and lane as the records hold it ([step][piece][lane]
 // of 4 ints): ne 16-bit codes (offset / 4 from the start of the CTA's dynamic
 // shared memory, for W warps of NS stages each), then the output position (-1:

@@ -180,7 +180,7 @@ struct Req {
   std::vector<int> posf;
   // strips (k_strip.cu): per direction the plan (less what the packed metadata
   // holds) and the metadata
-  bool strips = false;
+  bool strips = false, too_large = false;  // too_large: more than the whole budget with strips
   StripPlan strip[2];
   std::vector<int> smeta[2];
   size_t o_srec[2] = {}, o_schunk[2] = {}, o_sip[2] = {}, o_sit[2] = {}, o_sxch = 0;
@@ -333,8 +333,8 @@ namespace {
 
 // ---------------------------------------------------------------- symbolic
 
-// Which sweep kernel serves a solve whose rows do not fit strips (rows of
-// more than 16 entries do not get here; scattered numberings do).  One CTA per
+// Which sweep kernel serves a solve that strips do not suit (rows of more than 16
+// entries do not get here; scattered numberings do).  One CTA per
 // solve (k_solo.cu) keeps a solve's whole dependency chain on one SM; the
 // ranged kernel (k_sweep.cu) spreads one solve over many SMs at the price of
 // cross-SM hand-offs (about 0.75 us per dependency level).  Measured on GB300
@@ -352,8 +352,10 @@ bool use_solo(const dfg_server_s* S, const Req* r) {
   return S->fp32 && (r->b < 3 || r->n <= kSoloMaxNodes3x3);
 }
 
-// Strips (k_strip.cu) serve every solve whose rows fit them, unless the
-// configuration asks for one of the older kinds.  Measured on GB300, the
+// Strips (k_strip.cu) serve every solve whose numbering suits them (strip_serves,
+// with what was measured on both sides of its line), unless the configuration asks
+// for one of the older kinds or the request fits the budget only without them.  On
+// grids, measured on GB300, the
 // saturated 2D stream (solves/s, the rule above -> strips): FP64 45 -> 63, FP32
 // factor 87 -> 105, FP32 everything 59 -> 84; a batch of 24 requests of 2k-40k
 // nodes, FP32 factor, 257 -> 140 ms.  One strip per CTA and about four CTAs per
@@ -361,11 +363,12 @@ bool use_solo(const dfg_server_s* S, const Req* r) {
 // strip.
 constexpr int kServeStripWarps = 1;  // strips per CTA
 bool use_strips(const dfg_server_s* S, Req* r, int elem) {
-  if (S->sweeps != 0) return false;
+  if (S->sweeps != 0 || r->too_large) return false;
   // one class for both directions: a class's forward launch stands before its
   // backward launch on the class's stream, and nothing else orders a request's
   // backward sweep after the forward sweep that writes its input
-  if (strip_plan_both(r->n, r->b, elem, r->rowptr.data(), r->colind.data(), r->diaind.data(), false, r->strip)) {
+  if (strip_plan_both(r->n, r->b, elem, r->rowptr.data(), r->colind.data(), r->diaind.data(), false, r->strip, true) &&
+      strip_serves(r->strip[0]) && strip_serves(r->strip[1])) {
     const int k = strip_class_index(r->b, r->strip[0].ne);
     if (S->strip_ns[k][0] > 0 && S->strip_ns[k][1] > 0) {
       r->scls = k;
@@ -471,6 +474,7 @@ bool symbolic(dfg_server_s* S, Req* r) {
     r->alg[4] = rec(0) + dm * 2 * elem;
     r->alg[5] = rec(1) + dm * 2 * elem;
   }
+  r->P = r->T = Layout{};
   Layout& P = r->P;
   const size_t sblk = (size_t)std::max<long long>(r->sell.ptr.back(), 1);
   // mixed form: FP32 values beside the FP64 ones (the reliable updates'
@@ -811,6 +815,11 @@ void symbolic_worker(dfg_server_s* S) {
     const Clock::time_point t_sym = Clock::now();
     try {
       ok = symbolic(S, r);
+      if (ok && r->strips && r->P.total + r->T.total > S->arena.capacity()) {
+        r->too_large = true;
+        for (int dir = 0; dir < 2; ++dir) { r->strip[dir] = StripPlan{}; r->smeta[dir] = {}; }
+        ok = symbolic(S, r);
+      }
     } catch (const std::bad_alloc&) {
       r->error = "host allocation failed during the symbolic set-up";
     }

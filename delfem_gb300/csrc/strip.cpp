@@ -133,20 +133,48 @@ bool tile_strips(const Rows& R, int RW, std::vector<int>& strip, std::vector<int
   return true;
 }
 
+// The longest chain of steps: a step follows the one before it in its strip and,
+// a hand-off later, those of other strips that its rows depend on.
+long long longest_chain(const Rows& R, const std::vector<int>& strip, const std::vector<int>& lev,
+                        const std::vector<int>& steps) {
+  const int nstrips = (int)steps.size();
+  if (nstrips == 1) return steps[0];
+  std::vector<int> first(nstrips + 1, 0);  // a strip's first step
+  for (int r = 0; r < nstrips; ++r) first[r + 1] = first[r] + steps[r];
+  std::vector<int> ptr(first[nstrips] + 1, 0), rows(R.n);  // rows by step
+  for (int i = 0; i < R.n; ++i) ++ptr[first[strip[i]] + lev[i]];
+  for (int s = 0; s < first[nstrips]; ++s) ptr[s + 1] += ptr[s];
+  for (int i = R.n - 1; i >= 0; --i) rows[--ptr[first[strip[i]] + lev[i]]] = i;
+  std::vector<long long> t(first[nstrips]);
+  long long most = 0;
+  for (int r = 0; r < nstrips; ++r)
+    for (int s = first[r]; s < first[r + 1]; ++s) {
+      long long v = s > first[r] ? t[s - 1] : 0;
+      for (int p = ptr[s]; p < ptr[s + 1]; ++p)
+        for (int c = R.first(rows[p]); c < R.end(rows[p]); ++c) {
+          const int k = R.colind[c];
+          if (strip[k] != r) v = std::max(v, t[first[strip[k]] + lev[k]] + kStripHop);
+        }
+      t[s] = v + 1;
+      most = std::max(most, t[s]);
+    }
+  return most;
+}
+
 }  // namespace
 
 bool strip_plan(int n, int b, int elem, const int* rowptr, const int* colind, const int* diaind, bool forward, bool split,
-                StripPlan& P, int min_ne) {
+                StripPlan& P, int min_ne, bool suited) {
   P = StripPlan{};
   P.forward = forward;
   P.n = n;
   P.b = b;
   P.elem = elem;
   auto row_of = [&](int p) { return forward ? p : n - 1 - p; };
-  auto first = [&](int row) { return forward ? rowptr[row] : diaind[row]; };
+  auto first_entry = [&](int row) { return forward ? rowptr[row] : diaind[row]; };
   auto end = [&](int row) { return forward ? diaind[row] : rowptr[row + 1]; };
   int maxe = 0;
-  for (int i = 0; i < n; ++i) maxe = std::max(maxe, end(i) - first(i));
+  for (int i = 0; i < n; ++i) maxe = std::max(maxe, end(i) - first_entry(i));
   P.ne = strip_class(maxe);
   if (n == 0 || P.ne == 0) return false;
   P.ne = std::max(P.ne, min_ne);
@@ -158,7 +186,7 @@ bool strip_plan(int n, int b, int elem, const int* rowptr, const int* colind, co
   for (int p = 0; p < n; ++p) {
     const int row = row_of(p);
     int lv = 0;
-    for (int c = first(row); c < end(row); ++c) lv = std::max(lv, glev[colind[c]] + 1);
+    for (int c = first_entry(row); c < end(row); ++c) lv = std::max(lv, glev[colind[c]] + 1);
     glev[row] = lv;
   }
   const Rows R{n, forward, rowptr, colind, diaind, glev.data()};
@@ -170,6 +198,10 @@ bool strip_plan(int n, int b, int elem, const int* rowptr, const int* colind, co
   for (int r = 0; r < P.nstrips; ++r) P.strip_chunk.push_back(P.strip_chunk.back() + (steps[r] + CH - 1) / CH);
   P.nchunks = P.strip_chunk.back();
   const size_t nsteps = (size_t)P.steps();
+  if ((double)nsteps * RW * b > 2147483647.0) return false;  // places are int
+  P.levels = *std::max_element(glev.begin(), glev.end()) + 1;
+  P.chain = longest_chain(R, strip, lev, steps);
+  if (suited && !strip_suits(P)) return false;
   P.pos.resize(n);
   P.step_rows.assign(nsteps * RW, -1);
   for (int row = 0; row < n; ++row) {
@@ -198,9 +230,9 @@ bool strip_plan(int n, int b, int elem, const int* rowptr, const int* colind, co
         const size_t at = (size_t)(s0 + s) * RW + l;
         const int row = P.step_rows[at];
         if (row < 0) continue;
-        for (int c = first(row); c < end(row); ++c) {
+        for (int c = first_entry(row); c < end(row); ++c) {
           const int k = colind[c];
-          const size_t e = at * ne + (c - first(row));
+          const size_t e = at * ne + (c - first_entry(row));
           P.ent_slot[e] = c;
           if (strip[k] == r && s - lev[k] < kStripRing) {
             P.codes[e] = ring0 + ((lev[k] % kStripRing) * RW + lane[k]) * P.d.VS;
@@ -236,13 +268,13 @@ bool strip_plan(int n, int b, int elem, const int* rowptr, const int* colind, co
 }
 
 bool strip_plan_both(int n, int b, int elem, const int* rowptr, const int* colind, const int* diaind, bool split,
-                     StripPlan (&P)[2]) {
+                     StripPlan (&P)[2], bool suited) {
   int maxe = 0;
   for (int i = 0; i < n; ++i) maxe = std::max({maxe, diaind[i] - rowptr[i], rowptr[i + 1] - diaind[i]});
   const int ne = strip_class(maxe);
   if (ne == 0) return false;
   for (int dir = 0; dir < 2; ++dir)
-    if (!strip_plan(n, b, elem, rowptr, colind, diaind, dir == 0, split, P[dir], ne)) return false;
+    if (!strip_plan(n, b, elem, rowptr, colind, diaind, dir == 0, split, P[dir], ne, suited)) return false;
   return true;
 }
 

@@ -377,7 +377,7 @@ typedef struct {
   int size_groups;        /* solves grouped by size, each group iterating at its own pace on its own
                              streams: 1 = one table for all, 2-3 groups; 0 = 3 */
   int sweeps;             /* triangular-sweep kernel: 0 = strips (a warp per strip of grid lines) where a
-                             solve's rows fit them, else one CTA per solve in FP32 (except 3x3-block
+                             solve's numbering suits them, else one CTA per solve in FP32 (except 3x3-block
                              solves above 100,000 nodes) and ranged over several CTAs otherwise,
                              1 = ranged, 2 = one CTA per solve; the same bits either way */
 } dfg_server_config;
