@@ -1197,7 +1197,7 @@ PrecondLaunch precond_launch(dfg_ctx ctx_, dfg_precond pr, bool fp32, const void
                              int* tickets, const int* done) {
   PrecondLaunch L;
   const long long m = (long long)pr->n * pr->b;
-  if (pr->strips) {
+  if (pr->strips[fp32 ? 1 : 0]) {
     StripDev &f = pr->strip[0][fp32 ? 1 : 0], &b = pr->strip[1][fp32 ? 1 : 0];
     L.F = strip_launch(ctx_, pr, 0, fp32, b.in.p, tickets, done);
     L.B = strip_launch(ctx_, pr, 1, fp32, z, tickets + 1, done);
@@ -1251,10 +1251,10 @@ struct GraphHolder {
 };
 
 // Uploads one direction and precision of the strip sweeps; false when the
-// rows do not fit them (strip_plan).  out_pos: where results go (nullptr: row
-// order).
+// rows do not fit or suit them (strip_plan).  out_pos: where results go (nullptr:
+// row order).  grid: cleared when the strips are not those of a grid.
 bool setup_strip(dfg_ctx ctx_, dfg_precond pr, const FactorPattern& F, bool forward, bool fp32, const int* out_pos,
-                 std::vector<int>* pos) {
+                 std::vector<int>* pos, bool& grid) {
   StripDev& D = pr->strip[forward ? 0 : 1][fp32 ? 1 : 0];
   D = StripDev{};
   const int n = pr->n, b = pr->b, elem = fp32 ? 4 : 8;
@@ -1265,9 +1265,12 @@ bool setup_strip(dfg_ctx ctx_, dfg_precond pr, const FactorPattern& F, bool forw
   // 373 / 310).
   StripPlan P;
   const bool split = strip_can_split(b, elem);
-  if (!strip_plan(n, b, elem, F.rowptr, F.colind, F.diaind, forward, split, P)) return false;
-  if (P.d.Q > 1 && P.nstrips > 2 * ctx_->nsm && !strip_plan(n, b, elem, F.rowptr, F.colind, F.diaind, forward, false, P))
-    return false;
+  auto plan = [&](bool s) {
+    return strip_plan(n, b, elem, F.rowptr, F.colind, F.diaind, forward, s, P, 0, true);
+  };
+  if (!plan(split)) return false;
+  if (P.d.Q > 1 && P.nstrips > 2 * ctx_->nsm && !plan(false)) return false;
+  grid &= strip_like_grid(P);
   D.d = P.d;
   D.ne = P.ne;
   D.nstrips = P.nstrips;
@@ -1320,50 +1323,37 @@ bool setup_strip(dfg_ctx ctx_, dfg_precond pr, const FactorPattern& F, bool forw
   return true;
 }
 
-// Both directions and precisions of the strip sweeps.
-bool setup_strips(dfg_ctx ctx_, dfg_precond pr) {
+void drop_strips(dfg_precond pr, int p) {  // p: 0 FP64, 1 FP32
+  pr->strips[p] = false;
+  for (auto& dir : pr->strip) dir[p] = StripDev{};
+}
+
+// Both directions of the strip sweeps in one precision; false when the rows do
+// not fit or suit them.
+bool setup_strips(dfg_ctx ctx_, dfg_precond pr, bool fp32, bool& grid) {
   const FactorPattern F = factor_pattern(pr);
-  for (int k = 0; k < 2; ++k) {
-    std::vector<int> ypos;  // y lies where the backward sweep reads it
-    if (!setup_strip(ctx_, pr, F, false, k == 1, nullptr, &ypos) ||
-        !setup_strip(ctx_, pr, F, true, k == 1, ypos.data(), nullptr)) {
-      for (auto& dir : pr->strip)
-        for (StripDev& D : dir) D = StripDev{};
-      return false;
-    }
-  }
+  std::vector<int> ypos;  // y lies where the backward sweep reads it
+  if (!setup_strip(ctx_, pr, F, false, fp32, nullptr, &ypos, grid) ||
+      !setup_strip(ctx_, pr, F, true, fp32, ypos.data(), nullptr, grid))
+    return false;
   CK(strip_set_smem_limits(ctx_->smem_optin));
   return true;
 }
 
-// Schedule choice.  Ranged: the cost model keeps a few candidate range sizes
-// and the fullest-step plan joins them.  Level-scheduled: one launch per
-// dependency level.  Each candidate is timed on the device as one FP32 sweep
-// of the real structure (values do not change the timing; the level launches
-// as a graph, as the solvers replay them) and the fastest wins.  The
-// preconditioner's sweep mode can restrict the choice to one kind.
-// strips: the strip sweeps take the place of the ranged and the one-CTA kinds;
-// they are timed as the ranged kind and the caller makes the choice.
-void setup_sweep(dfg_ctx ctx_, dfg_precond pr, SweepDev& S, const dfg_system sys, bool forward, bool strips) {
-  const FactorPattern F = factor_pattern(pr);
-  const int mode = pr->sweep_mode;
-  const long long m = (long long)sys->n * sys->b;
-  S.forward = forward;
-  S.levels = false;
-  S.t_ranged = S.t_levels = -1.f;
-  DBuf vin, vout;
-  dalloc(ctx_, vin, (size_t)m * 4 + 64);
-  dalloc(ctx_, vout, (size_t)m * 4 + 64);
-  CK(cudaMemsetAsync(vin.p, 0, vin.bytes, ctx_->stream));
-  Scratch sc = scratch_of(ctx_);
-  cudaEvent_t e0, e1;
-  CK(cudaEventCreate(&e0));
-  CK(cudaEventCreate(&e1));
-  struct EventPair {
-    cudaEvent_t a, b;
-    ~EventPair() { cudaEventDestroy(a); cudaEventDestroy(b); }
-  } ev{e0, e1};
-  auto elapsed = [&](auto&& run) {
+// Milliseconds of a piece of work on the context's stream, the best of two.
+struct SweepTimer {
+  dfg_ctx ctx_;
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  explicit SweepTimer(dfg_ctx c) : ctx_(c) {
+    CK(cudaEventCreate(&e0));
+    const cudaError_t e = cudaEventCreate(&e1);
+    if (e != cudaSuccess) cudaEventDestroy(e0);
+    CK(e);
+  }
+  ~SweepTimer() { cudaEventDestroy(e0); cudaEventDestroy(e1); }
+  SweepTimer(const SweepTimer&) = delete;
+  template <typename F>
+  float operator()(F&& run) {
     float best = 1e30f;
     for (int rep = 0; rep < 2; ++rep) {
       CK(cudaEventRecord(e0, ctx_->stream));
@@ -1375,34 +1365,50 @@ void setup_sweep(dfg_ctx ctx_, dfg_precond pr, SweepDev& S, const dfg_system sys
       best = std::min(best, ms);
     }
     return best;
-  };
+  }
+};
+
+void check_timed(dfg_ctx ctx_) {
+  if (read_err(ctx_) == 0) return;
+  CK(cudaMemsetAsync(ctx_->err_word.p, 0, sizeof(int), ctx_->stream));
+  set_err(ctx_, "a triangular-sweep wait timed out while choosing the schedule");
+  throw Fail{DFG_TIMEOUT};
+}
+
+// Schedule choice.  Ranged: the cost model keeps a few candidate range sizes
+// and the fullest-step plan joins them.  Level-scheduled: one launch per
+// dependency level.  Each candidate is timed on the device as one FP32 sweep
+// of the real structure (values do not change the timing; the level launches
+// as a graph, as the solvers replay them) and the fastest wins.  The
+// preconditioner's sweep mode can restrict the choice to one kind.
+// levels_only: the ranged and the one-CTA kinds are left out (the strips of a
+// grid have been the faster ones at every size).  all: a single candidate is timed too.
+void setup_sweep(dfg_ctx ctx_, dfg_precond pr, SweepDev& S, const dfg_system sys, bool forward, bool levels_only,
+                 bool all) {
+  const FactorPattern F = factor_pattern(pr);
+  const int mode = pr->sweep_mode;
+  const long long m = (long long)sys->n * sys->b;
+  S.forward = forward;
+  S.levels = false;
+  S.t_ranged = S.t_levels = -1.f;
+  DBuf vin, vout;
+  dalloc(ctx_, vin, (size_t)m * 4 + 64);
+  dalloc(ctx_, vout, (size_t)m * 4 + 64);
+  CK(cudaMemsetAsync(vin.p, 0, vin.bytes, ctx_->stream));
+  Scratch sc = scratch_of(ctx_);
+  SweepTimer elapsed(ctx_);
   // ranged candidates
   std::vector<SweepPlan> cands;
   size_t best = 0;
   float best_ms = 1e30f;
-  if (strips) {
-    SweepLaunch L = strip_launch(ctx_, pr, forward ? 0 : 1, true, forward ? pr->strip[1][1].in.p : vout.p,
-                                 sc.tickets + 2, nullptr);
-    const StripDev& D = pr->strip[forward ? 0 : 1][1];
-    S.t_ranged = elapsed([&] {
-      CK(fill_sentinel(D.nxch, D.xch.p, true, ctx_->stream));
-      CK(cudaMemsetAsync(sc.tickets + 2, 0, sizeof(int), ctx_->stream));
-      CK(enqueue_sweep(L, ctx_->stream));
-    });
-    launched(ctx_, 4);
-    if (read_err(ctx_) != 0) {
-      CK(cudaMemsetAsync(ctx_->err_word.p, 0, sizeof(int), ctx_->stream));
-      set_err(ctx_, "a triangular-sweep wait timed out while choosing the schedule");
-      throw Fail{DFG_TIMEOUT};
-    }
-  } else if (mode != 2) {
+  if (!levels_only && mode != 2) {
     cands = candidate_sweep_plans(sys->n, sys->b, F.rowptr, F.colind, F.diaind, forward, 32, 4);
     // and the fullest-step plan (ranges of up to 32 grid lines), if it differs
     SweepPlan full = fullest_sweep_plan(sys->n, sys->b, F.rowptr, F.colind, F.diaind, forward, 32);
     bool seen = false;
     for (const SweepPlan& c : cands) seen |= (c.nranges == full.nranges && c.nsteps == full.nsteps);
     if (!seen) cands.push_back(std::move(full));
-    if (cands.size() > 1 || mode == 0) {
+    if (cands.size() > 1 || mode == 0 || all) {
       for (size_t c = 0; c < cands.size(); ++c) {
         SweepDev T;
         T.forward = forward;
@@ -1421,18 +1427,14 @@ void setup_sweep(dfg_ctx ctx_, dfg_precond pr, SweepDev& S, const dfg_system sys
         if (ms < best_ms) { best_ms = ms; best = c; }
         cands[c] = std::move(T.plan);
       }
-      if (read_err(ctx_) != 0) {
-        CK(cudaMemsetAsync(ctx_->err_word.p, 0, sizeof(int), ctx_->stream));
-        set_err(ctx_, "a triangular-sweep wait timed out while choosing the schedule");
-        throw Fail{DFG_TIMEOUT};
-      }
+      check_timed(ctx_);
       S.t_ranged = best_ms;
     }
   }
   // one-CTA candidate (k_solo.cu), timed in FP32 with its input permutation
   S.solo = false;
   S.t_solo = -1.f;
-  if ((mode == 0 && !strips) || mode == 3) {
+  if ((mode == 0 && !levels_only) || mode == 3) {
     const bool fits = setup_solo(ctx_, pr, S, F, forward);
     REQUIRE(fits || mode != 3, DFG_INVALID_ARGUMENT, "the one-CTA sweep's records do not fit in shared memory");
     if (fits) {
@@ -1443,11 +1445,7 @@ void setup_sweep(dfg_ctx ctx_, dfg_precond pr, SweepDev& S, const dfg_system sys
         CK(enqueue_sweep(L, ctx_->stream));
       });
       launched(ctx_, 4);
-      if (read_err(ctx_) != 0) {
-        CK(cudaMemsetAsync(ctx_->err_word.p, 0, sizeof(int), ctx_->stream));
-        set_err(ctx_, "a triangular-sweep wait timed out while choosing the schedule");
-        throw Fail{DFG_TIMEOUT};
-      }
+      check_timed(ctx_);
       S.t_solo = ms;
       if (mode == 3 || ms < best_ms) {
         best_ms = ms;
@@ -1500,7 +1498,7 @@ void setup_sweep(dfg_ctx ctx_, dfg_precond pr, SweepDev& S, const dfg_system sys
       const float ms = elapsed([&] { CK(cudaGraphLaunch(g.exec, ctx_->stream)); });
       launched(ctx_, 3 * launches_of(L));
       S.t_levels = ms;
-      take = strips || ms < best_ms;
+      take = levels_only || ms < best_ms;
     }
     if (take) {
       S.levels = true;
@@ -1515,12 +1513,142 @@ void setup_sweep(dfg_ctx ctx_, dfg_precond pr, SweepDev& S, const dfg_system sys
       return;
     }
   }
-  if (S.solo || strips) {
+  if (S.solo || levels_only) {
     S.plan = SweepPlan{};
     return;
   }
   S.plan = std::move(cands[best]);
   setup_sweep_plan(ctx_, S);
+}
+
+// Times both strip sweeps in one precision: forward, backward.
+void time_strips(dfg_ctx ctx_, dfg_precond pr, int p, float (&ms)[2]) {
+  const bool fp32 = p == 1;
+  DBuf z;
+  dalloc(ctx_, z, (size_t)pr->n * pr->b * (fp32 ? 4 : 8) + 64);
+  SweepTimer elapsed(ctx_);
+  int* ticket = scratch_of(ctx_).tickets + 2;
+  for (int dir = 0; dir < 2; ++dir) {
+    const StripDev& D = pr->strip[dir][p];
+    const SweepLaunch L = strip_launch(ctx_, pr, dir, fp32, dir == 0 ? pr->strip[1][p].in.p : z.p, ticket, nullptr);
+    ms[dir] = elapsed([&] {
+      CK(fill_sentinel(D.nxch, D.xch.p, fp32, ctx_->stream));
+      CK(cudaMemsetAsync(ticket, 0, sizeof(int), ctx_->stream));
+      CK(enqueue_sweep(L, ctx_->stream));
+    });
+    launched(ctx_, 4);
+  }
+  check_timed(ctx_);
+}
+
+// One sweep of the kind that setup_sweep chose, in FP64 (on a zero factor).
+float time_sweep64(dfg_ctx ctx_, dfg_precond pr, SweepDev& S) {
+  const size_t m = (size_t)pr->n * pr->b;
+  DBuf in, out;
+  dalloc(ctx_, in, m * 8 + 64);
+  dalloc(ctx_, out, m * 8 + 64);
+  CK(cudaMemsetAsync(in.p, 0, in.bytes, ctx_->stream));
+  CK(cudaMemsetAsync(pr->fdiag.p, 0, pr->fdiag.bytes, ctx_->stream));
+  CK(cudaMemsetAsync(pr->foffd.p, 0, pr->foffd.bytes, ctx_->stream));
+  SweepTimer elapsed(ctx_);
+  int* ticket = scratch_of(ctx_).tickets + 2;
+  const SweepLaunch L = sweep_launch(ctx_, pr, S, false, in.p, out.p, ticket, nullptr);
+  GraphHolder g;
+  if (L.levels) {
+    CK(cudaStreamBeginCapture(ctx_->stream, cudaStreamCaptureModeThreadLocal));
+    const cudaError_t ce = enqueue_sweep(L, ctx_->stream);
+    CK(cudaStreamEndCapture(ctx_->stream, &g.graph));
+    CK(ce);
+    CK(cudaGraphInstantiate(&g.exec, g.graph, 0));
+    CK(cudaGraphLaunch(g.exec, ctx_->stream));  // first replay uploads the graph
+  }
+  const float ms = elapsed([&] {
+    if (L.levels) {
+      CK(cudaGraphLaunch(g.exec, ctx_->stream));
+      return;
+    }
+    CK(fill_sentinel((long long)m, out.p, false, ctx_->stream));
+    CK(cudaMemsetAsync(ticket, 0, sizeof(int), ctx_->stream));
+    CK(enqueue_sweep(L, ctx_->stream));
+  });
+  launched(ctx_, 4 * launches_of(L));
+  check_timed(ctx_);
+  return ms;
+}
+
+// The sweeps' schedule.  Strips where they are a grid's in both precisions, unless
+// both directions together are faster level-scheduled (in mode 1: always).  Other
+// strips are timed beside all the older kinds, each precision by itself, and have to
+// be faster by a tenth, since they take more memory.  Measured on GB300, FP64 / FP32
+// us per iteration, older kinds -> chosen, 20,000-node Delaunay meshes of jittered
+// grid points: 3D 3x3 in their own order 1,126 / 752 -> 1,122 / 346 (strips in FP32
+// only; in FP64 1,278), 2D 2x2 1,499 / 405 -> 692 / 397 (in FP64 only), 3D grids by
+// reverse Cuthill-McKee 1,648 / 455 -> 490 / 297 (both).  Set-up takes up to twice as
+// long where they lose (3D 3x3, 100,000 nodes: 346 -> 682 ms).
+void setup_sweeps(dfg_ctx ctx_, dfg_precond pr, const dfg_system sys) {
+  const int mode = pr->sweep_mode;
+  SweepDev* S[2] = {&pr->fwd, &pr->bwd};
+  for (SweepDev* s : S) *s = SweepDev{};
+  auto fits = [&](auto&& work) {  // false: no memory for it on the device
+    try {
+      work();
+      return true;
+    } catch (const Fail& f) {
+      if (f.status != DFG_OOM_REJECTED) throw;
+      CK(cudaStreamSynchronize(ctx_->stream));
+      return false;
+    }
+  };
+  // per precision: strips built, their set-up times (forward, backward)
+  bool have[2] = {}, grid = true;
+  float ts[2][2] = {};
+  for (int p = 0; p < 2; ++p) {
+    drop_strips(pr, p);
+    auto build = [&] {
+      if (!setup_strips(ctx_, pr, p == 1, grid)) return;
+      if (p == 1 || !grid) time_strips(ctx_, pr, p, ts[p]);
+      have[p] = true;
+    };
+    if ((mode != 0 && mode != 1) || !fits(build) || !have[p]) {
+      have[p] = grid = false;
+      drop_strips(pr, p);
+    }
+  }
+  if (!grid && have[0] && ts[0][0] == 0.f) time_strips(ctx_, pr, 0, ts[0]);
+  const bool strips = have[0] || have[1];
+  if (!grid || mode == 0) {
+    float t64 = 0.f;
+    auto older = [&] {
+      for (int dir = 0; dir < 2; ++dir) setup_sweep(ctx_, pr, *S[dir], sys, dir == 0, grid, strips);
+      for (int dir = 0; dir < 2 && have[0] && !grid; ++dir) t64 += time_sweep64(ctx_, pr, *S[dir]);
+    };
+    if (!strips) return older();
+    if (!fits(older)) {  // no memory beside the strips
+      for (SweepDev* s : S) *s = SweepDev{};
+      for (int p = 0; p < 2; ++p) drop_strips(pr, p);
+      have[0] = have[1] = grid = false;
+      return older();
+    }
+    auto t32 = [&](const SweepDev& s) { return s.solo ? s.t_solo : s.levels ? s.t_levels : s.t_ranged; };
+    const float t[2] = {t64, t32(pr->fwd) + t32(pr->bwd)};
+    for (int p = 0; p < 2; ++p) {
+      const float strip = ts[p][0] + ts[p][1];
+      pr->strips[p] = have[p] && (grid ? ts[1][0] + ts[1][1] <= t[1] : 1.1f * strip < t[p]);
+      if (!pr->strips[p]) drop_strips(pr, p);
+    }
+  } else {
+    pr->strips[0] = pr->strips[1] = true;
+  }
+  for (int dir = 0; dir < 2; ++dir) {
+    if (grid || pr->strips[1]) S[dir]->t_ranged = ts[1][dir];  // strips count as the ranged kind
+    if (pr->strips[0] && pr->strips[1]) {
+      SweepDev T;  // the timings stay
+      T.t_ranged = S[dir]->t_ranged;
+      T.t_levels = S[dir]->t_levels;
+      T.t_solo = S[dir]->t_solo;
+      *S[dir] = std::move(T);
+    }
+  }
 }
 
 }  // namespace
@@ -1569,7 +1697,7 @@ extern "C" int dfg_precond_get_sweep_mode(dfg_precond prec, int* fwd, int* bwd) 
     prec->ctx->last_error = "dfg_precond_set_linear_system must come first";
     return DFG_NOT_READY;
   }
-  if (prec->strips) {  // the ranged kind's kernel where the rows fit it
+  if (prec->strips[1]) {  // the ranged kind's kernel where the rows fit it
     if (fwd) *fwd = 1;
     if (bwd) *bwd = 1;
     return DFG_OK;
@@ -1651,25 +1779,7 @@ extern "C" int dfg_precond_set_linear_system(dfg_precond prec, dfg_system sys) {
     prec->ilu = ilu_plan(sys->b, prec->lev_fwd.ptr, prec->lev_fwd.rows, F.rowptr, F.colind, F.diaind);
     upload(ctx, prec->ilu_units, prec->ilu.units.data(), prec->ilu.units.size());
     dalloc(ctx, prec->ilu_sync, kIluSync * 4);
-    // strips where the rows fit them, unless both directions together are
-    // faster level-scheduled
-    prec->fwd = SweepDev{};
-    prec->bwd = SweepDev{};
-    prec->strips = (prec->sweep_mode == 0 || prec->sweep_mode == 1) && setup_strips(ctx, prec);
-    setup_sweep(ctx, prec, prec->fwd, sys, true, prec->strips);
-    setup_sweep(ctx, prec, prec->bwd, sys, false, prec->strips);
-    if (prec->strips && prec->sweep_mode == 0 &&
-        prec->fwd.t_levels + prec->bwd.t_levels < prec->fwd.t_ranged + prec->bwd.t_ranged) {
-      prec->strips = false;
-      for (auto& dir : prec->strip)
-        for (StripDev& D : dir) D = StripDev{};
-    } else if (prec->strips) {
-      for (SweepDev* S : {&prec->fwd, &prec->bwd}) {
-        S->levels = false;
-        S->lev = Levels{};
-        S->lev_info.release();
-      }
-    }
+    setup_sweeps(ctx, prec, sys);
     dalloc(ctx, prec->ybuf64, vec_bytes(sys, 8));
     dalloc(ctx, prec->ybuf32, vec_bytes(sys, 4));
     CK(cudaStreamSynchronize(ctx->stream));
@@ -1740,7 +1850,7 @@ extern "C" int dfg_precond_set_value(dfg_precond prec, dfg_system sys) {
     const int* h_sync = host_area(ctx).words;
     static_assert(kIluSync <= 16, "kIluSync words of HostArea");
     CK(cudaMemcpyAsync(host_area(ctx).words, sync, kIluSync * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    if (prec->strips) {
+    if (prec->strips[0]) {
       pack_strips(ctx, prec, false);
     } else {
       pack_sweep(ctx, prec, prec->fwd, false);
@@ -1765,7 +1875,7 @@ extern "C" int dfg_precond_set_value(dfg_precond prec, dfg_system sys) {
 namespace {
 void ensure_numeric32(dfg_ctx ctx_, dfg_precond prec) {
   if (prec->numeric32) return;
-  if (prec->strips) {
+  if (prec->strips[1]) {
     pack_strips(ctx_, prec, true);
     prec->numeric32 = true;
     return;
@@ -1794,7 +1904,7 @@ extern "C" int dfg_precond_solve(dfg_precond prec, dfg_system sys, int iv) {
     const long long m = (long long)sys->n * sys->b;
     Scratch sc = scratch_of(ctx);
     PrecondLaunch L = precond_launch(ctx, prec, false, v, nullptr, v, sc.tickets, nullptr);
-    if (prec->strips) {
+    if (prec->strips[0]) {
       CK(sweep_feed(L.feed, m, v, sc.tickets, ctx->stream));
       launched(ctx, 1);
       run_sweep(ctx, L.F);
@@ -1805,7 +1915,7 @@ extern "C" int dfg_precond_solve(dfg_precond prec, dfg_system sys, int iv) {
       run_sweep(ctx, L.F);
       CK(fill_sentinel(m, v, false, ctx->stream));
     }
-    run_sweep(ctx, L.B, prec->strips);
+    run_sweep(ctx, L.B, prec->strips[0]);
     if (read_err(ctx) != 0) {
       CK(cudaMemsetAsync(ctx->err_word.p, 0, sizeof(int), ctx->stream));
       set_err(ctx, "a triangular-sweep wait timed out");

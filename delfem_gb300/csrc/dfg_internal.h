@@ -299,7 +299,7 @@ struct dfg_precond_s {
   dfg::IluPlan ilu;                       // one-launch factorisation (units on the device)
   dfg::DBuf ilu_units, ilu_sync, ilu_src;  // ilu_src: A on a pattern with fill-in
   dfg::SweepDev fwd, bwd;
-  bool strips = false;             // both directions sweep in strips (fwd, bwd then unused)
+  bool strips[2] = {};             // [FP64, FP32]: both directions sweep in strips (fwd, bwd then unused)
   dfg::StripDev strip[2][2];       // [forward, backward][FP64, FP32]
   dfg::DBuf ybuf64, ybuf32;        // forward-sweep outputs
 };

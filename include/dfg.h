@@ -233,17 +233,21 @@ int dfg_precond_set_fill_level(dfg_precond prec, int lev);
 int dfg_precond_set_linear_system(dfg_precond prec, dfg_system sys);
 /* How the triangular sweeps are scheduled (no counterpart in the reference,
  * whose substitutions are sequential loops): 0 (default) times the kinds
- * on the device at the symbolic set-up and keeps the faster; 1 = ranged (rows
- * pipelined across CTAs: in strips of grid lines, a warp each, where the rows
- * fit them, else in contiguous row ranges); 2 = level-scheduled (one launch per
+ * on the device at the symbolic set-up and keeps the fastest; 1 = ranged (rows
+ * pipelined across CTAs: in strips of grid lines, a warp each, or in contiguous
+ * row ranges); 2 = level-scheduled (one launch per
  * dependency level, good for matrices with few wide levels, such as those of
  * unordered meshes); 3 = one CTA (the whole sweep on one SM, level after
  * level, its input first permuted into the schedule's order).  Where the rows
- * fit strips, 0 chooses between 1 and 2 for both directions together; else
- * among all three kinds per direction.  Takes effect at the next
- * dfg_precond_set_linear_system; results agree to rounding. */
+ * are numbered as a grid's, 1 takes strips, and 0 chooses between strips and 2 for
+ * both directions together.  Elsewhere 0 chooses among all three kinds per
+ * direction, 1 takes ranges, and where strips are possible they have to be faster
+ * than that choice by a tenth for both directions together, in FP64 and FP32 each by
+ * itself.  Takes effect at the next dfg_precond_set_linear_system; results agree to
+ * rounding. */
 int dfg_precond_set_sweep_mode(dfg_precond prec, int mode);
-/* The kind chosen per direction after the symbolic set-up (1, 2 or 3). */
+/* The kind chosen per direction for FP32 sweeps after the symbolic set-up (1, 2 or
+ * 3; strips are 1). */
 int dfg_precond_get_sweep_mode(dfg_precond prec, int* fwd, int* bwd);
 /* The set-up's timings behind that choice, ms per FP32 sweep: ms[0..3] =
  * forward ranged, forward level-scheduled, backward ranged, backward
