@@ -71,6 +71,34 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+// What a sweep takes off a row's right-hand side, entry after entry: component p of
+// t[p] - sum over e, q of block(e)(p, q) x(e)(q), in one order for every kernel that
+// evaluates a row in one lane or a lane per component.  FP32 rows of 3x3 blocks (21
+// products per component in a tetrahedral mesh) are added up in four sums, entry e
+// in sum e % 4, apart from the right-hand side: one chain from the right-hand side on
+// has 1.9 times the error of the level-scheduled kernel's sums over lanes (elasticity
+// on 56^3 cells, sweep against FP64: 1.02e-7, 5.4e-8, in four sums 5.4e-8), and takes
+// as long (that solve 130.7 and 131.1 ms).
+template <typename T, int B, int P = B>
+struct RowSum {
+  static constexpr int N = sizeof(T) == 4 && B == 3 ? 4 : 1;
+  T s[N][P];
+  __device__ __forceinline__ void start(const T (&t)[P]) {
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+#pragma unroll
+      for (int p = 0; p < P; ++p) s[k][p] = N == 1 ? t[p] : T(0);
+  }
+  __device__ __forceinline__ void add(int e, int p, T a, T x) {
+    if (N == 1) s[0][p] -= a * x;
+    else s[e % N][p] += a * x;
+  }
+  __device__ __forceinline__ T row(int p, T t) const {
+    if constexpr (N == 1) return s[0][p];
+    else return t - ((s[0][p] + s[1][p]) + (s[2][p] + s[3][p]));
+  }
+};
+
 // Programmatic dependent launch (kernels launched with
 // cudaLaunchAttributeProgrammaticStreamSerialization): wait until the
 // previous kernel in the stream has finished and its writes are visible,

@@ -181,6 +181,8 @@ __global__ void __launch_bounds__((kSoloWarps + 1) * 32) k_solo(SoloArgs a) {
               T t[B];
 #pragma unroll
               for (int d = 0; d < B; ++d) t[d] = val[lane * B + d];
+              RowSum<T, B> sum;
+              sum.start(t);
               if constexpr (MAXE > 0) {
                 // all dependency values first, then the FMAs.  The codes are
                 // loaded together, then every value from the ring together
@@ -214,36 +216,36 @@ __global__ void __launch_bounds__((kSoloWarps + 1) * 32) k_solo(SoloArgs a) {
                 for (int e = 0; e < MAXE; ++e) {
                   if (e < nent) {
 #pragma unroll
-                    for (int p = 0; p < B; ++p) {
-                      T acc = t[p];
+                    for (int p = 0; p < B; ++p)
 #pragma unroll
-                      for (int q = 0; q < B; ++q) acc -= blk[(e * BS + p * B + q) * 32 + lane] * v[e][q];
-                      t[p] = acc;
-                    }
+                      for (int q = 0; q < B; ++q) sum.add(e, p, blk[(e * BS + p * B + q) * 32 + lane], v[e][q]);
                   }
                 }
               } else {
-                for (int e = 0; e < nent; ++e) {
-                  const int cd = code[e * 32 + lane];
-                  T v[B];
-                  if (cd >= 0) {
-                    const T* vp = reinterpret_cast<const T*>(ringreg + cd);
+                for (int e0 = 0; e0 < nent; e0 += RowSum<T, B>::N)
 #pragma unroll
-                    for (int d = 0; d < B; ++d) v[d] = vp[d];
-                  } else {
-                    const T* gp = out + (size_t)(-cd - 1) * B;
+                  for (int k = 0; k < RowSum<T, B>::N; ++k) {
+                    const int e = e0 + k;
+                    if (e >= nent) break;
+                    const int cd = code[e * 32 + lane];
+                    T v[B];
+                    if (cd >= 0) {
+                      const T* vp = reinterpret_cast<const T*>(ringreg + cd);
 #pragma unroll
-                    for (int d = 0; d < B; ++d) v[d] = __ldcg(gp + d);
+                      for (int d = 0; d < B; ++d) v[d] = vp[d];
+                    } else {
+                      const T* gp = out + (size_t)(-cd - 1) * B;
+#pragma unroll
+                      for (int d = 0; d < B; ++d) v[d] = __ldcg(gp + d);
+                    }
+#pragma unroll
+                    for (int p = 0; p < B; ++p)
+#pragma unroll
+                      for (int q = 0; q < B; ++q) sum.add(k, p, blk[(e * BS + p * B + q) * 32 + lane], v[q]);
                   }
-#pragma unroll
-                  for (int p = 0; p < B; ++p) {
-                    T acc = t[p];
-#pragma unroll
-                    for (int q = 0; q < B; ++q) acc -= blk[(e * BS + p * B + q) * 32 + lane] * v[q];
-                    t[p] = acc;
-                  }
-                }
               }
+#pragma unroll
+              for (int p = 0; p < B; ++p) t[p] = sum.row(p, t[p]);
               T y[B];
               if constexpr (FWD) {
                 const T* dinv = blk + nent * BS * 32;

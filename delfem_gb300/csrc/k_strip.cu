@@ -35,9 +35,9 @@
 // Every wait is bounded; one that gives up records kErrTimeout, and the launch
 // drains its copies and returns.
 //
-// A row is evaluated by the operations of the other sweep kernels in their
-// order (entries ascending, FMA chain, then D^-1), so the ranged and one-CTA
-// kernels give the same bits; with split, column by column.
+// A row is evaluated by the operations of the ranged and one-CTA kernels in their
+// order (RowSum, then D^-1), so these give the same bits; with split, column by
+// column.
 //
 // Chunk layout: [need: CH ints, kStripHdr bytes][steps: step_bytes each]; a
 // step is pieces of 16 bytes per lane, piece j of lane l at (j*32 + l)*16:
@@ -504,15 +504,17 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
             if (SZ == 8 && more) decode((j + 1) % K2);
             // the rows
             if constexpr (LPR == 1) {
-              T acc[B];
-#pragma unroll
-              for (int d = 0; d < B; ++d) acc[d] = t[k][d];
+              RowSum<T, B> sum;
+              sum.start(t[k]);
 #pragma unroll
               for (int e = 0; e < NE; ++e)
 #pragma unroll
                 for (int d = 0; d < B; ++d)
 #pragma unroll
-                  for (int q = 0; q < B; ++q) acc[d] -= A(e * EV + d * B + q) * x[e].v[q];
+                  for (int q = 0; q < B; ++q) sum.add(e, d, A(e * EV + d * B + q), x[e].v[q]);
+              T acc[B];
+#pragma unroll
+              for (int d = 0; d < B; ++d) acc[d] = sum.row(d, t[k][d]);
               Vec<T, BP> y;
               y.v[BP - 1] = 0;
 #pragma unroll
@@ -540,11 +542,13 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
               yl.v[0] = acc;
               if (XNOW) xstore(xs[k], xp[k], yl);
             } else {
-              T acc = t[k][0];
+              RowSum<T, B, 1> sum;
+              sum.start(t[k]);
 #pragma unroll
               for (int e = 0; e < NE; ++e)
 #pragma unroll
-                for (int q = 0; q < B; ++q) acc -= A(e * EV + q) * x[e].v[q];
+                for (int q = 0; q < B; ++q) sum.add(e, 0, A(e * EV + q), x[e].v[q]);
+              T acc = sum.row(0, t[k][0]);
               if constexpr (FWD) {
                 const int l0 = lane - p;
                 T y = A(NE * EV) * __shfl_sync(0xffffffffu, acc, l0);
