@@ -1062,6 +1062,7 @@ SoloArgs solo_launch_args(dfg_ctx ctx_, SweepDev& S, bool fp32, void* out, int* 
   a.NS = D.shape.ns;
   a.R = D.shape.R;
   a.max_nent = D.plan.P.max_nent;
+  a.single = true;
   return a;
 }
 

@@ -71,17 +71,21 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// What a sweep takes off a row's right-hand side, entry after entry: component p of
-// t[p] - sum over e, q of block(e)(p, q) x(e)(q), in one order for every kernel that
-// evaluates a row in one lane or a lane per component.  FP32 rows of 3x3 blocks (21
-// products per component in a tetrahedral mesh) are added up in four sums, entry e
-// in sum e % 4, apart from the right-hand side: one chain from the right-hand side on
-// has 1.9 times the error of the level-scheduled kernel's sums over lanes (elasticity
-// on 56^3 cells, sweep against FP64: 1.02e-7, 5.4e-8, in four sums 5.4e-8), and takes
-// as long (that solve 130.7 and 131.1 ms).
-template <typename T, int B, int P = B>
+// What a sweep takes off a row's right-hand side: component p of t[p] - sum over e, q
+// of block(e)(p, q) x(e)(q), entry after entry, as the strip and the one-CTA kernel
+// evaluate a row.
+//
+// FOUR (single solves, FP32, 3x3 blocks: 21 products per component in a tetrahedral
+// mesh): four sums, entry e in sum e % 4, apart from the right-hand side.  One chain
+// from the right-hand side on has 1.9 times the error of the level-scheduled kernel's
+// sums over lanes, where these solves would otherwise sweep (elasticity on 56^3 cells,
+// sweep against FP64: 1.02e-7, levels 5.4e-8, four sums 5.4e-8), and takes as long
+// (that solve 130.7 and 131.1 ms).  The server's kernels give the same bits in one
+// chain.
+constexpr bool sweep_four(bool fp32, int b) { return fp32 && b == 3; }
+template <typename T, int B, int P, bool FOUR>
 struct RowSum {
-  static constexpr int N = sizeof(T) == 4 && B == 3 ? 4 : 1;
+  static constexpr int N = FOUR ? 4 : 1;
   T s[N][P];
   __device__ __forceinline__ void start(const T (&t)[P]) {
 #pragma unroll

@@ -44,7 +44,7 @@
 
 namespace dfg {
 
-template <typename T, int B, bool FWD, int MAXE>
+template <typename T, int B, bool FWD, int MAXE, bool FOUR>
 __global__ void __launch_bounds__((kSoloWarps + 1) * 32) k_solo(SoloArgs a) {
   constexpr int BS = B * B;
   constexpr int SZ = (int)sizeof(T);
@@ -181,7 +181,7 @@ __global__ void __launch_bounds__((kSoloWarps + 1) * 32) k_solo(SoloArgs a) {
               T t[B];
 #pragma unroll
               for (int d = 0; d < B; ++d) t[d] = val[lane * B + d];
-              RowSum<T, B> sum;
+              RowSum<T, B, B, FOUR> sum;
               sum.start(t);
               if constexpr (MAXE > 0) {
                 // all dependency values first, then the FMAs.  The codes are
@@ -222,9 +222,9 @@ __global__ void __launch_bounds__((kSoloWarps + 1) * 32) k_solo(SoloArgs a) {
                   }
                 }
               } else {
-                for (int e0 = 0; e0 < nent; e0 += RowSum<T, B>::N)
+                for (int e0 = 0; e0 < nent; e0 += decltype(sum)::N)
 #pragma unroll
-                  for (int k = 0; k < RowSum<T, B>::N; ++k) {
+                  for (int k = 0; k < decltype(sum)::N; ++k) {
                     const int e = e0 + k;
                     if (e >= nent) break;
                     const int cd = code[e * 32 + lane];
@@ -314,12 +314,12 @@ cudaError_t launch_solo_permute(bool fp32, long long n, int b, const int* pos, c
   return cudaGetLastError();
 }
 
-template <typename T, int B, bool FWD>
+template <typename T, int B, bool FWD, bool FOUR = false>
 static cudaError_t launch_e(const SoloArgs& a, int grid, size_t smem, cudaStream_t st) {
   constexpr int NT = (kSoloWarps + 1) * 32;
-  if (a.max_nent <= 4) k_solo<T, B, FWD, 4><<<grid, NT, smem, st>>>(a);
-  else if (a.max_nent <= 8) k_solo<T, B, FWD, 8><<<grid, NT, smem, st>>>(a);
-  else k_solo<T, B, FWD, 0><<<grid, NT, smem, st>>>(a);
+  if (a.max_nent <= 4) k_solo<T, B, FWD, 4, FOUR><<<grid, NT, smem, st>>>(a);
+  else if (a.max_nent <= 8) k_solo<T, B, FWD, 8, FOUR><<<grid, NT, smem, st>>>(a);
+  else k_solo<T, B, FWD, 0, FOUR><<<grid, NT, smem, st>>>(a);
   return cudaGetLastError();
 }
 
@@ -334,17 +334,19 @@ static cudaError_t launch_b(int B, const SoloArgs& a, int grid, size_t smem, cud
 }
 
 cudaError_t launch_solo(bool forward, bool fp32, int B, const SoloArgs& a, int grid, size_t smem, cudaStream_t st) {
+  if (a.single && sweep_four(fp32, B))
+    return forward ? launch_e<float, 3, true, true>(a, grid, smem, st) : launch_e<float, 3, false, true>(a, grid, smem, st);
   if (fp32) return forward ? launch_b<float, true>(B, a, grid, smem, st) : launch_b<float, false>(B, a, grid, smem, st);
   return forward ? launch_b<double, true>(B, a, grid, smem, st) : launch_b<double, false>(B, a, grid, smem, st);
 }
 
-template <typename T, int B, bool FWD>
+template <typename T, int B, bool FWD, bool FOUR = false>
 static cudaError_t set_attr(size_t max_smem) {
-  cudaError_t e = cudaFuncSetAttribute(k_solo<T, B, FWD, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem);
+  cudaError_t e = cudaFuncSetAttribute(k_solo<T, B, FWD, 4, FOUR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_solo<T, B, FWD, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem);
+    e = cudaFuncSetAttribute(k_solo<T, B, FWD, 8, FOUR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_solo<T, B, FWD, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem);
+    e = cudaFuncSetAttribute(k_solo<T, B, FWD, 0, FOUR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem);
   return e;
 }
 
@@ -356,6 +358,8 @@ cudaError_t solo_set_smem_limits(size_t max_smem) {
   DFG_ATTR(double, 1) DFG_ATTR(double, 2) DFG_ATTR(double, 3)
   DFG_ATTR(float, 1) DFG_ATTR(float, 2) DFG_ATTR(float, 3)
 #undef DFG_ATTR
+  if (e == cudaSuccess) e = set_attr<float, 3, true, true>(max_smem);
+  if (e == cudaSuccess) e = set_attr<float, 3, false, true>(max_smem);
   return e;
 }
 

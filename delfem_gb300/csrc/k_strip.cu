@@ -35,9 +35,9 @@
 // Every wait is bounded; one that gives up records kErrTimeout, and the launch
 // drains its copies and returns.
 //
-// A row is evaluated by the operations of the ranged and one-CTA kernels in their
-// order (RowSum, then D^-1), so these give the same bits; with split, column by
-// column.
+// A row is evaluated by the operations of the one-CTA kernel in its order (RowSum,
+// then D^-1), and of the ranged kernel in batched launches, so these give the same
+// bits; with split, column by column.
 //
 // Chunk layout: [need: CH ints, kStripHdr bytes][steps: step_bytes each]; a
 // step is pieces of 16 bytes per lane, piece j of lane l at (j*32 + l)*16:
@@ -210,7 +210,7 @@ __device__ __forceinline__ void receive(const StripSlot& S, int r, unsigned char
 
 // (one CTA per SM in the bounds: without it ptxas aims at several and keeps
 // steps to 64 registers and fewer, 2 to 10 % slower)
-template <typename T, int B, bool FWD, int NE, bool SPLIT>
+template <typename T, int B, bool FWD, int NE, bool SPLIT, bool FOUR>
 __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(StripArgs a) {
   constexpr int SZ = (int)sizeof(T);
   constexpr StripDims D = strip_dims(B, SZ, FWD, NE, SPLIT);
@@ -504,7 +504,7 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
             if (SZ == 8 && more) decode((j + 1) % K2);
             // the rows
             if constexpr (LPR == 1) {
-              RowSum<T, B> sum;
+              RowSum<T, B, B, FOUR> sum;
               sum.start(t[k]);
 #pragma unroll
               for (int e = 0; e < NE; ++e)
@@ -542,7 +542,7 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
               yl.v[0] = acc;
               if (XNOW) xstore(xs[k], xp[k], yl);
             } else {
-              RowSum<T, B, 1> sum;
+              RowSum<T, B, 1, FOUR> sum;
               sum.start(t[k]);
 #pragma unroll
               for (int e = 0; e < NE; ++e)
@@ -663,14 +663,14 @@ cudaError_t launch_strip_pack(bool forward, bool fp32, const StripPackArgs& a, c
   return forward ? pack_t<double, true>(a, st) : pack_t<double, false>(a, st);
 }
 
-// calls f(kernel) for the instance of (fp32, b, forward, ne, split)
-template <typename T, int B, bool FWD, bool SPLIT, typename F>
+// calls f(kernel) for the instance of (fp32, b, forward, ne, split, four)
+template <typename T, int B, bool FWD, bool SPLIT, bool FOUR = false, typename F>
 static cudaError_t with_class(int ne, F&& f) {
   switch (ne) {
-    case 3: return f(k_strip<T, B, FWD, 3, SPLIT>);
-    case 4: return f(k_strip<T, B, FWD, 4, SPLIT>);
-    case 7: return f(k_strip<T, B, FWD, 7, SPLIT>);
-    case 16: return f(k_strip<T, B, FWD, 16, SPLIT>);
+    case 3: return f(k_strip<T, B, FWD, 3, SPLIT, FOUR>);
+    case 4: return f(k_strip<T, B, FWD, 4, SPLIT, FOUR>);
+    case 7: return f(k_strip<T, B, FWD, 7, SPLIT, FOUR>);
+    case 16: return f(k_strip<T, B, FWD, 16, SPLIT, FOUR>);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -684,7 +684,9 @@ static cudaError_t with_block(int b, bool forward, int ne, F&& f) {
   }
 }
 template <typename F>
-static cudaError_t with_kernel(bool fp32, int b, bool forward, int ne, bool split, F&& f) {
+static cudaError_t with_kernel(bool fp32, int b, bool forward, int ne, bool split, bool four, F&& f) {
+  if (four)
+    return forward ? with_class<float, 3, true, false, true>(ne, f) : with_class<float, 3, false, false, true>(ne, f);
   if (split && b == 2) return forward ? with_class<double, 2, true, true>(ne, f) : with_class<double, 2, false, true>(ne, f);
   if (split && b == 3) return forward ? with_class<double, 3, true, true>(ne, f) : with_class<double, 3, false, true>(ne, f);
   return fp32 ? with_block<float>(b, forward, ne, f) : with_block<double>(b, forward, ne, f);
@@ -703,7 +705,7 @@ cudaError_t launch_strip(bool forward, bool fp32, int b, const StripArgs& a, int
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = dep ? 1 : 0;
-  return with_kernel(fp32, b, forward, a.ne, a.split, [&](auto k) { return cudaLaunchKernelEx(&cfg, k, a); });
+  return with_kernel(fp32, b, forward, a.ne, a.split, !a.batch && sweep_four(fp32, b), [&](auto k) { return cudaLaunchKernelEx(&cfg, k, a); });
 }
 
 cudaError_t strip_set_smem_limits(size_t max_smem) {
@@ -712,8 +714,8 @@ cudaError_t strip_set_smem_limits(size_t max_smem) {
     for (int ne : {3, 4, 7, 16})
       for (int b = 1; b <= 3; ++b)
         for (int fp32 = 0; fp32 < 2; ++fp32)
-          for (int split = 0; split <= (strip_can_split(b, fp32 ? 4 : 8) ? 1 : 0); ++split) {
-            const cudaError_t e = with_kernel(fp32, b, fwd, ne, split, set);
+          for (int form = 0; form <= (strip_can_split(b, fp32 ? 4 : 8) || sweep_four(fp32, b) ? 1 : 0); ++form) {
+            const cudaError_t e = with_kernel(fp32, b, fwd, ne, form && !fp32, form && fp32, set);
             if (e != cudaSuccess) return e;
           }
   return cudaSuccess;

@@ -223,8 +223,6 @@ __global__ void __launch_bounds__(64) k_sweep(SweepArgs a) {
           T t[B];
 #pragma unroll
           for (int d = 0; d < B; ++d) t[d] = reinterpret_cast<const T*>(val)[lane * B + d];
-          RowSum<T, B> sum;
-          sum.start(t);
           if constexpr (MAXE > 0) {
             // all dependency values first (independent shared-memory loads),
             // one staleness test, then the FMAs
@@ -258,44 +256,44 @@ __global__ void __launch_bounds__(64) k_sweep(SweepArgs a) {
             for (int e = 0; e < MAXE; ++e) {
               if (e < nent) {
 #pragma unroll
-                for (int p = 0; p < B; ++p)
+                for (int p = 0; p < B; ++p) {
+                  T acc = t[p];
 #pragma unroll
-                  for (int q = 0; q < B; ++q) sum.add(e, p, blk[(e * BS + p * B + q) * 32 + lane], v[e][q]);
+                  for (int q = 0; q < B; ++q) acc -= blk[(e * BS + p * B + q) * 32 + lane] * v[e][q];
+                  t[p] = acc;
+                }
               }
             }
           } else {
-            for (int e0 = 0; e0 < nent; e0 += RowSum<T, B>::N)
+            for (int e = 0; e < nent; ++e) {
+              const int c = code[e * 32 + lane];
+              const unsigned char* base = (c < 0) ? val : ringreg;
+              const T* vp = reinterpret_cast<const T*>(base + (c & 0x7fffffff));
+              T v[B];
+              bool stale = false;
 #pragma unroll
-              for (int k = 0; k < RowSum<T, B>::N; ++k) {
-                const int e = e0 + k;
-                if (e >= nent) break;
-                const int c = code[e * 32 + lane];
-                const unsigned char* base = (c < 0) ? val : ringreg;
-                const T* vp = reinterpret_cast<const T*>(base + (c & 0x7fffffff));
-                T v[B];
-                bool stale = false;
-#pragma unroll
-                for (int d = 0; d < B; ++d) {
-                  v[d] = vp[d];
-                  stale |= is_sentinel(v[d]);
-                }
-                if (stale) {
-                  int ab = 0;
-#pragma unroll
-                  for (int d = 0; d < B; ++d)
-                    if (is_sentinel(v[d]))
-                      v[d] = poll_value<T>(&out[(size_t)grow[e * 32 + lane] * B + d], a.err, &ab, jslot,
-                                           grow[e * 32 + lane]);
-                  abort |= ab != 0;
-                }
-#pragma unroll
-                for (int p = 0; p < B; ++p)
-#pragma unroll
-                  for (int q = 0; q < B; ++q) sum.add(k, p, blk[(e * BS + p * B + q) * 32 + lane], v[q]);
+              for (int d = 0; d < B; ++d) {
+                v[d] = vp[d];
+                stale |= is_sentinel(v[d]);
               }
-          }
+              if (stale) {
+                int ab = 0;
 #pragma unroll
-          for (int p = 0; p < B; ++p) t[p] = sum.row(p, t[p]);
+                for (int d = 0; d < B; ++d)
+                  if (is_sentinel(v[d]))
+                    v[d] = poll_value<T>(&out[(size_t)grow[e * 32 + lane] * B + d], a.err, &ab, jslot,
+                                         grow[e * 32 + lane]);
+                abort |= ab != 0;
+              }
+#pragma unroll
+              for (int p = 0; p < B; ++p) {
+                T acc = t[p];
+#pragma unroll
+                for (int q = 0; q < B; ++q) acc -= blk[(e * BS + p * B + q) * 32 + lane] * v[q];
+                t[p] = acc;
+              }
+            }
+          }
           T y[B];
           if constexpr (FWD) {
             const T* dinv = blk + nent * BS * 32;

@@ -112,6 +112,7 @@ struct SoloArgs {
   int NS;            // pipeline stages
   int R;             // ring depth in steps (a power of two)
   int max_nent;      // selects the unrolled variant
+  bool single;       // a single solve: its order of sums (RowSum)
 };
 // compute warps per CTA (plus one producer warp)
 constexpr int kSoloWarps = 16;
