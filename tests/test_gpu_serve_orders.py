@@ -43,3 +43,28 @@ def test_served_orders(gpu_ctx, mode):
     for a, c in zip(*got):
         assert a["status"] == 0 and a["rel_true"] <= 1e-8 and a["iterations"] == c["iterations"]
         assert np.array_equal(a["x"], c["x"])
+
+
+def test_budget_that_fits_without_strips(gpu_ctx):
+    """A request that fits the whole budget only in the kind that needs less memory
+    than strips is served by it, with the same bits."""
+    import re
+    from delfem_gb300 import meshgen as mg
+    from delfem_gb300.capi import DFG_OOM_REJECTED
+    from delfem_gb300.serve import Server
+    coords, conn = mg.tet_grid(14, 13, 12)
+    coords, conn = renumber(coords, conn, boundary_first(coords, conn))
+    p = mg.mesh_problem(mg.SOLID3D, coords, conn, seed=2, coef_sigma=0.5)
+    need = {}
+    for sweeps in (0, 2):
+        with Server(gpu_ctx, budget_bytes=1 << 20, sweeps=sweeps) as S:
+            r = S.wait(S.submit(p))
+            assert r["status"] == DFG_OOM_REJECTED
+            need[sweeps] = int(re.search(r"needs (\d+) device bytes", r["error"]).group(1))
+    assert need[0] <= need[2]
+    got = []
+    for budget in (need[2], 1 << 30):
+        with Server(gpu_ctx, budget_bytes=budget) as S:
+            got.append(S.wait(S.submit(p)))
+    assert got[0]["status"] == 0 and got[0]["iterations"] == got[1]["iterations"]
+    assert np.array_equal(got[0]["x"], got[1]["x"])
