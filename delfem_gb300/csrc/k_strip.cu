@@ -322,8 +322,8 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
       bool failing = false;
       for (unsigned n = 1; __any_sync(0xffffffffu, issued < nch && !failing); ++n) {
         if (issued < nch && !failing) {
-          const int end = strip_issue_end(ld_acquire_s(consumed), CH, NS, nch);
-          for (; issued < end; ++issued) {
+          const int done = ld_acquire_s(consumed) / CH;
+          for (; issued < strip_issue_end(done, NS, nch); ++issued) {
             const int s = (st + issued) % NS;
             mbar_expect_tx(&full[s], D.chunk_bytes + RHS_CHUNK);
             tma_load_1d(rstage + (size_t)s * D.chunk_bytes, rec, D.chunk_bytes, &full[s]);
@@ -568,7 +568,7 @@ __global__ void __launch_bounds__((2 * kStripMaxWarps + 1) * 32, 1) k_strip(Stri
           }
           if (Q == 1 && abort) break;
           // the chunk's stage is free (warp 0 waited for its copies, unless it gave up)
-          if (const int steps = strip_publish(Q > 1 && abort, c, CH); tid == 0 && steps) st_release_s(consumed, steps);
+          if (strip_publishes(Q > 1 && abort) && tid == 0) st_release_s(consumed, (c + 1) * CH);
           sp = sp1;
           vp = vp1;
           rg = (c + 1) * CH % kStripRing == 0 ? ring0 : rg + CH * RW * BP;

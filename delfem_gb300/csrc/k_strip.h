@@ -195,11 +195,11 @@ std::vector<int> strip_meta(const StripPlan& P, const int* out_pos, int W, int N
 // when its copies have landed and been read.  A strip that has given up
 // publishes nothing more: the chunks from `consumed` on that were issued are then
 // those whose copies may be in flight, and the launch waits for them.
-__host__ __device__ constexpr int strip_publish(bool gave_up, int chunk, int CH) {  // 0: nothing to publish
-  return gave_up ? 0 : (chunk + 1) * CH;
-}
-__host__ __device__ constexpr int strip_issue_end(int consumed, int CH, int NS, int nchunks) {
-  return consumed / CH + NS < nchunks ? consumed / CH + NS : nchunks;
+// (Conditions without a value to test: one more test per chunk on the compute warp's
+// way cost 0.9 % of elasticity on 401x199 cells.)
+__host__ __device__ constexpr bool strip_publishes(bool gave_up) { return !gave_up; }  // (chunk + 1) * CH steps
+__host__ __device__ constexpr int strip_issue_end(int chunks_done, int NS, int nchunks) {
+  return nchunks < chunks_done + NS ? nchunks : chunks_done + NS;
 }
 __host__ __device__ constexpr int strip_drain_begin(int consumed, int CH) { return consumed / CH; }
 

@@ -21,7 +21,7 @@ extern "C" int emul_strip_stages(int nch, int CH, int NS, int fail, int slow, un
   while (!done) {
     const unsigned what = rng() % (slow ? 8 : 3);
     if (what == 0) {  // loader
-      for (const int end = strip_issue_end(consumed, CH, NS, nch); issued < end; ++issued) {
+      for (const int done_chunks = consumed / CH; issued < strip_issue_end(done_chunks, NS, nch); ++issued) {
         if (issued_at[issued % NS]) return 1;
         issued_at[issued % NS] = 1;
         stage_chunk[issued % NS] = issued;
@@ -30,7 +30,7 @@ extern "C" int emul_strip_stages(int nch, int CH, int NS, int fail, int slow, un
       issued_at[rng() % NS] = 0;
     } else if (what == 2 || c >= fail) {  // first warp: a chunk
       if (c < nch && (c >= fail || (stage_chunk[c % NS] == c && !issued_at[c % NS]))) {
-        if (const int steps = strip_publish(c >= fail, c, CH)) consumed = steps;
+        if (strip_publishes(c >= fail)) consumed = (c + 1) * CH;
         ++c;
       }
       done = c == nch;

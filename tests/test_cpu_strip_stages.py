@@ -1,5 +1,5 @@
 """The chunk stages of a strip whose warps give up half-way (k_strip.h,
-strip_publish): no stage is issued again while its copy is in flight, and the
+strip_publishes): no stage is issued again while its copy is in flight, and the
 launch waits for every copy that it issued."""
 import ctypes
 import os
