@@ -740,7 +740,7 @@ def compose_serve_line(args, world, cfg, items, timed_items, timed_probs, result
         achieved = v["bytes"] / (v["ms"] * 1e-3) / 1e9
         roof = {"bound": "hbm", "achieved": round(achieved, 1), "peak": hbm_peak, "unit": "GB/s",
                 "frac": round(achieved / hbm_peak, 4),
-                # served sweeps run in strips where the rows fit them
+                # the streams' sweeps run in strips (their meshes are numbered row by row)
                 "traffic": ncu_traffic(dom + ":strips" if dom.startswith("sweep") else dom, v["bytes"]),
                 "peak_source": peak_kind,
                 "kernel": dom, "ms_per_launch": round(v["ms"], 4), "algorithmic_bytes": int(v["bytes"]),
