@@ -79,9 +79,11 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // mesh): four sums, entry e in sum e % 4, apart from the right-hand side.  One chain
 // from the right-hand side on has 1.9 times the error of the level-scheduled kernel's
 // sums over lanes, where these solves would otherwise sweep (elasticity on 56^3 cells,
-// sweep against FP64: 1.02e-7, levels 5.4e-8, four sums 5.4e-8), and takes as long
-// (that solve 130.7 and 131.1 ms).  The server's kernels give the same bits in one
-// chain.
+// sweep against FP64: 1.02e-7, levels 5.4e-8, four sums 5.4e-8).  It costs 1 % on 24^3
+// cells (84.2 -> 85.3 us per iteration) and less on 56^3 (130.7 -> 131.0 ms).  Four sums
+// of which one starts at the right-hand side are 1.15 times as inexact as the levels,
+// two sums 1.07 times, and either half of that cost.  The server's kernels give the
+// same bits in one chain.
 constexpr bool sweep_four(bool fp32, int b) { return fp32 && b == 3; }
 template <typename T, int B, int P, bool FOUR>
 struct RowSum {
